@@ -59,18 +59,27 @@ __global__ void k_mask_bits(long long K, long long J, const double *lmn, const i
   if (lane == 0) bits[word] = b;
 }
 
-// Locality key of a direction: its HEALPix NESTED index at Nside 2^13
-// (standard ang2pix_nest).  NESTED indices are hierarchical, so sorting by the
-// key puts every 4^k-aligned run of pixels in a compact patch of sky -- for a
-// HEALPix grid of any Nside <= 2^13 the sorted order is its NESTED order.
-__device__ unsigned long long spread32(unsigned long long x) {
-  x &= 0xffffffffull;
-  x = (x | (x << 16)) & 0x0000ffff0000ffffull;
-  x = (x | (x << 8)) & 0x00ff00ff00ff00ffull;
-  x = (x | (x << 4)) & 0x0f0f0f0f0f0f0f0full;
-  x = (x | (x << 2)) & 0x3333333333333333ull;
-  x = (x | (x << 1)) & 0x5555555555555555ull;
-  return x;
+// Locality key of a direction: its base face and the position of its face
+// coordinates at Nside 2^13 (standard ang2pix_nest) along a Hilbert curve.  The
+// curve visits the same hierarchy of squares as the NESTED index, so for a
+// HEALPix grid of a power-of-two Nside every aligned run of 4^k records is the
+// NESTED pixel of that size; but it never jumps, so runs that are not aligned
+// (every run of another Nside, or of any other pixel set) stay compact too.  At
+// Nside 101 the chord radius of 128-record tiles, in tile sides, is 0.88 / 1.12 /
+// 4.8 (median, 90 %, 99 %) against 1.10 / 2.0 / 8.7 in NESTED order.
+__device__ unsigned long long hilbert_index(long long N, long long x, long long y) {
+  unsigned long long d = 0;
+  for (long long s = N / 2; s > 0; s >>= 1) {
+    const bool rx = (x & s) != 0, ry = (y & s) != 0;
+    d += static_cast<unsigned long long>(s * s) * ((rx ? 3u : 0u) ^ (ry ? 1u : 0u));
+    if (!ry) {
+      if (rx) x = N - 1 - x, y = N - 1 - y;
+      const long long t = x;
+      x = y;
+      y = t;
+    }
+  }
+  return d;
 }
 
 __global__ void k_pix_keys(long long J, const double *lmn, unsigned long long *keys, int *idx) {
@@ -105,7 +114,7 @@ __global__ void k_pix_keys(long long J, const double *lmn, unsigned long long *k
   face = face < 0 ? 0 : (face > 11 ? 11 : face);
   ix = ix < 0 ? 0 : (ix >= N ? N - 1 : ix);
   iy = iy < 0 ? 0 : (iy >= N ? N - 1 : iy);
-  keys[i] = static_cast<unsigned long long>(face) * N * N + spread32(ix) + (spread32(iy) << 1);
+  keys[i] = static_cast<unsigned long long>(face) * N * N + hilbert_index(N, ix, iy);
   idx[i] = static_cast<int>(i);
 }
 

@@ -6,7 +6,7 @@
 // no occultation mask (vissgen3d_noblockage.cu:167-182).  Evaluated directly
 // (k_adjoint) it costs K x J exponentials.  Here the sky is cut into facets:
 // runs of the plan's pixel records, which are sorted by a hierarchical
-// (NESTED) key, so a facet of 4^n records is a compact sky patch.  In the
+// key, so a facet of 4^n records is a compact sky patch.  In the
 // local frame of facet f (e3 = its centre direction c, e1 and e2 across it)
 // a pixel is s = x e1 + y e2 + (1 + zc + z) e3 with |x|, |y| small and z
 // tiny, so
