@@ -71,8 +71,9 @@ BIG_WORKLOADS = ("prod_1mhz",)
 
 
 # the translation units of the kernels a traffic record measures (k_forward,
-# k_adjoint, k_form_forward, k_form_adjoint) and every header they include
-TRAFFIC_KERNEL_SOURCES = ("formation.cu", "visibility.cu", "visibility.cuh", "viss_common.cuh")
+# k_adjoint, k_form_forward, k_form_adjoint, k_track_*) and every header they include
+TRAFFIC_KERNEL_SOURCES = ("direct.cuh", "formation.cu", "tcgen05.cuh", "tracks.cu", "tracks.cuh", "tracks_impl.cuh",
+                          "visibility.cu", "visibility.cuh", "viss_common.cuh")
 
 
 def kernel_sources_sha() -> str:

@@ -128,8 +128,14 @@ int viss_plan_set_samples(viss_plan *plan, int64_t K, const double *uvw, const d
  *   V_k = sum_j sky_j vis_kj exp(-2 pi i (u_k . s_j + off_k)),  k < K
  * sky: J FP32; V: K complex64.  Split precision by default (FP64 phase and
  * turn reduction, FP32 sincos, compensated FP32 sums, FP64 cross-block sum);
- * VISS_FP64 selects the plain FP64 path.  Asynchronous: VISS_OK means the
- * work was launched.  A bounded device-side wait that gave up inside the
+ * VISS_FP64 selects the plain FP64 path.  From 1e10 sample x pixel terms on,
+ * samples that lie on smooth tracks (the baselines of a formation) go through
+ * track blocks: most exponentials interpolated from a few samples per block, to
+ * the same accuracy.  The first split call after the samples or pixels were
+ * staged builds them (a few waits for the device, 1-3 ms) and every call then
+ * uses device buffers of the plan, about 1 GiB and 1 KiB per sample; without
+ * that memory, under stream capture, and for other samples every term is
+ * evaluated.  Asynchronous: VISS_OK means the work was launched.  A bounded device-side wait that gave up inside the
  * kernel (V then incomplete) is reported only by the next
  * viss_plan_last_stats / viss_plan_last_counts on this plan, which return
  * VISS_ERR_TIMEOUT; callers that need the guarantee check it after the call. */
@@ -137,8 +143,8 @@ int viss_forward(viss_plan *plan, const float *sky, float *V, int flags, void *s
 
 /* Imaging adjoint, replaces computeC (vissgen3d_blockage.cu:167-192):
  *   image_j = scale * sum_k Re(coef_k exp(+2 pi i (u_k . s_j + off_k))) vis_kj
- * coef: K complex64 (the weighted visibilities w_k V_k); image: J FP32.
- * Asynchronous; a timed-out wait is reported as for viss_forward, only
+ * coef: K complex64 (the weighted visibilities w_k V_k); image: J FP32.  Track
+ * blocks as in viss_forward.  Asynchronous; a timed-out wait is reported as for viss_forward, only
  * through viss_plan_last_stats / viss_plan_last_counts. */
 int viss_adjoint(viss_plan *plan, const float *coef, float *image, float scale, int flags,
                  void *stream);
@@ -158,7 +164,7 @@ int viss_plan_tune(viss_plan *plan, const float *sky, const float *coef, float *
  * relative, split precision),
  *   image_j = scale * sum_k Re(coef_k exp(+2 pi i (u_k . s_j + off_k))) vis_kj,
  * through per-facet type-3 NUFFTs.  The plan's pixel records (sorted by a
- * NESTED key) are cut into facets of `facet_pixels` records; 0 picks the size
+ * hierarchical key) are cut into facets of `facet_pixels` records; 0 picks the size
  * 4^n with the least modelled time among those whose grid fits, from the
  * facets' measured extents.  Each facet: the samples spread onto a uniform
  * frequency grid in the facet's local frame ("exponential of semicircle"

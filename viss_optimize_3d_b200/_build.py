@@ -24,8 +24,9 @@ LIB = os.path.join(PKG, "libviss.so")
 BIN = os.path.join(PKG, "bin")
 
 CU_SOURCES = ["healpix.cu", "geometry.cu", "visibility.cu", "dcf.cu", "capi.cu", "noalloc.cu",
-              "days.cu", "formation.cu", "gridded.cu"]
-HEADERS = ["viss_common.cuh", "visibility.cuh"]
+              "days.cu", "formation.cu", "gridded.cu", "tracks.cu", "tracks_build.cu"]
+HEADERS = ["viss_common.cuh", "visibility.cuh", "tracks.cuh", "tracks_impl.cuh", "direct.cuh",
+           "tcgen05.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE,

@@ -62,6 +62,7 @@ int gridded_adjoint(void **state, long long J, const double4 *pix, const int *pe
 void gridded_free(void *state);
 }  // namespace viss
 
+#include "tracks.cuh"
 #include "visibility.cuh"
 
 namespace {
@@ -181,6 +182,10 @@ struct viss_plan {
   long long gridded_facet = 0;
   long long gridded_hbm_blocks = 0;
   long long geom_version = 0;   // bumped by every call that restages pixels or samples
+  // track blocks of the staged samples (tracks.cu), for geometry tracks_version
+  void *tracks = nullptr;
+  long long tracks_version = -1;
+  bool tracks_usable = false;
 };
 
 namespace {
@@ -356,6 +361,7 @@ int viss_plan_destroy(viss_plan *p) {
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->gridded) viss::gridded_free(p->gridded);
+  if (p->tracks) viss::tracks_free(p->tracks);
   delete p;
   return VISS_OK;
 }
@@ -374,7 +380,7 @@ int viss_plan_set_pixels(viss_plan *p, int64_t J, const double *lmn, void *strea
     return s;
   if (int s = ensure(p->perm, p->perm_cap, sizeof(int) * J, "pixel order")) return s;
   const cudaStream_t st = as_stream(stream);
-  // compact tiles: order the pixels by a hierarchical (NESTED) locality key
+  // compact tiles: order the pixels along a hierarchical curve (launch_pix_keys)
   void *tmp = nullptr;
   const size_t kbytes = sizeof(unsigned long long) * J, ibytes = sizeof(int) * J;
   VISS_CUDA(cudaMallocAsync(&tmp, 2 * kbytes + ibytes, st), "viss_plan_set_pixels: keys");
@@ -444,8 +450,53 @@ static int workspace(viss_plan *p, size_t bytes) {
   return ensure(p->part, p->part_cap, bytes, "partial-sum workspace");
 }
 
+static viss::TrackInputs track_inputs(const viss_plan *p) {
+  viss::TrackInputs in{};
+  in.pix = p->pix;
+  in.cones = p->cones;
+  in.perm = p->perm;
+  in.J = p->J;
+  in.Jpad = p->Jpad;
+  in.ntiles = p->ntiles;
+  in.samp = p->samp;
+  in.refs = p->has_refs ? p->refs : nullptr;
+  in.occ = p->occ;
+  in.occ32 = p->occ32;
+  in.K = p->K;
+  in.Kc = p->Kc;
+  in.channels = p->channels;
+  in.nsm = p->nsm;
+  in.max_turns = p->max_turns;
+  return in;
+}
+
+// Whether a split-precision call goes through the track blocks, built here for
+// newly staged samples.  From kTrackMinTerms terms on: the build takes 1-2 ms
+// (a few waits for the device among it), so a single call has to be longer.
+// Not under stream capture: a captured call is replayed after the samples were
+// staged again, and the blocks' launch sizes depend on the samples.
+constexpr double kTrackMinTerms = 1e10;
+static int tracks_ready(viss_plan *p, cudaStream_t st, bool *use) {
+  *use = false;
+  if (static_cast<double>(p->K) * p->J < kTrackMinTerms) return VISS_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return VISS_OK;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return VISS_OK;
+  if (p->tracks_version != p->geom_version) {
+    bool ok = false;
+    if (int s = viss::tracks_build(&p->tracks, track_inputs(p), st, &ok)) return s;
+    p->tracks_usable = ok;
+    p->tracks_version = p->geom_version;
+  }
+  *use = p->tracks_usable;
+  return VISS_OK;
+}
+
 static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cudaStream_t st,
-                        int shape) {
+                        int shape, bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
   const int nchunk = fwd_chunks(p, shape, fp64);
@@ -457,6 +508,20 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                                    p->channels, st),
             "viss_forward: sky");
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_forward");
+  bool use = false;
+  if (tracks && !fp64)
+    if (int s = tracks_ready(p, st, &use)) return s;
+  if (use) {
+    const int s = viss::tracks_forward(p->tracks, track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V), masked,
+                                       !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
+                                       reinterpret_cast<int *>(p->dev_words + 1), p->drop_tile, st);
+    if (s != VISS_ERR_ALLOC) {   // short of memory for its sums: the direct kernel has its workspace
+      p->drop_tile = -1;
+      p->last_total = p->K * p->J;
+      p->last_stream = st;
+      return s;
+    }
+  }
   viss::FwdParams fp;
   fp.samp = p->samp;
   fp.refs = masked ? p->refs : nullptr;
@@ -512,7 +577,8 @@ int viss_forward(viss_plan *p, const float *sky, float *V, int flags, void *stre
 // adjoint; facets of facet_pix records, nfacets of them.
 static int adjoint_impl(viss_plan *p, const float *coef, float *image, float scale, int flags,
                         cudaStream_t st, int shape, const float4 *fcones = nullptr, long long facet_pix = 0,
-                        long long nfacets = 0, const unsigned *mixbits = nullptr, long long mix_words = 0) {
+                        long long nfacets = 0, const unsigned *mixbits = nullptr, long long mix_words = 0,
+                        bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
   int spc = 0;
@@ -522,6 +588,20 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
   VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, st),
             "viss_adjoint: coef");
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint");
+  bool use = false;
+  if (tracks && !fp64 && !fcones)
+    if (int s = tracks_ready(p, st, &use)) return s;
+  if (use) {
+    const int s = viss::tracks_adjoint(p->tracks, track_inputs(p), p->coef, image, scale, masked,
+                                       !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
+                                       reinterpret_cast<int *>(p->dev_words + 1), p->drop_tile, st);
+    if (s != VISS_ERR_ALLOC) {
+      p->drop_tile = -1;
+      p->last_total = p->K * p->J;
+      p->last_stream = st;
+      return s;
+    }
+  }
   viss::AdjParams ap;
   ap.samp = p->samp;
   ap.coef = p->coef;
@@ -582,10 +662,10 @@ int viss_plan_tune(viss_plan *p, const float *sky, const float *coef, float *V_s
   float best_f = 1e30f, best_a = 1e30f;
   int bf = p->fwd_shape, ba = p->adj_shape, status = VISS_OK;
   for (int s = 0; s < viss::kNumFwdShapes && status == VISS_OK; ++s) {
-    status = forward_impl(p, sky, V_scratch, flags, st, s);
+    status = forward_impl(p, sky, V_scratch, flags, st, s, false);
     if (status) break;
     cudaEventRecord(e0, st);
-    status = forward_impl(p, sky, V_scratch, flags, st, s);
+    status = forward_impl(p, sky, V_scratch, flags, st, s, false);
     cudaEventRecord(e1, st);
     if (cudaEventSynchronize(e1) != cudaSuccess) { status = cuda_fail(cudaGetLastError(), "viss_plan_tune"); break; }
     float ms = 0;
@@ -593,10 +673,10 @@ int viss_plan_tune(viss_plan *p, const float *sky, const float *coef, float *V_s
     if (ms < best_f) { best_f = ms; bf = s; }
   }
   for (int s = 0; s < viss::kNumAdjShapes && status == VISS_OK; ++s) {
-    status = adjoint_impl(p, coef, img_scratch, 1.0f, flags, st, s);
+    status = adjoint_impl(p, coef, img_scratch, 1.0f, flags, st, s, nullptr, 0, 0, nullptr, 0, false);
     if (status) break;
     cudaEventRecord(e0, st);
-    status = adjoint_impl(p, coef, img_scratch, 1.0f, flags, st, s);
+    status = adjoint_impl(p, coef, img_scratch, 1.0f, flags, st, s, nullptr, 0, 0, nullptr, 0, false);
     cudaEventRecord(e1, st);
     if (cudaEventSynchronize(e1) != cudaSuccess) { status = cuda_fail(cudaGetLastError(), "viss_plan_tune"); break; }
     float ms = 0;

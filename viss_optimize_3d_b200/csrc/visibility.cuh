@@ -10,6 +10,8 @@ constexpr int kSampTile = 128;  // samples per adjoint staging tile
 constexpr int kFwdStages = 3;   // shared-memory ring depth: forward pixel tiles
 constexpr int kAdjStages = 4;   // shared-memory ring depth: adjoint sample tiles
 
+constexpr int kTrackT = 128;    // samples per track block (tracks.cu)
+
 struct FwdParams {
   const double4 *samp;   // [K] (u, v, w, off)
   const int4 *refs;      // [K] occulter rows or null

@@ -199,6 +199,19 @@ __device__ __forceinline__ void sfu_sincos(float a, float &s, float &c) {
   asm("cos.approx.ftz.f32 %0, %1;" : "=f"(c) : "f"(a));
 }
 
+// Kahan-compensated add of x into (s, c).
+__device__ __forceinline__ void kahan_add(float &s, float &c, float x) {
+  const float y = __fsub_rn(x, c);
+  const float t = __fadd_rn(s, y);
+  c = __fsub_rn(__fsub_rn(t, s), y);
+  s = t;
+}
+
+// Sky value of a pixel + sky record (the low word of .w).
+__device__ __forceinline__ float sky_of(const double4 &p) {
+  return __int_as_float(__double2loint(p.w));
+}
+
 // Exact-op-order dot product used by the occultation predicate (the oracle
 // evaluates the same IEEE operations).
 __device__ __forceinline__ double dot_exact(double s0, double s1, double s2, const double4 &q) {
