@@ -4,13 +4,14 @@ numpy on synthetic formation tracks.
 A block's nodes are picked by a Cholesky factorisation of the correlation
 sinc(2 rho |u - u'|), pivoted on the worst predicted sample, until the mean
 squared error of the weights -- interpolation and independent node errors of
-3e-7 together -- is below 0.7 (3e-7)^2."""
+2e-7 together -- is below 1.8 (2e-7)^2."""
 import numpy as np
 import pytest
 
 from viss_optimize_3d_b200 import synth
 
-NOISE = 3e-7
+NOISE = 2e-7          # relative error of a node value
+EVALUATED = 3.7e-7    # of an exponential term of the direct kernels
 T = 128
 
 
@@ -18,7 +19,7 @@ def nodes_and_weights(u, rho):
     n = len(u)
     G = np.sinc(2 * rho * np.linalg.norm(u[:, None] - u[None], axis=2))
     L, diag, used, piv, ld = np.zeros((n, n)), np.ones(n), np.zeros(n, bool), [], []
-    while diag.max() > 2 * NOISE ** 2 or diag.mean() > 0.7 * NOISE ** 2:
+    while diag.max() > 4.5 * NOISE ** 2 or diag.mean() > 1.8 * NOISE ** 2:
         r = len(piv)
         if r == n * 3 // 4:
             return None, None
@@ -26,6 +27,8 @@ def nodes_and_weights(u, rho):
         d = 1.0 - L[p, :r] @ L[p, :r]
         ld.append(np.sqrt(max(d, 0.0) + NOISE ** 2))
         L[:, r] = (G[:, p] - L[:, :r] @ L[p, :r]) / ld[-1]
+        if r == 0 and np.all(G[:, p] == 1.0):           # one point: one node
+            return [p], L[:, :1] / ld[-1]
         diag = np.maximum(diag - L[:, r] ** 2, 0.0)
         used[p] = True
         piv.append(p)
@@ -65,17 +68,16 @@ def test_predicted_samples_are_as_accurate_as_evaluated_ones(name, pixels):
         bias.append(np.sqrt(np.mean(np.abs(err) ** 2) / np.sum(sky ** 2)))
         noise.append(np.mean(np.sum(W ** 2, axis=1)))
     assert len(ranks) >= 3
-    # fewer nodes than samples; the weights pass on no more node error than a
-    # node has, and their own error is a fraction of it
+    # fewer nodes than samples, and a predicted sample (its weights' own error and
+    # the nodes' together) no further off than an evaluated one
     assert max(ranks) <= T // 2 and np.mean(ranks) < 0.45 * T, ranks
-    assert max(noise) < 1.0 and max(bias) < NOISE / 2, (noise, bias)
+    total = [np.hypot(e, NOISE * np.sqrt(n)) for e, n in zip(bias, noise)]
+    assert max(total) < EVALUATED, (noise, bias)
 
 
-def test_equal_samples_share_two_nodes():
-    """Zero baselines: every sample is the same, two nodes halve the node error,
-    and each sample's two FP32 weights add up to one to FP32 rounding (how they
-    share it is open: the two nodes are the same), so sums of ones up to the
-    largest pixel counts still round to the right integer."""
+def test_equal_samples_take_one_node():
+    """Zero baselines: every sample is the same; one node whose FP32 weights are
+    exactly one, so that sums of ones stay exact integers."""
     piv, W = nodes_and_weights(np.zeros((T, 3)), 0.05)
-    assert len(piv) == 2
-    assert np.abs(W.astype(np.float32).astype(np.float64).sum(axis=1) - 1).max() <= 2.0 ** -24
+    assert len(piv) == 1
+    assert np.all(W.astype(np.float32) == np.float32(1.0))

@@ -42,7 +42,7 @@ cudaError_t launch_form_reduce_fwd(long long, int, const double2 *, const double
                                    cudaStream_t);
 cudaError_t launch_stage_sky(long long, long long, const double4 *, const int *, const float *,
                              float, double4 *, int, cudaStream_t);
-cudaError_t launch_stage_coef(long long, long long, const float2 *, float2 *, cudaStream_t);
+cudaError_t launch_stage_coef(long long, long long, const float2 *, float2 *, bool, cudaStream_t);
 cudaError_t launch_stage_samples(long long, const double *, const double *, const int32_t *,
                                  long long, double4 *, int4 *, unsigned long long *, int *,
                                  cudaStream_t);
@@ -544,7 +544,7 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
   p->drop_tile = -1;
   VISS_CUDA(viss::launch_forward(fp, shape, real_chunks, masked, fp64, st), "viss_forward: kernel");
   VISS_CUDA(viss::launch_reduce_fwd(p->K, real_chunks, fp.part, reinterpret_cast<float2 *>(V),
-                                    (flags & VISS_ACCUMULATE) ? 1 : 0, st),
+                                    (flags & VISS_ACCUMULATE) ? 1 : 0, fp64, st),
             "viss_forward: reduce");
   p->last_total = p->K * p->J;
   p->last_stream = st;
@@ -585,14 +585,14 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
   const int nchunk = adj_chunks(p, shape, fp64, &spc);
   if (int s = workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * p->channels * p->Jpad))
     return s;
-  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, st),
+  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, !fp64, st),
             "viss_adjoint: coef");
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint");
   bool use = false;
   if (tracks && !fp64 && !fcones)
     if (int s = tracks_ready(p, st, &use)) return s;
   if (use) {
-    const int s = viss::tracks_adjoint(p->tracks, track_inputs(p), p->coef, image, scale, masked,
+    const int s = viss::tracks_adjoint(p->tracks, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
                                        !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                        reinterpret_cast<int *>(p->dev_words + 1), p->drop_tile, st);
     if (s != VISS_ERR_ALLOC) {
@@ -888,7 +888,7 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   const long long max_cells = 1LL << 29;   // 4 GiB of FP32 complex grid
   long long fp = facet_pixels, info = 0;
   const cudaStream_t st = as_stream(stream);
-  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, st),
+  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, false, st),
             "viss_adjoint_gridded: coef");
   const float4 *fcones = nullptr;
   const unsigned *mixbits = nullptr;

@@ -352,17 +352,19 @@ cudaError_t launch_stage_sky(long long J, long long Jpad, const double4 *pix, co
 }
 
 // Coefficient staging for the adjoint: a 16-byte aligned copy padded to an
-// even count (bulk copies move whole 16-byte units).
-__global__ void k_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out) {
+// even count (bulk copies move whole 16-byte units); biased: for k_adjoint's
+// split-precision terms.
+__global__ void k_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out, int biased) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= Kpad) return;
-  out[i] = i < K ? coef[i] : make_float2(0.f, 0.f);
+  const float2 a = i < K ? coef[i] : make_float2(0.f, 0.f);
+  out[i] = biased ? unbias_coef(a) : a;
 }
 
 cudaError_t launch_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out,
-                              cudaStream_t st) {
+                              bool biased, cudaStream_t st) {
   if (Kpad <= 0) return cudaSuccess;
-  k_stage_coef<<<nblk(Kpad, 256), 256, 0, st>>>(K, Kpad, coef, out);
+  k_stage_coef<<<nblk(Kpad, 256), 256, 0, st>>>(K, Kpad, coef, out, biased ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -222,7 +222,7 @@ extern "C" int viss_forward_noalloc(int64_t J, const double *lmn, const float *s
   fp.drop_tile = viss::take_noalloc_drop_tile();
   if ((e = viss::launch_forward(fp, shape, real_chunks, refs != nullptr, false, st)) != cudaSuccess)
     return na_cuda(e, "forward kernel");
-  if ((e = viss::launch_reduce_fwd(K, real_chunks, part, reinterpret_cast<float2 *>(V), 0, st)) !=
+  if ((e = viss::launch_reduce_fwd(K, real_chunks, part, reinterpret_cast<float2 *>(V), 0, false, st)) !=
       cudaSuccess)
     return na_cuda(e, "reduce");
   // the kernel's error word: a bounded staging wait that gave up leaves V

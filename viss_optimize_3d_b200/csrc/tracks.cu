@@ -22,10 +22,14 @@
 // sinc(2 rho |u - u'|).  A Cholesky factorisation of that matrix, pivoted on
 // the sample that the nodes so far predict worst, picks the nodes; P is the
 // least-squares predictor for node values that carry an independent relative
-// error of kNodeNoise (that of one SFU exponential, 3e-7).  A block stops when
-// its mean squared prediction error, node errors included, is below 0.7
-// kNodeNoise^2 (no sample above 2): a predicted value is then no further off
-// than an evaluated one.  Blocks that need more than kTrackRankMax nodes, or
+// error of kNodeNoise = 2e-7 (1.7e-7 of one node exponential, and FP32 sums).  A
+// block stops when its mean squared prediction error, node errors included, is
+// below 1.8 kNodeNoise^2 (no sample above 4.5): (2.7e-7)^2, where a term that
+// k_forward evaluates is off by 3.7e-7 (a phase of 23 bits).  Measured against
+// FP64 on 1 and 10 MHz Nside 256 observations: V 2.6e-7 - 3.7e-7 and images of
+// random coefficients 4.2e-7, the direct kernels 3.6e-7 - 5.2e-7 and 5.6e-7.
+// Stopping at 0.85 (3e-7)^2 with the same node error costs 25 % more nodes
+// for 8 % less error, stopping at 2.5 saves 1 %.  Blocks that need more than kTrackRankMax nodes, or
 // three quarters of their samples, are left to the remainder kernels.
 //
 // Group size.  Long baselines turn faster: every block takes the group size
@@ -76,6 +80,18 @@ struct TrackNodeParams {
 // Node sums are stored per unit: a half tile (2 t + h) in the 64-pixel class, else
 // a tile; a merged group's sum stands at its first tile.
 namespace {
+
+// Angle of t = kTurn32 + phase, |phase| < 2^19 turns: its low 32 bits are the
+// phase's fraction in 2^-32 turn, as a signed integer in [-1/2, 1/2) turn, so the
+// conversion and one product give the angle to FP32 rounding, in as many
+// instructions as turn_angle (whose 23-bit fraction covers 2^28 turns) and in the
+// same time: exponentials 1.7e-7 off instead of 3.7e-7, so fewer nodes will do
+// (with turn_angle the 10 MHz forward took 68.4 ms and the adjoint 78.7 ms
+// instead of 54 and 67).
+constexpr double kTurn32 = 1572864.0;            // 1.5 * 2^20
+__device__ __forceinline__ float turn_angle32(double t) {
+  return static_cast<float>(__double2loint(t)) * 1.46291807926716e-9f;
+}
 
 constexpr int kNodeNT = 256;
 constexpr int kNodeR = 4;
@@ -167,7 +183,7 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
         for (int r = 0; r < R; ++r) t_re[r] = t_im[r] = 0.f;
         auto term = [&](int r, const double4 &q, float I, double magic) {
           float sn, cs;
-          sfu_sincos(turn_angle(fma(uz[r], q.z, fma(uy[r], q.y, fma(ux[r], q.x, magic)))), sn, cs);
+          sfu_sincos(turn_angle32(fma(uz[r], q.z, fma(uy[r], q.y, fma(ux[r], q.x, magic)))), sn, cs);
           t_re[r] = fmaf(I, cs, t_re[r]);
           t_im[r] = fmaf(-I, sn, t_im[r]);
         };
@@ -177,8 +193,8 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
             const float I0 = sky_of(q0), I1 = -sky_of(q1);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              term(r, q0, I0, kMagic);
-              term(r, q1, I1, kMagic + 0.5);         // odd records half a turn on (k_forward)
+              term(r, q0, I0, kTurn32);
+              term(r, q1, I1, kTurn32 + 0.5);         // odd records half a turn on (k_forward)
             }
           }
         } else {
@@ -188,8 +204,8 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
 #pragma unroll 4
             for (int j = 0; j < kSpan; j += 2) {
               const double4 q0 = tp[j], q1 = tp[j + 1];
-              term(r, q0, sky_of(q0), kMagic);
-              term(r, q1, -sky_of(q1), kMagic + 0.5);
+              term(r, q0, sky_of(q0), kTurn32);
+              term(r, q1, -sky_of(q1), kTurn32 + 0.5);
             }
           }
         }
@@ -516,13 +532,14 @@ __global__ void k_track_reduce_fwd(long long n, long long first, const int *slot
   const long long k = slot[first + i];
   if (k < 0) return;
   double re = 0, im = 0;
-  for (int c = 0; c < nv; ++c) {
-    const double2 v = vacc[c * vstride + i];
+  for (int c = 0; c < nchunk; ++c) {
+    const double2 v = part[static_cast<long long>(c) * Ks + first + i];
     re += v.x;
     im += v.y;
   }
-  for (int c = 0; c < nchunk; ++c) {
-    const double2 v = part[static_cast<long long>(c) * Ks + first + i];
+  unbias(re, im);                                  // evaluated terms; the interpolated ones are
+  for (int c = 0; c < nv; ++c) {
+    const double2 v = vacc[c * vstride + i];
     re += v.x;
     im += v.y;
   }
@@ -724,7 +741,7 @@ __global__ void __launch_bounds__(kRestNT, 6) k_track_adj_rest(const TrackRestPa
           double4 u = p.samp[i];
           u.w = kMagic + (p.use_off ? u.w : 0.0);
           L.u[at] = u;
-          L.c[at] = p.coef[i];
+          L.c[at] = unbias_coef(p.coef[i]);
           L.meta[at] = meta;
           if (meta >> 8) exact_rows(p.occ, i0, i1, i2, L.q[0][at], L.q[1][at], L.q[2][at]);
         }
@@ -998,7 +1015,7 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
   }
   __syncthreads();
   const bool odd_lane = (lane & 1) != 0;             // half a turn on, negated at the end (k_adjoint)
-  const double magic = odd_lane ? kMagic + 0.5 : kMagic;
+  const double magic = odd_lane ? kTurn32 + 0.5 : kTurn32;
   unsigned long long evaluated = 0;
   int next = 0;
   for (int it = 0; it < ntile; ++it) {
@@ -1033,7 +1050,7 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
     for (int q = 0; q < P; ++q) acc[q] = 0.f;
     auto term = [&](int q, const double4 &u, const float2 &c) {
       float sn, cs;
-      sfu_sincos(turn_angle(fma(u.z, sz[q], fma(u.y, sy[q], fma(u.x, sx[q], magic)))), sn, cs);
+      sfu_sincos(turn_angle32(fma(u.z, sz[q], fma(u.y, sy[q], fma(u.x, sx[q], magic)))), sn, cs);
       acc[q] = fmaf(-c.y, sn, fmaf(c.x, cs, acc[q]));
     };
 #pragma unroll 1

@@ -13,7 +13,7 @@ namespace viss {
 
 namespace {
 
-constexpr double kNodeNoise2 = 9e-14;            // kNodeNoise^2
+constexpr double kNodeNoise2 = 4e-14;            // kNodeNoise^2
 constexpr int kLagMax = 1024;                    // tracks interleaved in the caller's order, at most
 constexpr int kLagSamples = 128;
 constexpr int kRankSamples = 48;                 // blocks that decide whether nodes pay at all
@@ -143,7 +143,7 @@ __device__ int track_factor(TrackFactor &f, bool valid, const double4 &u, double
     key = max(max(f.best[0], f.best[1]), max(f.best[2], f.best[3]));
     sum = (f.sum[0] + f.sum[1]) + (f.sum[2] + f.sum[3]);
     top = fmax(fmax(f.top[0], f.top[1]), fmax(f.top[2], f.top[3]));
-    if (top <= 2.0 * kNodeNoise2 && sum <= 0.7 * kNodeNoise2 * nvalid) return r;
+    if (top <= 4.5 * kNodeNoise2 && sum <= 1.8 * kNodeNoise2 * nvalid) return r;
     if (r >= cap || key == 0) return 0;
     const int p = static_cast<int>(key & 127u);
     const double dx = u.x - f.u[0][p], dy = u.y - f.u[1][p], dz = u.z - f.u[2][p];
@@ -154,6 +154,12 @@ __device__ int track_factor(TrackFactor &f, bool valid, const double4 &u, double
     const double ld = sqrt(d + kNodeNoise2);
     const double l = valid ? c / ld : 0.0;
     f.L[r * kTrackT + k] = l;
+    if (r == 0 && __syncthreads_and(!valid || x <= 1e-9)) {
+      // one point (zero baselines): one node, whose weights are one exactly
+      if (k == p) f.piv[0] = static_cast<unsigned char>(p), f.ld[0] = ld;
+      __syncthreads();
+      return 1;
+    }
     diag = fmax(fma(-l, l, diag), 0.0);
     if (k == p) {
       used = true;

@@ -268,9 +268,10 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
   }
 }
 
-// V_k = sum over chunks (FP64) -> complex64, optionally accumulated.
+// V_k = sum over chunks (FP64) -> complex64, optionally accumulated; biased: of
+// split-precision terms.
 __global__ void k_reduce_fwd(long long K, int nchunk, const double2 *part, float2 *V,
-                             int accumulate) {
+                             int accumulate, int biased) {
   const long long k = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= K) return;
   double re = 0, im = 0;
@@ -279,6 +280,7 @@ __global__ void k_reduce_fwd(long long K, int nchunk, const double2 *part, float
     re += v.x;
     im += v.y;
   }
+  if (biased) unbias(re, im);
   if (accumulate) {
     const float2 o = V[k];
     re += o.x;
@@ -579,9 +581,9 @@ int forward_ctas_per_sm(int shape, bool fp64) {
 }
 
 cudaError_t launch_reduce_fwd(long long K, int nchunk, const double2 *part, float2 *V, int acc,
-                              cudaStream_t st) {
+                              bool fp64, cudaStream_t st) {
   if (K <= 0) return cudaSuccess;
-  k_reduce_fwd<<<static_cast<unsigned>((K + 255) / 256), 256, 0, st>>>(K, nchunk, part, V, acc);
+  k_reduce_fwd<<<static_cast<unsigned>((K + 255) / 256), 256, 0, st>>>(K, nchunk, part, V, acc, fp64 ? 0 : 1);
   return cudaGetLastError();
 }
 

@@ -117,7 +117,7 @@ cudaError_t launch_forward(const FwdParams &p, int shape, int nchunk, bool maske
 int forward_samples_per_block(int shape, bool fp64);
 int forward_ctas_per_sm(int shape, bool fp64);
 cudaError_t launch_reduce_fwd(long long K, int nchunk, const double2 *part, float2 *V, int acc,
-                              cudaStream_t st);
+                              bool fp64, cudaStream_t st);
 // The occulted split-precision adjoint without the pairs whose facet is
 // wholly visible to the sample (p.fcones, p.facet_pix, p.nfacets set).
 cudaError_t launch_adjoint_hybrid(const AdjParams &p, int shape, int nchunk, cudaStream_t st);

@@ -184,11 +184,29 @@ __device__ __forceinline__ void ring_drain(uint64_t *full, int next) {
 // mantissa bits of t are frac(phase + 1/2) in units of 2^-23 turn; placed
 // under the exponent of 1.0f (one LOP3: (lo & 0x7fffff) | 0x3f800000) they
 // give f in [1, 2), and 2 pi f - 3 pi is the phase reduced mod one turn.
+//
+// The FP32 rounding of 2 pi f - 3 pi (6.2831855f f - 9.424778f) puts the angle
+// kAngleBias radians ahead at the middle of the range, f = 1.5 (at most 9e-8
+// around that elsewhere).  Every term of a sum shares it, so it does not
+// average out: sums of e^{-i angle} are turned back once at their end
+// (unbias), coefficients that multiply e^{+i angle} once beforehand.
+constexpr double kAngleBias = 2.384185791e-07;
 __device__ __forceinline__ float turn_angle(double t) {
   const uint32_t lo = static_cast<uint32_t>(__double2loint(t));
   uint32_t bits;
   asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(bits) : "r"(lo), "r"(0x007fffffu), "r"(0x3f800000u));
   return fmaf(__uint_as_float(bits), 6.28318530717958648f, -9.42477796076937972f);
+}
+
+// z e^{+i kAngleBias} of a sum of e^{-i angle} terms.
+__device__ __forceinline__ void unbias(double &re, double &im) {
+  const double r = re;
+  re = fma(-kAngleBias, im, re);
+  im = fma(kAngleBias, r, im);
+}
+// a e^{-i kAngleBias} of a coefficient of e^{+i angle}.
+__device__ __forceinline__ float2 unbias_coef(float2 a) {
+  return make_float2(fmaf(static_cast<float>(kAngleBias), a.y, a.x), fmaf(-static_cast<float>(kAngleBias), a.x, a.y));
 }
 
 // SFU sine and cosine of an angle in [-pi, pi) (flush-to-zero variants: the
