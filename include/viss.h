@@ -170,6 +170,9 @@ int viss_plan_tune(viss_plan *plan, const float *sky, const float *coef, float *
  * frequency grid in the facet's local frame ("exponential of semicircle"
  * kernel, width 7, oversampling 2), one FFT (cuFFT, oversampling 1.5),
  * interpolation at its pixels (width 9).
+ * With facet_pixels = 0 and samples on smooth tracks, track blocks (see
+ * viss_forward) make the image instead where they are modelled faster; the
+ * facet choice is reported all the same.
  * Unmasked (VISS_NO_MASK, or no occulter refs): computeC of the noblockage
  * programs (vissgen3d_noblockage.cu:167-182), every sample gridded.
  * Occulted: computeC of the blockage programs (vissgen3d_blockage.cu:167-192)

@@ -125,3 +125,70 @@ def test_restaged_samples_and_captured_calls(cuda_device):
     graph.replay()
     torch.cuda.synchronize()
     close(out, want)
+
+
+@pytest.mark.parametrize("n_sat,n_snap,channels,rows", [
+    (10, 4801, 1, ("moon", "earth")),
+    (3, 24000, 3, ("earth",)),              # one occulter kind only, channels
+    (4, 35011, 1, ()),                      # few satellites, nothing occulted
+])
+def test_formation_pairs(cuda_device, n_sat, n_snap, channels, rows):
+    """Formation calls whose pairs lie on dense tracks, against the FP64 direct
+    kernels on the pairs' baselines and rows."""
+    nside, f_hz = 64, 1e6
+    obs = observation(nside, n_sat, n_snap, f_hz, True, True)
+    lmn = api.pix2lmn(nside, "ring", device=cuda_device)
+    T, S, B = n_snap, n_sat, n_sat * (n_sat - 1) // 2
+    P = torch.as_tensor(obs.positions, device=cuda_device)
+    U = (P - P.mean(dim=1, keepdim=True)) / (synth.C_LIGHT / f_hz)
+    U = torch.stack([U * (1 + 0.2 * c) for c in range(channels)])
+    _, occ = tables(obs, cuda_device)
+    refs = torch.as_tensor(obs.refs, device=cuda_device).clone()
+    if "moon" not in rows:
+        refs[:, :2] = -1
+    if "earth" not in rows:
+        refs[:, 2] = -1
+    g = torch.Generator(device=cuda_device).manual_seed(6)
+    off = torch.rand(channels * T * B, generator=g, device=cuda_device, dtype=torch.float64)
+    a, b = (torch.as_tensor(obs.pairs[:, i].astype(np.int64), device=cuda_device) for i in (0, 1))
+    uvw = (U[:, :, a] - U[:, :, b]).reshape(-1, 3)
+    plan = api.Plan(lmn, uvw, off, refs.repeat(channels, 1), occ, channels=channels)
+    plan.set_formation(U if channels > 1 else U[0], off.view(channels, T, B) if channels > 1 else off.view(T, B),
+                       occ[:T * S].view(T, S, 4) if "moon" in rows else None,
+                       occ[T * S:] if "earth" in rows else None)
+    sky = torch.rand(channels * plan.J, generator=g, device=cuda_device) + 0.1
+    coef = torch.randn(plan.K, generator=g, device=cuda_device, dtype=torch.complex64)
+    assert plan.K * plan.J >= 1e10
+    for kw in (dict(), dict(mask=False), dict(use_offset=False)):
+        close(plan.forward_formation(sky, **kw), plan.forward(sky, fp64=True, **kw))
+        close(plan.adjoint_formation(coef, **kw), plan.adjoint(coef, fp64=True, **kw))
+    acc = plan.forward_formation(sky)
+    plan.forward_formation(sky, out=acc, accumulate=True)
+    close(acc, 2 * plan.forward(sky, fp64=True))
+
+
+def test_gridded_call_through_the_blocks(cuda_device):
+    """The gridded entry point with its own choice of facets: blocks where they
+    are modelled faster, reporting that choice; an explicit facet size grids; a
+    NaN coefficient is refused either way."""
+    from viss_optimize_3d_b200 import _capi
+    obs = observation(64, 8, 7600, 1e6, True, True)
+    lmn = api.pix2lmn(64, "ring", device=cuda_device)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(lmn, torch.as_tensor(obs.uvw(1e6), device=cuda_device), None, refs, occ)
+    g = torch.Generator(device=cuda_device).manual_seed(8)
+    coef = torch.randn(plan.K, generator=g, device=cuda_device, dtype=torch.complex64)
+    for kw in (dict(), dict(mask=False)):
+        want = plan.adjoint(coef, fp64=True, **kw)
+        close(plan.adjoint_gridded(coef, **kw), want)
+        info = plan.gridded_info()
+        assert info["facet_pixels"] >= 64 and min(info["grid"]) >= 16
+        got = plan.adjoint_gridded(coef, facet_pixels=256, **kw)
+        assert float((got - want).double().norm() / want.double().norm()) < 1e-5
+        base = torch.ones(plan.J, device=cuda_device)
+        close(plan.adjoint_gridded(coef, out=base, accumulate=True, **kw) - 1, want)
+    bad = coef.clone()
+    bad[7] = complex(float("nan"), 0.0)
+    with pytest.raises(_capi.VissError, match="non-finite"):
+        plan.adjoint_gridded(bad, mask=False)
+    close(plan.adjoint_gridded(coef, mask=False), plan.adjoint(coef, fp64=True, mask=False))

@@ -58,8 +58,11 @@ int gridded_adjoint(void **state, long long J, const double4 *pix, const int *pe
                     float *img, int accumulate, long long max_cells, cudaStream_t st, int *grid_dims,
                     long long *facet_used, long long *info, const int4 *refs, const float4 *occ32,
                     const float4 **fcones_out, const unsigned **mixbits_out, long long *mix_words_out,
-                    long long geom_version);
+                    long long geom_version, double other_seconds);
 void gridded_free(void *state);
+cudaError_t launch_pair_samples(long long T, int S, const double4 *U, const double *off, int sat_rows, int snap_rows,
+                                double4 *samp, int4 *refs, cudaStream_t st);
+cudaError_t launch_nonfinite(long long n, const float2 *v, unsigned long long *flag, cudaStream_t st);
 }  // namespace viss
 
 #include "tracks.cuh"
@@ -186,6 +189,13 @@ struct viss_plan {
   void *tracks = nullptr;
   long long tracks_version = -1;
   bool tracks_usable = false;
+  // the same for the formation's pairs, as samples u = U_a - U_b
+  void *form_tracks = nullptr;
+  long long form_version = 0, form_tracks_version = -1;
+  bool form_tracks_usable = false;
+  double form_turns = 0;        // bound on |U.s| and |off|
+  double4 *form_samp = nullptr; size_t form_samp_cap = 0;
+  int4 *form_refs = nullptr;    size_t form_refs_cap = 0;
 };
 
 namespace {
@@ -357,17 +367,18 @@ int viss_plan_destroy(viss_plan *p) {
   void *bufs[] = {p->pix,    p->pixsky,  p->cones,    p->perm,      p->samp,
                   p->refs,   p->occ,     p->occ32,    p->coef,      p->part,
                   p->dev_words, p->form_U, p->form_off, p->form_occ, p->form_occ32,
-                  p->form_coef};
+                  p->form_coef, p->form_samp, p->form_refs};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->gridded) viss::gridded_free(p->gridded);
   if (p->tracks) viss::tracks_free(p->tracks);
+  if (p->form_tracks) viss::tracks_free(p->form_tracks);
   delete p;
   return VISS_OK;
 }
 
 int viss_plan_set_pixels(viss_plan *p, int64_t J, const double *lmn, void *stream) {
-  if (p) ++p->geom_version;
+  if (p) ++p->geom_version, ++p->form_version;
   if (!p || J <= 0 || !lmn) return fail(VISS_ERR_ARG, "viss_plan_set_pixels: bad arguments");
   if (J > (1LL << 31) * viss::kTilePix / 2)
     return fail(VISS_ERR_ARG, "viss_plan_set_pixels: too many pixels");
@@ -476,15 +487,19 @@ static viss::TrackInputs track_inputs(const viss_plan *p) {
 // Not under stream capture: a captured call is replayed after the samples were
 // staged again, and the blocks' launch sizes depend on the samples.
 constexpr double kTrackMinTerms = 1e10;
-static int tracks_ready(viss_plan *p, cudaStream_t st, bool *use) {
-  *use = false;
-  if (static_cast<double>(p->K) * p->J < kTrackMinTerms) return VISS_OK;
+static bool tracks_allowed(double terms, cudaStream_t st) {
+  if (terms < kTrackMinTerms) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
     cudaGetLastError();
-    return VISS_OK;
+    return false;
   }
-  if (cap != cudaStreamCaptureStatusNone) return VISS_OK;
+  return cap == cudaStreamCaptureStatusNone;
+}
+
+static int tracks_ready(viss_plan *p, cudaStream_t st, bool *use) {
+  *use = false;
+  if (!tracks_allowed(static_cast<double>(p->K) * p->J, st)) return VISS_OK;
   if (p->tracks_version != p->geom_version) {
     bool ok = false;
     if (int s = viss::tracks_build(&p->tracks, track_inputs(p), st, &ok)) return s;
@@ -711,6 +726,7 @@ int viss_plan_set_channels(viss_plan *p, int channels) {
 // -------------------------------------------------------- formation mode
 int viss_plan_set_formation(viss_plan *p, int64_t T, int S, const double *U, const double *off,
                             const double *occ_sat, const double *occ_snap, void *stream) {
+  if (p) ++p->form_version;
   if (!p || T < 1 || !U) return fail(VISS_ERR_ARG, "viss_plan_set_formation: bad arguments");
   if (S < 2 || S > 10)
     return fail(VISS_ERR_ARG, "viss_plan_set_formation: S must be 2 to 10 satellites");
@@ -753,6 +769,7 @@ int viss_plan_set_formation(viss_plan *p, int64_t T, int S, const double *U, con
   p->form_T = T;
   p->form_S = S;
   p->form_C = 1;
+  p->form_turns = bound;
   p->form_has_off = off != nullptr;
   p->form_sat = occ_sat != nullptr;
   p->form_snap = occ_snap != nullptr;
@@ -760,6 +777,7 @@ int viss_plan_set_formation(viss_plan *p, int64_t T, int S, const double *U, con
 }
 
 int viss_plan_set_formation_channels(viss_plan *p, int channels) {
+  if (p) ++p->form_version;
   if (!p || channels < 1) return fail(VISS_ERR_ARG, "viss_plan_set_formation_channels: bad arguments");
   if (p->form_T <= 0) return fail(VISS_ERR_STATE, "viss_plan_set_formation_channels: formation not set");
   if (p->form_T % channels != 0)
@@ -797,6 +815,49 @@ static viss::FormParams form_params(viss_plan *p, int flags) {
   return fp;
 }
 
+static viss::TrackInputs form_track_inputs(const viss_plan *p) {
+  viss::TrackInputs in = track_inputs(p);
+  const long long B = viss::form_pairs(p->form_S);
+  in.samp = p->form_samp;
+  in.refs = (p->form_sat || p->form_snap) ? p->form_refs : nullptr;
+  in.occ = p->form_occ;
+  in.occ32 = p->form_occ32;
+  in.K = p->form_T * B;
+  in.Kc = p->form_T / p->form_C * B;
+  in.channels = p->form_C;
+  in.max_turns = 3.0 * p->form_turns;              // |U_a.s| + |U_b.s| + |off|
+  return in;
+}
+
+// Whether a formation call goes through track blocks of its pairs (u = U_a -
+// U_b, the same rows): when they are modelled faster than the formation kernels'
+// `per_term` seconds (forward 3.07e-13, adjoint 2.43e-13 at S = 10, Nside 256 x 388,800 samples,
+// Moon + Earth, per sample and pixel; measured 94.1 against 54 ms and 74.5
+// against 67 ms at 10 MHz).  Per pair S exponentials serve S - 1 / 2: with fewer
+// satellites a pair costs the formation kernels more, which only favours the blocks.
+static int form_tracks_ready(viss_plan *p, bool masked, double per_term, cudaStream_t st, bool *use) {
+  *use = false;
+  const long long K = p->form_T * viss::form_pairs(p->form_S);
+  if (!tracks_allowed(static_cast<double>(K) * p->J, st) || !(3.0 * p->form_turns < 262144.0)) return VISS_OK;
+  if (p->form_tracks_version != p->form_version) {
+    const bool rows = p->form_sat || p->form_snap;
+    if (ensure(p->form_samp, p->form_samp_cap, sizeof(double4) * K, "formation samples") ||
+        (rows && ensure(p->form_refs, p->form_refs_cap, sizeof(int4) * K, "formation samples")))
+      return VISS_OK;                              // without that memory: the formation kernels
+    VISS_CUDA(viss::launch_pair_samples(p->form_T, p->form_S, p->form_U, p->form_has_off ? p->form_off : nullptr,
+                                        p->form_sat, p->form_snap, p->form_samp, rows ? p->form_refs : nullptr, st),
+              "formation samples");
+    bool ok = false;
+    if (int s = viss::tracks_build(&p->form_tracks, form_track_inputs(p), st, &ok)) return s;
+    p->form_tracks_usable = ok;
+    p->form_tracks_version = p->form_version;
+  }
+  const viss::TrackInputs in = form_track_inputs(p);
+  *use = p->form_tracks_usable &&
+         viss::tracks_seconds(p->form_tracks, in, masked) < 0.95 * per_term * static_cast<double>(in.K) * in.J;
+  return VISS_OK;
+}
+
 int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, void *stream) {
   if (int s = check_formation(p, sky, V, flags, "viss_forward_formation")) return s;
   const NvtxRange range("viss_forward_formation");
@@ -819,6 +880,19 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
   VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky, C, st),
             "viss_forward_formation: sky");
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_forward_formation");
+  bool use = false;
+  const bool masked = (fp.sat_rows || fp.snap_rows);
+  if (int s = form_tracks_ready(p, masked, 3.07e-13, st, &use)) return s;
+  if (use) {
+    const int s = viss::tracks_forward(p->form_tracks, form_track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V),
+                                       masked, !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
+                                       reinterpret_cast<int *>(p->dev_words + 1), -1, st);
+    if (s != VISS_ERR_ALLOC) {
+      p->last_total = T * B * p->J;
+      p->last_stream = st;
+      return s;
+    }
+  }
   fp.pix = p->pixsky;
   fp.part_fwd = static_cast<double2 *>(p->part);
   VISS_CUDA(viss::launch_form_forward(fp, p->form_S, nchunk, st), "viss_forward_formation: kernel");
@@ -859,6 +933,20 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
   if (int s = workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * C * p->Jpad)) return s;
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint_formation");
   viss::FormParams fp = form_params(p, flags);
+  bool use = false;
+  const bool masked = (fp.sat_rows || fp.snap_rows);
+  if (int s = form_tracks_ready(p, masked, 2.43e-13, st, &use)) return s;
+  if (use) {
+    const int s = viss::tracks_adjoint(p->form_tracks, form_track_inputs(p), reinterpret_cast<const float2 *>(coef),
+                                       image, scale, masked, !(flags & VISS_NO_OFFSET),
+                                       (flags & VISS_ACCUMULATE) != 0, p->dev_words,
+                                       reinterpret_cast<int *>(p->dev_words + 1), -1, st);
+    if (s != VISS_ERR_ALLOC) {
+      p->last_total = T * B * p->J;
+      p->last_stream = st;
+      return s;
+    }
+  }
   fp.pix = p->pix;
   fp.snaps_per_chunk = static_cast<int>(spc);
   fp.nchunk = nchunk;
@@ -893,14 +981,46 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   const float4 *fcones = nullptr;
   const unsigned *mixbits = nullptr;
   long long mix_words = 0;
-  const int s = viss::gridded_adjoint(&p->gridded, p->J, p->pix, p->perm, p->K, p->samp, p->coef,
+  // with the library's choice of facets, track blocks where they are modelled
+  // faster (not for non-finite coefficients, which gridding reports)
+  double other = 0;
+  if (facet_pixels == 0) {
+    bool use = false;
+    if (int s = tracks_ready(p, st, &use)) return s;
+    if (use) {
+      VISS_CUDA(cudaMemsetAsync(p->dev_words + 3, 0, sizeof(unsigned long long), st), "viss_adjoint_gridded");
+      VISS_CUDA(viss::launch_nonfinite(p->K, reinterpret_cast<const float2 *>(coef), p->dev_words + 3, st),
+                "viss_adjoint_gridded: coefficients");
+      unsigned long long bad = 0;
+      VISS_CUDA(cudaMemcpyAsync(&bad, p->dev_words + 3, sizeof(bad), cudaMemcpyDeviceToHost, st), "viss_adjoint_gridded");
+      VISS_CUDA(cudaStreamSynchronize(st), "viss_adjoint_gridded");
+      if (!bad) other = viss::tracks_seconds(p->tracks, track_inputs(p), masked);
+    }
+  }
+  int s = viss::gridded_adjoint(&p->gridded, p->J, p->pix, p->perm, p->K, p->samp, p->coef,
                                       (flags & VISS_NO_OFFSET) ? 0 : 1, fp, scale, image,
                                       (flags & VISS_ACCUMULATE) ? 1 : 0, max_cells, st, p->gridded_dims, &fp,
                                       &info, masked ? p->refs : nullptr, masked ? p->occ32 : nullptr, &fcones,
-                                      &mixbits, &mix_words, p->geom_version);
+                                      &mixbits, &mix_words, p->geom_version, other);
   p->gridded_facet = fp;
   p->gridded_hbm_blocks = info;
   p->last_stream = st;
+  if (s == 1) {
+    VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint_gridded");
+    s = viss::tracks_adjoint(p->tracks, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
+                             !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
+                             reinterpret_cast<int *>(p->dev_words + 1), -1, st);
+    if (s == VISS_OK) p->last_total = p->K * p->J;
+    if (s != VISS_ERR_ALLOC) return s;
+    // short of memory for the blocks' sums: grid after all
+    fp = 0;
+    s = viss::gridded_adjoint(&p->gridded, p->J, p->pix, p->perm, p->K, p->samp, p->coef,
+                              (flags & VISS_NO_OFFSET) ? 0 : 1, fp, scale, image, (flags & VISS_ACCUMULATE) ? 1 : 0,
+                              max_cells, st, p->gridded_dims, &fp, &info, masked ? p->refs : nullptr,
+                              masked ? p->occ32 : nullptr, &fcones, &mixbits, &mix_words, p->geom_version, 0.0);
+    p->gridded_facet = fp;
+    p->gridded_hbm_blocks = info;
+  }
   if (s != VISS_OK || !masked) return s;
   // the occulted adjoint: the direct kernel adds every pair the gridded part
   // left out (facets the sample does not see wholly)

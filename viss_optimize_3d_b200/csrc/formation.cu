@@ -584,7 +584,33 @@ __global__ void k_form_reduce_fwd(long long K, int nchunk, const double2 *part, 
   V[k] = make_float2(static_cast<float>(re), static_cast<float>(im));
 }
 
+// The pairs as ordinary samples (u = U_a - U_b, the offset) and their rows in
+// the table [T S satellites][T snapshots].
+__global__ void k_pair_samples(long long T, int S, const double4 *U, const double *off, int sat_rows, int snap_rows,
+                               double4 *samp, int4 *refs) {
+  const long long k = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int B = form_pairs(S);
+  if (k >= T * B) return;
+  const long long t = k / B;
+  int i = static_cast<int>(k - t * B), a = 0;
+  for (int n = S - 1; i >= n; --n) i -= n, ++a;
+  const int b = a + 1 + i;
+  const double4 ua = U[t * S + a], ub = U[t * S + b];
+  samp[k] = make_double4(ua.x - ub.x, ua.y - ub.y, ua.z - ub.z, off ? off[k] : 0.0);
+  if (refs)
+    refs[k] = make_int4(sat_rows ? static_cast<int>(t * S + a) : -1, sat_rows ? static_cast<int>(t * S + b) : -1,
+                        snap_rows ? static_cast<int>(T * S + t) : -1, -1);
+}
+
 static inline unsigned nblk(long long n, int bs) { return static_cast<unsigned>((n + bs - 1) / bs); }
+
+cudaError_t launch_pair_samples(long long T, int S, const double4 *U, const double *off, int sat_rows, int snap_rows,
+                                double4 *samp, int4 *refs, cudaStream_t st) {
+  const long long K = T * form_pairs(S);
+  if (K <= 0) return cudaSuccess;
+  k_pair_samples<<<nblk(K, 256), 256, 0, st>>>(T, S, U, off, sat_rows, snap_rows, samp, refs);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_form_stage(long long T, int S, const double *U, const double *off,
                               double4 *U4, unsigned long long *bound, cudaStream_t st) {

@@ -361,6 +361,18 @@ __global__ void k_stage_coef(long long K, long long Kpad, const float2 *coef, fl
   out[i] = biased ? unbias_coef(a) : a;
 }
 
+// *flag != 0 if any component is infinite or NaN.
+__global__ void k_nonfinite(long long n, const float2 *v, unsigned long long *flag) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n && !(isfinite(v[i].x) && isfinite(v[i].y))) atomicOr(flag, 1ull);
+}
+
+cudaError_t launch_nonfinite(long long n, const float2 *v, unsigned long long *flag, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_nonfinite<<<nblk(n, 256), 256, 0, st>>>(n, v, flag);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out,
                               bool biased, cudaStream_t st) {
   if (Kpad <= 0) return cudaSuccess;

@@ -651,6 +651,12 @@ struct GriddedState {
   long long cache_version = -1, cache_request = -1, cache_fp = 0, cache_words = 0;
   bool cache_masked = false, cache_mix = false;
   double cache_umax = 0, cache_X[3] = {0, 0, 0};
+  // the library's own choice of facets (request 0) and its modelled time, for a
+  // geometry version
+  long long choice_version = -1, choice_fp = 0;
+  bool choice_masked = false;
+  double choice_seconds = 0;
+  int choice_dims[3] = {0, 0, 0};
   ~GriddedState() {
     if (fft_ok) cufftDestroy(fft);
     void *bufs[] = {grid, frames, fcones, rs, mixbits, pre, tabs, status, red, sort, ss, cs};
@@ -784,13 +790,17 @@ int sort_samples(GriddedState &S, long long K, const double4 *samp, const float2
 // modelled time whose grid holds at most max_cells points; the choice is
 // returned in *facet_used).  samp / coef are the plan's staged samples and
 // coefficients.  info[0] = blocks that spread into HBM directly, summed over
-// the facets.  Returns a viss status (0 = ok).
+// the facets.  other_seconds > 0: the modelled time of another way to the same
+// image; if the library's choice of facets is modelled slower, that choice is
+// reported and kOtherWay returned, nothing gridded.  Returns a viss status
+// (0 = ok).
 int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *perm, long long K,
                     const double4 *samp, const float2 *coef, int use_off, long long facet_pix,
                     float scale, float *img, int accumulate, long long max_cells, cudaStream_t st,
                     int *grid_dims, long long *facet_used, long long *info, const int4 *refs,
                     const float4 *occ32, const float4 **fcones_out, const unsigned **mixbits_out,
-                    long long *mix_words_out, long long geom_version) {
+                    long long *mix_words_out, long long geom_version, double other_seconds) {
+  constexpr int kOtherWay = 1;
   if (K > INT_MAX) return record_error(-1, "viss_adjoint_gridded: more than 2^31 - 1 samples");
   const bool masked = refs != nullptr;
   if (masked && facet_pix % kHybridAlign != 0)
@@ -802,6 +812,15 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
       (!S.status && cudaMalloc(&S.status, 2 * sizeof(int)) != cudaSuccess) ||
       (!S.red && cudaMalloc(&S.red, 6 * sizeof(unsigned long long)) != cudaSuccess))
     return record_error(-3, "viss_adjoint_gridded: device allocation failed");
+  // the model is within a fifth of the measured times either side
+  auto other_way = [&]() { return facet_pix == 0 && other_seconds > 0 && other_seconds < 0.8 * S.choice_seconds; };
+  if (geom_version >= 0 && S.choice_version == geom_version && S.choice_masked == masked && other_way()) {
+    if (facet_used) *facet_used = S.choice_fp;
+    if (grid_dims)
+      for (int d = 0; d < 3; ++d) grid_dims[d] = S.choice_dims[d];
+    if (info) info[0] = 0;
+    return kOtherWay;
+  }
   cudaError_t e;
   if ((e = cudaMemsetAsync(S.red + 3, 0, sizeof(unsigned long long), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(S.status, 0, 2 * sizeof(int), st)) != cudaSuccess)
@@ -831,6 +850,7 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
     // modelled time
     double best_t = 1e300;
     long long last = 0;
+    S.choice_version = -1;
     for (long long c = masked ? kHybridAlign : 64;; c *= 4) {
       if (int s = facet_frames(S, J, c, pix, st, X)) return s;
       last = c;
@@ -850,6 +870,19 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
     if (fp == 0) return record_error(-1, "viss_adjoint_gridded: no facet size keeps the grid under its limit");
     if (fp != last)
       if (int s = facet_frames(S, J, fp, pix, st, X)) return s;
+    const GridGeom chosen = grid_geom(X, umax);
+    S.choice_version = geom_version;
+    S.choice_masked = masked;
+    S.choice_fp = fp;
+    S.choice_seconds = best_t;
+    for (int d = 0; d < 3; ++d) S.choice_dims[d] = chosen.M[d];
+    if (other_way()) {
+      if (facet_used) *facet_used = fp;
+      if (grid_dims)
+        for (int d = 0; d < 3; ++d) grid_dims[d] = chosen.M[d];
+      if (info) info[0] = 0;
+      return kOtherWay;
+    }
   } else if (int s = facet_frames(S, J, fp, pix, st, X)) {
     return s;
   }

@@ -403,6 +403,11 @@ __global__ void k_track_masks(int W, const int *slot, const int4 *refs, const fl
 
 void tracks_free(void *state) { delete static_cast<TrackState *>(state); }
 
+double tracks_seconds(const void *state, const TrackInputs &in, bool masked) {
+  const TrackState &S = *static_cast<const TrackState *>(state);
+  return static_cast<double>(in.K) * in.J * (3.2e-14 * S.cost + (masked ? 7e-14 : 0.0));
+}
+
 int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *usable) {
   *usable = false;
   if (!*statep) *statep = new (std::nothrow) TrackState();
@@ -525,7 +530,7 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     for (double v : least) mean += v / nsamp;
     // against `term`, the cost of a call without track blocks (occultation adds
     // to both); larger groups only help where the smallest already do
-    if (!(mean < (pass ? 0.62 : 0.75) * term)) return 0;
+    if (!(mean < (pass ? 0.63 : 0.75) * term)) return 0;
   }
   // every block's ranks in the classes some sampled block takes (the smallest always)
   chosen[kHalf] = true;
@@ -660,6 +665,7 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   S.has_rest[1] = pairs_of[0] != 0;
   S.has_rest[0] = false;                           // unocculted: wide groups, blocks without nodes
   for (const TrackSlab &sl : S.slabs) S.has_rest[0] = S.has_rest[0] || wide[sl.cls] || wide[kTile];
+  S.cost = mean;
   *usable = true;
   return 0;
 }

@@ -91,6 +91,7 @@ struct TrackState {
   int gat[kClasses] = {0, 0, 0, 0};        // a class's first centre in gcen
   long long Ks = 0, ld_max = 0;
   bool has_rest[2] = {false, false};       // unocculted, occulted
+  double cost = 0;                         // modelled issue slots per (sample, pixel); an evaluated term is 21
   std::vector<TrackSlab> slabs;
 
   TrackBits bits(bool occulted) const {
