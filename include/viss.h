@@ -240,8 +240,8 @@ int viss_adjoint_formation(viss_plan *plan, const float *coef, float *image, flo
 
 /* Test hook for the failure path: the next viss_forward or viss_adjoint on
  * this plan has its first thread block skip the staging copy of its `tile`-th
- * tile (a pixel tile in the forward, a sample tile in the adjoint), so that
- * block's bounded waits give up (about 1 s each, no fault, no trap), the
+ * tile (a pixel tile in the forward, a sample tile in the adjoint; its last
+ * one if it has fewer), so that block's bounded waits give up (about 1 s each, no fault, no trap), the
  * kernel ends, and viss_plan_last_stats / viss_plan_last_counts then return
  * VISS_ERR_TIMEOUT; the plan and the context stay usable.  The results of
  * that one call are incomplete.  With plan == NULL the hook arms the next
@@ -249,7 +249,8 @@ int viss_adjoint_formation(viss_plan *plan, const float *coef, float *image, flo
  * VISS_ERR_TIMEOUT itself.  No counterpart in the reference. */
 int viss_plan_debug_drop_copy(viss_plan *plan, int tile);
 
-/* Sets the launch shapes directly (indices 0..3 each). */
+/* Sets the launch shapes directly (indices 0..3 each).  A plan that has neither
+ * been tuned nor given shapes picks them by the sizes of each call. */
 int viss_plan_set_shapes(viss_plan *plan, int fwd_shape, int adj_shape);
 
 /* Terms evaluated by the last viss_forward / viss_adjoint on this plan

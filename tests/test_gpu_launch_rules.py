@@ -1,0 +1,61 @@
+"""Launch shapes and chunk sums at the sizes where their rules change, against
+the defining sums in 64 bits (plain torch).
+
+A split-precision term is within 4e-7 of its value, and at most 128 terms are
+added in plain FP32 (2^-24 of the running sum each, at most 128 of them) before
+a Kahan or FP64 sum takes over, so a value is within (4e-7 + 128 * 2^-24) of the
+sum of its terms' sizes.  A chunk left out or added twice moves a value by
+~1e-3 of it or more at these sizes.
+"""
+import math
+
+import pytest
+import torch
+
+from viss_optimize_3d_b200 import api
+
+pytestmark = pytest.mark.gpu
+BOUND = 4e-7 + 128 * 2.0 ** -24
+
+
+def oracle(lmn, uvw, refs, occ, sky, coef):
+    V = torch.zeros(len(uvw), dtype=torch.complex128, device=lmn.device)
+    img = torch.zeros(len(lmn), dtype=torch.float64, device=lmn.device)
+    for k0 in range(0, len(uvw), 1024):
+        u = uvw[k0:k0 + 1024]
+        ph = u @ lmn.T
+        e = torch.polar(torch.ones_like(ph), -2 * math.pi * (ph - ph.round()))
+        if refs is not None:
+            for r in refs[k0:k0 + 1024].long().T:
+                rows = occ[r.clamp(min=0)]
+                e = torch.where((r < 0)[:, None] | (rows[:, :3] @ lmn.T >= rows[:, 3:]), e, 0)
+        V[k0:k0 + 1024] = e @ sky.to(torch.complex128)
+        img += (coef[k0:k0 + 1024].to(torch.complex128)[:, None] * e.conj()).real.sum(0)
+    return V, img
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("nside,K", [
+    (2, 1),         # one tile, one chunk
+    (4, 31),        # two tiles; less than a row of the chunk sums
+    (8, 33),        # a second block of the sums with one sample
+    (24, 450),      # fewer blocks than SMs: the occulted forward keeps its wide blocks
+    (37, 3330),     # a last pixel block that is mostly padding
+    (12, 9001),     # 71 sample chunks of 14 pixel tiles
+    (64, 1000),     # wide blocks padded by a quarter
+])
+def test_sums(cuda_device, nside, K, masked):
+    lmn = api.pix2lmn(nside, "ring", device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(K)
+    uvw = 60 * torch.randn(K, 3, generator=g, device=cuda_device, dtype=torch.float64)
+    refs = occ = None
+    if masked:
+        n = torch.nn.functional.normalize(torch.randn(20, 3, generator=g, device=cuda_device, dtype=torch.float64), dim=1)
+        occ = torch.cat([n, torch.empty(20, 1, device=cuda_device, dtype=torch.float64).uniform_(-0.9, 0.3, generator=g)], 1)
+        refs = torch.randint(-1, 20, (K, 3), generator=g, device=cuda_device, dtype=torch.int32)
+    sky = torch.rand(len(lmn), generator=g, device=cuda_device) + 0.1
+    coef = torch.randn(K, generator=g, device=cuda_device, dtype=torch.complex64)
+    V, img = oracle(lmn, uvw, refs, occ, sky, coef)
+    plan = api.Plan(lmn, uvw, None, refs, occ)
+    assert float((plan.forward(sky) - V).abs().max()) <= BOUND * float(sky.double().sum())
+    assert float((plan.adjoint(coef) - img).abs().max()) <= BOUND * math.sqrt(2) * float(coef.abs().double().sum())

@@ -41,8 +41,9 @@ cudaError_t launch_form_stage_coef(long long, int, const float2 *, const double 
 cudaError_t launch_form_reduce_fwd(long long, int, const double2 *, const double *, float2 *, int,
                                    cudaStream_t);
 cudaError_t launch_stage_sky(long long, long long, const double4 *, const int *, const float *,
-                             float, double4 *, int, cudaStream_t);
-cudaError_t launch_stage_coef(long long, long long, const float2 *, float2 *, bool, cudaStream_t);
+                             float, double4 *, int, unsigned long long *, cudaStream_t);
+cudaError_t launch_stage_coef(long long, long long, const float2 *, float2 *, bool, unsigned long long *,
+                              cudaStream_t);
 cudaError_t launch_stage_samples(long long, const double *, const double *, const int32_t *,
                                  long long, double4 *, int4 *, unsigned long long *, int *,
                                  cudaStream_t);
@@ -174,8 +175,8 @@ struct viss_plan {
   long long last_total = 0;
   cudaStream_t last_stream = nullptr;
   // launch shape
-  int fwd_shape = 0;   // index into viss::kFwdShapes (viss_plan_tune picks it)
-  int adj_shape = 0;   // index into viss::kAdjShapes
+  int fwd_shape = -1;  // index into viss::kFwdShapes (viss_plan_tune, _set_shapes); -1: auto_fwd_shape
+  int adj_shape = -1;  // index into viss::kAdjShapes; -1: auto_adj_shape
   int drop_tile = -1;  // test hook for the next kernel (viss_plan_debug_drop_copy)
   int fwd_waves = 16;
   int adj_waves = 16;
@@ -200,23 +201,27 @@ struct viss_plan {
 
 namespace {
 
+// Pixel-tile chunks of the forward: about 16 waves of resident CTAs, down to one
+// tile each (10,080 samples x 96 tiles: 480 CTAs of two tiles give the busiest
+// of 148 SMs 8 tiles where 6.5 are its share, 960 CTAs of one tile 7: 91 -> 84 us).
 int fwd_chunks(const viss_plan *p, int shape, bool fp64) {
   const long long per = viss::forward_samples_per_block(shape, fp64);
   const long long blocks = (p->Kc + per - 1) / per * p->channels;
   const long long slots = static_cast<long long>(p->nsm) * viss::forward_ctas_per_sm(shape, fp64);
   long long c = (static_cast<long long>(p->fwd_waves) * slots + blocks - 1) / blocks;
-  c = std::max<long long>(1, std::min<long long>(c, std::max(1, p->ntiles / 2)));
+  c = std::max<long long>(1, std::min<long long>(c, p->ntiles));
   return static_cast<int>(c);
 }
 
 // Sample chunks per channel for the adjoint (and their size, a multiple of
-// the staging tile).
+// the staging tile), in the same way: 102 -> 91 us at that size with chunks of
+// one staging tile instead of two.
 int adj_chunks(const viss_plan *p, int shape, bool fp64, int *samples_per_chunk) {
   const long long per = viss::adjoint_pixels_per_block(shape, fp64);  // pixels per CTA
   const long long blocks = (p->Jpad + per - 1) / per * p->channels;
   const long long slots = static_cast<long long>(p->nsm) * viss::adjoint_ctas_per_sm(shape, fp64);
   long long c = (static_cast<long long>(p->adj_waves) * slots + blocks - 1) / blocks;
-  const long long max_c = std::max<long long>(1, (p->Kc + 255) / 256);
+  const long long max_c = std::max<long long>(1, (p->Kc + viss::kSampTile - 1) / viss::kSampTile);
   c = std::max<long long>(1, std::min(c, max_c));
   c = std::min<long long>(c, std::max<long long>(1, 65535 / p->channels));
   long long spc = (p->Kc + c - 1) / c;
@@ -224,6 +229,47 @@ int adj_chunks(const viss_plan *p, int shape, bool fp64, int *samples_per_chunk)
   c = (p->Kc + spc - 1) / spc;
   *samples_per_chunk = static_cast<int>(spc);
   return static_cast<int>(std::max<long long>(1, c));
+}
+
+// Sample (pixel) x tile units of the busiest SM when a shape's grid is dealt out
+// evenly: whole CTAs per SM, and the padding of the last sample (pixel) block.
+double fwd_load(const viss_plan *p, int shape) {
+  const long long per = viss::forward_samples_per_block(shape, false);
+  const long long blocks = (p->Kc + per - 1) / per * p->channels;
+  const int c = fwd_chunks(p, shape, false), tpc = (p->ntiles + c - 1) / c;
+  const long long ctas = blocks * ((p->ntiles + tpc - 1) / tpc);
+  return static_cast<double>((ctas + p->nsm - 1) / p->nsm) * tpc * static_cast<double>(per);
+}
+
+double adj_load(const viss_plan *p, int shape) {
+  const long long per = viss::adjoint_pixels_per_block(shape, false);
+  int spc = 0;
+  const long long ctas = (p->Jpad + per - 1) / per * p->channels * adj_chunks(p, shape, false, &spc);
+  return static_cast<double>((ctas + p->nsm - 1) / p->nsm) * static_cast<double>(std::min<long long>(spc, p->Kc)) *
+         static_cast<double>(per);
+}
+
+// The launch shape of a plan that has not been given one.  Measured over 16 sizes
+// of 3e6 to 1e10 terms, against shape 0 = (4 samples, 2 CTAs) and (8 pixels, 4):
+// forward, unocculted: (2, 3) takes .98 of its time, down to .59 where the wider
+// blocks leave SMs idle; occulted it takes 1.02 (a row fetch serves two samples
+// instead of four) unless the busiest SM has less to do: loads of .50 to .95 gave
+// .84 to .96, but with fewer blocks than SMs latency decides, not load (450
+// samples: 1.08).
+int auto_fwd_shape(const viss_plan *p, bool masked) {
+  if (!masked) return 2;
+  const long long per = viss::forward_samples_per_block(0, false);
+  const long long ctas = (p->Kc + per - 1) / per * p->channels * p->ntiles;
+  return ctas >= p->nsm && fwd_load(p, 2) < 0.97 * fwd_load(p, 0) ? 2 : 0;
+}
+
+// Adjoint, unocculted: (8, 5) takes .93 to .96 of the time of (8, 4), and (4, 6),
+// 1.02 at most sizes, .76 to .83 where its load is below .9.  Occulted: (4, 6)
+// takes .83 to .99 (a warp's tile is half as wide, so fewer samples are mixed on
+// it); with a load of 1.08 it took 1.01.
+int auto_adj_shape(const viss_plan *p, bool masked) {
+  if (masked) return adj_load(p, 3) <= 1.05 * adj_load(p, 0) ? 3 : 0;
+  return adj_load(p, 3) < 0.93 * adj_load(p, 1) ? 3 : 1;
 }
 
 cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
@@ -514,15 +560,15 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                         int shape, bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
+  if (shape < 0) shape = auto_fwd_shape(p, masked);
   const int nchunk = fwd_chunks(p, shape, fp64);
   if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * p->K)) return s;
   if (int s = ensure(p->pixsky, p->pixsky_cap, sizeof(double4) * p->Jpad * p->channels,
                      "pixel+sky records"))
     return s;
   VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky,
-                                   p->channels, st),
+                                   p->channels, p->dev_words, st),
             "viss_forward: sky");
-  VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_forward");
   bool use = false;
   if (tracks && !fp64)
     if (int s = tracks_ready(p, st, &use)) return s;
@@ -596,13 +642,14 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
                         bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
+  if (shape < 0) shape = fcones ? 0 : auto_adj_shape(p, masked);
   int spc = 0;
   const int nchunk = adj_chunks(p, shape, fp64, &spc);
   if (int s = workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * p->channels * p->Jpad))
     return s;
-  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, !fp64, st),
+  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, !fp64, p->dev_words,
+                                    st),
             "viss_adjoint: coef");
-  VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint");
   bool use = false;
   if (tracks && !fp64 && !fcones)
     if (int s = tracks_ready(p, st, &use)) return s;
@@ -675,7 +722,7 @@ int viss_plan_tune(viss_plan *p, const float *sky, const float *coef, float *V_s
   VISS_CUDA(cudaEventCreate(&e0), "viss_plan_tune");
   VISS_CUDA(cudaEventCreate(&e1), "viss_plan_tune");
   float best_f = 1e30f, best_a = 1e30f;
-  int bf = p->fwd_shape, ba = p->adj_shape, status = VISS_OK;
+  int bf = 0, ba = 0, status = VISS_OK;
   for (int s = 0; s < viss::kNumFwdShapes && status == VISS_OK; ++s) {
     status = forward_impl(p, sky, V_scratch, flags, st, s, false);
     if (status) break;
@@ -877,9 +924,8 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
   if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * T * B)) return s;
   if (int s = ensure(p->pixsky, p->pixsky_cap, sizeof(double4) * p->Jpad * C, "pixel+sky records"))
     return s;
-  VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky, C, st),
+  VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky, C, p->dev_words, st),
             "viss_forward_formation: sky");
-  VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_forward_formation");
   bool use = false;
   const bool masked = (fp.sat_rows || fp.snap_rows);
   if (int s = form_tracks_ready(p, masked, 3.07e-13, st, &use)) return s;
@@ -976,7 +1022,7 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   const long long max_cells = 1LL << 29;   // 4 GiB of FP32 complex grid
   long long fp = facet_pixels, info = 0;
   const cudaStream_t st = as_stream(stream);
-  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, false, st),
+  VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, false, nullptr, st),
             "viss_adjoint_gridded: coef");
   const float4 *fcones = nullptr;
   const unsigned *mixbits = nullptr;

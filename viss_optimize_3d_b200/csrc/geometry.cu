@@ -245,10 +245,13 @@ __global__ void k_occ32(long long G, const double4 *occ, float4 *out) {
 
 // Sky staging: pixel record + sky value in the low word of .w (zero past J),
 // so one 32-byte record per pixel carries everything the forward reads.
-// One channel per blockIdx.y: out[ch][i] = (pix[i], sky[ch][perm[i]]).
+// One channel per blockIdx.y: out[ch][i] = (pix[i], sky[ch][perm[i]]).  It clears
+// the call's three status words on the way: a memset of its own cost 4 us of the
+// smallest calls' 30 us beside the sums.
 __global__ void k_stage_sky(long long J, long long Jpad, const double4 *pix, const int *perm,
-                            const float *sky, float scale, double4 *out) {
+                            const float *sky, float scale, double4 *out, unsigned long long *zero) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (zero && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3) zero[threadIdx.x] = 0;
   if (i >= Jpad) return;
   const long long ch = blockIdx.y;
   double4 r = pix[i];
@@ -345,17 +348,20 @@ cudaError_t launch_occ32(long long G, const double4 *occ, float4 *out, cudaStrea
 
 cudaError_t launch_stage_sky(long long J, long long Jpad, const double4 *pix, const int *perm,
                              const float *sky, float scale, double4 *out, int channels,
-                             cudaStream_t st) {
+                             unsigned long long *zero, cudaStream_t st) {
   dim3 grid(nblk(Jpad, 256), static_cast<unsigned>(channels));
-  k_stage_sky<<<grid, 256, 0, st>>>(J, Jpad, pix, perm, sky, scale, out);
+  k_stage_sky<<<grid, 256, 0, st>>>(J, Jpad, pix, perm, sky, scale, out, zero);
   return cudaGetLastError();
 }
 
 // Coefficient staging for the adjoint: a 16-byte aligned copy padded to an
 // even count (bulk copies move whole 16-byte units); biased: for k_adjoint's
-// split-precision terms.
-__global__ void k_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out, int biased) {
+// split-precision terms.  zero: the call's three status words, which it clears
+// on the way, or null.
+__global__ void k_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out, int biased,
+                             unsigned long long *zero) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (zero && blockIdx.x == 0 && threadIdx.x < 3) zero[threadIdx.x] = 0;
   if (i >= Kpad) return;
   const float2 a = i < K ? coef[i] : make_float2(0.f, 0.f);
   out[i] = biased ? unbias_coef(a) : a;
@@ -374,9 +380,9 @@ cudaError_t launch_nonfinite(long long n, const float2 *v, unsigned long long *f
 }
 
 cudaError_t launch_stage_coef(long long K, long long Kpad, const float2 *coef, float2 *out,
-                              bool biased, cudaStream_t st) {
+                              bool biased, unsigned long long *zero, cudaStream_t st) {
   if (Kpad <= 0) return cudaSuccess;
-  k_stage_coef<<<nblk(Kpad, 256), 256, 0, st>>>(K, Kpad, coef, out, biased ? 1 : 0);
+  k_stage_coef<<<nblk(Kpad, 256), 256, 0, st>>>(K, Kpad, coef, out, biased ? 1 : 0, zero);
   return cudaGetLastError();
 }
 
