@@ -260,7 +260,7 @@ int auto_fwd_shape(const viss_plan *p, bool masked) {
   if (!masked) return 2;
   const long long per = viss::forward_samples_per_block(0, false);
   const long long ctas = (p->Kc + per - 1) / per * p->channels * p->ntiles;
-  return ctas >= p->nsm && fwd_load(p, 2) < 0.97 * fwd_load(p, 0) ? 2 : 0;
+  return ctas >= p->nsm && fwd_load(p, 2) < 0.95 * fwd_load(p, 0) ? 2 : 0;
 }
 
 // Adjoint, unocculted: (8, 5) takes .93 to .96 of the time of (8, 4), and (4, 6),
@@ -878,12 +878,13 @@ static viss::TrackInputs form_track_inputs(const viss_plan *p) {
 
 // Whether a formation call goes through track blocks of its pairs (u = U_a -
 // U_b, the same rows): when they are modelled faster than the formation kernels'
-// `per_term` seconds (forward 3.07e-13, adjoint 2.43e-13 at S = 10, Nside 256 x 388,800 samples,
-// Moon + Earth, per sample and pixel; measured 94.1 against 54 ms and 74.5
-// against 67 ms at 10 MHz).  Per pair S exponentials serve S - 1 / 2: with fewer
+// seconds (forward 3.07e-13, adjoint 2.43e-13 per sample and pixel at S = 10, Nside
+// 256 x 388,800 samples, Moon + Earth; measured 94.1 against 55 ms and 74.5
+// against 63 ms at 10 MHz).  Per pair S exponentials serve S - 1 / 2: with fewer
 // satellites a pair costs the formation kernels more, which only favours the blocks.
-static int form_tracks_ready(viss_plan *p, bool masked, double per_term, cudaStream_t st, bool *use) {
+static int form_tracks_ready(viss_plan *p, bool masked, bool adjoint, cudaStream_t st, bool *use) {
   *use = false;
+  const double per_term = adjoint ? 2.43e-13 : 3.07e-13;
   const long long K = p->form_T * viss::form_pairs(p->form_S);
   if (!tracks_allowed(static_cast<double>(K) * p->J, st) || !(3.0 * p->form_turns < 262144.0)) return VISS_OK;
   if (p->form_tracks_version != p->form_version) {
@@ -901,7 +902,7 @@ static int form_tracks_ready(viss_plan *p, bool masked, double per_term, cudaStr
   }
   const viss::TrackInputs in = form_track_inputs(p);
   *use = p->form_tracks_usable &&
-         viss::tracks_seconds(p->form_tracks, in, masked) < 0.95 * per_term * static_cast<double>(in.K) * in.J;
+         viss::tracks_seconds(p->form_tracks, in, masked, adjoint) < 0.95 * per_term * static_cast<double>(in.K) * in.J;
   return VISS_OK;
 }
 
@@ -928,7 +929,7 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
             "viss_forward_formation: sky");
   bool use = false;
   const bool masked = (fp.sat_rows || fp.snap_rows);
-  if (int s = form_tracks_ready(p, masked, 3.07e-13, st, &use)) return s;
+  if (int s = form_tracks_ready(p, masked, false, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_forward(p->form_tracks, form_track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V),
                                        masked, !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
@@ -981,7 +982,7 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
   viss::FormParams fp = form_params(p, flags);
   bool use = false;
   const bool masked = (fp.sat_rows || fp.snap_rows);
-  if (int s = form_tracks_ready(p, masked, 2.43e-13, st, &use)) return s;
+  if (int s = form_tracks_ready(p, masked, true, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_adjoint(p->form_tracks, form_track_inputs(p), reinterpret_cast<const float2 *>(coef),
                                        image, scale, masked, !(flags & VISS_NO_OFFSET),
@@ -1040,7 +1041,7 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
       unsigned long long bad = 0;
       VISS_CUDA(cudaMemcpyAsync(&bad, p->dev_words + 3, sizeof(bad), cudaMemcpyDeviceToHost, st), "viss_adjoint_gridded");
       VISS_CUDA(cudaStreamSynchronize(st), "viss_adjoint_gridded");
-      if (!bad) other = viss::tracks_seconds(p->tracks, track_inputs(p), masked);
+      if (!bad) other = viss::tracks_seconds(p->tracks, track_inputs(p), masked, true);
     }
   }
   int s = viss::gridded_adjoint(&p->gridded, p->J, p->pix, p->perm, p->K, p->samp, p->coef,

@@ -30,11 +30,13 @@ struct TrackInputs {
 int tracks_build(void **state, const TrackInputs &in, cudaStream_t st, bool *usable);
 void tracks_free(void *state);
 
-// Modelled time of one call with the built blocks, in seconds (an occulted call
-// also evaluates the pairs at the rims): 3.2e-14 s per (sample, pixel) and
-// modelled issue slot, and 7e-14 s per occulted pair, from the adjoint at Nside 256 x
-// 388,800 samples, 1 and 10 MHz (20.8 / 41.5 ms and 54.8 / 66.8 ms).
-double tracks_seconds(const void *state, const TrackInputs &in, bool masked);
+// Modelled time of one call with the built blocks, in seconds: per (sample, pixel)
+// and modelled issue slot 3.1e-14 (forward) or 3.3e-14 s (adjoint), and in an
+// occulted call 0.85 of that, for what is hidden, plus the pairs at the rims, whose
+// share goes with the width of a tile: 4.3e-11 or 5.5e-11 / sqrt(J).  Within 10 %
+// of nine calls of 1e10 to 3e11 terms at Nside 128 and 256, 1 to 10 MHz, occulted
+// and not (9.6e-14 to 3.4e-13 s per term).
+double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint);
 
 // V (channel-major, caller's order) and images of the built blocks.  pixsky:
 // the staged pixel + sky records of every channel; coef: the caller's

@@ -403,9 +403,11 @@ __global__ void k_track_masks(int W, const int *slot, const int4 *refs, const fl
 
 void tracks_free(void *state) { delete static_cast<TrackState *>(state); }
 
-double tracks_seconds(const void *state, const TrackInputs &in, bool masked) {
+double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint) {
   const TrackState &S = *static_cast<const TrackState *>(state);
-  return static_cast<double>(in.K) * in.J * (3.2e-14 * S.cost + (masked ? 7e-14 : 0.0));
+  double per = (adjoint ? 3.3e-14 : 3.1e-14) * S.cost;
+  if (masked) per = 0.85 * per + (adjoint ? 5.5e-11 : 4.3e-11) / std::sqrt(static_cast<double>(in.J));
+  return static_cast<double>(in.K) * in.J * per;
 }
 
 int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *usable) {
@@ -529,8 +531,10 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     mean = 0;
     for (double v : least) mean += v / nsamp;
     // against `term`, the cost of a call without track blocks (occultation adds
-    // to both); larger groups only help where the smallest already do
-    if (!(mean < (pass ? 0.63 : 0.75) * term)) return 0;
+    // to both): at .63 to .70 an occulted call takes .81 to .95 of the direct
+    // kernels' time, and a build about 3 % of the smallest call's that gets here.
+    // Larger groups only help where the smallest already do.
+    if (!(mean < (pass ? 0.70 : 0.82) * term)) return 0;
   }
   // every block's ranks in the classes some sampled block takes (the smallest always)
   chosen[kHalf] = true;
