@@ -141,6 +141,13 @@ int viss_plan_set_samples(viss_plan *plan, int64_t K, const double *uvw, const d
  * VISS_ERR_TIMEOUT; callers that need the guarantee check it after the call. */
 int viss_forward(viss_plan *plan, const float *sky, float *V, int flags, void *stream);
 
+/* n skies over the plan's samples (a plan of one channel):
+ *   V[c][k] = sum_j sky[c][j] exp(-2 pi i (u_k . s_j + off_k)) vis_kj
+ * sky: n x J, V: n x K.  The same values as n channels of repeated samples, and
+ * as there K must be even when n > 1.  Used for the three phase derivatives of
+ * the gradient.  No counterpart in the reference. */
+int viss_forward_skies(viss_plan *plan, int n, const float *sky, float *V, int flags, void *stream);
+
 /* Imaging adjoint, replaces computeC (vissgen3d_blockage.cu:167-192):
  *   image_j = scale * sum_k Re(coef_k exp(+2 pi i (u_k . s_j + off_k))) vis_kj
  * coef: K complex64 (the weighted visibilities w_k V_k); image: J FP32.  Track

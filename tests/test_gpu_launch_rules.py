@@ -59,3 +59,38 @@ def test_sums(cuda_device, nside, K, masked):
     plan = api.Plan(lmn, uvw, None, refs, occ)
     assert float((plan.forward(sky) - V).abs().max()) <= BOUND * float(sky.double().sum())
     assert float((plan.adjoint(coef) - img).abs().max()) <= BOUND * math.sqrt(2) * float(coef.abs().double().sum())
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("nside,K,n", [
+    (2, 2, 3),       # one tile, one block
+    (13, 254, 3),    # a block that is not full, a part of a last tile
+    (24, 4098, 3),   # 17 blocks of samples, several chunks
+    (24, 450, 2),    # not three: one sky after the other
+    (16, 33, 1),     # one sky, odd count
+])
+def test_skies(cuda_device, nside, K, n, masked):
+    lmn = api.pix2lmn(nside, "ring", device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(K)
+    uvw = 60 * torch.randn(K, 3, generator=g, device=cuda_device, dtype=torch.float64)
+    refs = occ = None
+    if masked:
+        v = torch.nn.functional.normalize(torch.randn(20, 3, generator=g, device=cuda_device, dtype=torch.float64), dim=1)
+        occ = torch.cat([v, torch.empty(20, 1, device=cuda_device, dtype=torch.float64).uniform_(-0.9, 0.3, generator=g)], 1)
+        refs = torch.randint(-1, 20, (K, 3), generator=g, device=cuda_device, dtype=torch.int32)
+    sky = torch.randn(n, len(lmn), generator=g, device=cuda_device)
+    plan = api.Plan(lmn, uvw, None, refs, occ)
+    for fp64 in (False, True):
+        V = plan._forward_skies(sky, fp64=fp64)
+        assert V.shape == (n, K) and plan.last_stats()[2] == n * K * len(lmn)
+        for c in range(n):
+            want, _ = oracle(lmn, uvw, refs, occ, sky[c], torch.zeros(K, dtype=torch.complex64, device=cuda_device))
+            assert float((V[c] - want).abs().max()) <= BOUND * float(sky[c].abs().double().sum())
+
+
+def test_skies_refuse_odd_counts(cuda_device):
+    """As three channels of repeated samples do."""
+    lmn = api.pix2lmn(4, "ring", device=cuda_device)
+    plan = api.Plan(lmn, torch.ones(3, 3, dtype=torch.float64, device=cuda_device))
+    with pytest.raises(RuntimeError, match="must be even"):
+        plan._forward_skies(torch.ones(3, len(lmn), device=cuda_device))

@@ -58,6 +58,7 @@ _SIGS = {
     "viss_plan_set_pixels": (_i, [_v, _i64, _v, _v]),
     "viss_plan_set_samples": (_i, [_v, _i64, _v, _v, _v, _i64, _v, _v]),
     "viss_forward": (_i, [_v, _v, _v, _i, _v]),
+    "viss_forward_skies": (_i, [_v, _i, _v, _v, _i, _v]),
     "viss_adjoint": (_i, [_v, _v, _v, _f, _i, _v]),
     "viss_adjoint_gridded": (_i, [_v, _v, _v, _f, _i, _i64, _v]),
     "viss_plan_gridded_info": (_i, [_v, _v, _v, _v]),

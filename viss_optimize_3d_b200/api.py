@@ -209,6 +209,15 @@ class Plan:
                                _stream(sky)), "viss_forward")
         return out
 
+    def _forward_skies(self, sky, fp64: bool = False) -> torch.Tensor:
+        """V (n x K complex64) of n skies (n x J) over the plan's samples; an
+        even K, one channel."""
+        sky = _cuda(sky, torch.float32, self.device)
+        out = torch.empty((sky.shape[0], self.K), dtype=torch.complex64, device=self.device)
+        check(lib.viss_forward_skies(self._h, sky.shape[0], _p(sky), _p(out), self._flags(fp64, True, True),
+                                     _stream(sky)), "viss_forward_skies")
+        return out
+
     def adjoint(self, coef, scale: float = 1.0, fp64: bool = False, mask: bool = True,
                 use_offset: bool = True, out: torch.Tensor | None = None) -> torch.Tensor:
         """computeC (vissgen3d_blockage.cu:167-192):

@@ -13,8 +13,8 @@ backward pass recomputes the exponentials in the GPU kernels.
 
 where g = dL/dV in PyTorch's convention for complex tensors (for a real loss,
 the gradient of V is 2 dL/dconj(V)).  D is the phase derivative: three extra
-visibility sums with the sky weighted by l, m and n, computed as one
-three-channel viss_forward.  The occultation mask is held fixed (it is not
+visibility sums with the sky weighted by l, m and n, computed by one
+viss_forward_skies.  The occultation mask is held fixed (it is not
 differentiable in u).  Gradients w.r.t. satellite positions follow from u's
 torch graph (u = (P_a - P_b) / lambda).
 
@@ -57,9 +57,7 @@ class VisibilityModel:
 
     def _stage_d(self, uvw: torch.Tensor):
         if self._du is None or self._du.shape != uvw.shape or not torch.equal(self._du, uvw):
-            refs3 = None if self.refs is None else self.refs.repeat(3, 1)
-            self.dplan.set_samples(uvw.repeat(3, 1), None, refs3, self.occ)
-            self.dplan.set_channels(3)
+            self.dplan.set_samples(uvw, None, self.refs, self.occ)
             self._du = uvw.detach().clone()
 
     def forward_raw(self, sky: torch.Tensor, uvw: torch.Tensor) -> torch.Tensor:
@@ -74,8 +72,7 @@ class VisibilityModel:
         """D (K, 3) complex: sum_j I_j vis_kj s_jc exp(-2 pi i u_k . s_j)."""
         self._stage_d(uvw)
         sky3 = (sky.to(torch.float64)[None, :] * self.lmn.T).to(torch.float32).contiguous()
-        D = self.dplan.forward(sky3, fp64=self.fp64)
-        return D.view(3, -1).T
+        return self.dplan._forward_skies(sky3, fp64=self.fp64).T
 
     def __call__(self, sky: torch.Tensor, uvw: torch.Tensor) -> torch.Tensor:
         return _Visibility.apply(sky, uvw, self)

@@ -42,6 +42,8 @@ cudaError_t launch_form_reduce_fwd(long long, int, const double2 *, const double
                                    cudaStream_t);
 cudaError_t launch_stage_sky(long long, long long, const double4 *, const int *, const float *,
                              float, double4 *, int, unsigned long long *, cudaStream_t);
+cudaError_t launch_stage_skies(long long, long long, const int *, const float *, float4 *, unsigned long long *,
+                               cudaStream_t);
 cudaError_t launch_stage_coef(long long, long long, const float2 *, float2 *, bool, unsigned long long *,
                               cudaStream_t);
 cudaError_t launch_stage_samples(long long, const double *, const double *, const int32_t *,
@@ -195,6 +197,7 @@ struct viss_plan {
   long long form_version = 0, form_tracks_version = -1;
   bool form_tracks_usable = false;
   double form_turns = 0;        // bound on |U.s| and |off|
+  float4 *skies = nullptr;      size_t skies_cap = 0;   // viss_forward_skies
   double4 *form_samp = nullptr; size_t form_samp_cap = 0;
   int4 *form_refs = nullptr;    size_t form_refs_cap = 0;
 };
@@ -413,7 +416,7 @@ int viss_plan_destroy(viss_plan *p) {
   void *bufs[] = {p->pix,    p->pixsky,  p->cones,    p->perm,      p->samp,
                   p->refs,   p->occ,     p->occ32,    p->coef,      p->part,
                   p->dev_words, p->form_U, p->form_off, p->form_occ, p->form_occ32,
-                  p->form_coef, p->form_samp, p->form_refs};
+                  p->form_coef, p->form_samp, p->form_refs, p->skies};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->gridded) viss::gridded_free(p->gridded);
@@ -556,8 +559,12 @@ static int tracks_ready(viss_plan *p, cudaStream_t st, bool *use) {
   return VISS_OK;
 }
 
+// Three skies at once, seconds per (sample, pixel): measured 6.0e-13 to 6.3e-13
+// occulted and 6.8e-13 not, at 4e9 to 4e10.
+constexpr double kSkiesSeconds[2] = {6.8e-13, 6.0e-13};
+
 static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cudaStream_t st,
-                        int shape, bool tracks = true) {
+                        int shape, bool tracks = true, bool first = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
   if (shape < 0) shape = auto_fwd_shape(p, masked);
@@ -567,7 +574,7 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                      "pixel+sky records"))
     return s;
   VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky,
-                                   p->channels, p->dev_words, st),
+                                   p->channels, first ? p->dev_words : nullptr, st),
             "viss_forward: sky");
   bool use = false;
   if (tracks && !fp64)
@@ -631,6 +638,70 @@ int viss_forward(viss_plan *p, const float *sky, float *V, int flags, void *stre
   const NvtxRange range("viss_forward");
   if (int s = check_call(p, sky, V, flags, "viss_forward")) return s;
   return forward_impl(p, sky, V, flags, as_stream(stream), p->fwd_shape);
+}
+
+// Several skies over the plan's samples.  Three at once take one exponential per
+// (sample, pixel) where three channels of repeated samples take three (23 against
+// 54 ms at 194,400 samples x Nside 128, 10 MHz, Moon).  Through track blocks, a sky
+// at a time, where those are modelled faster (the same at 3 MHz: 29 ms, not taken;
+// Nside 256 x 388,800 samples at 1 MHz: 3 x 29 against 183 ms).
+int viss_forward_skies(viss_plan *p, int n, const float *sky, float *V, int flags, void *stream) {
+  const NvtxRange range("viss_forward_skies");
+  if (n < 1) return fail(VISS_ERR_ARG, "viss_forward_skies: bad arguments");
+  if (int s = check_call(p, sky, V, flags, "viss_forward_skies")) return s;
+  if (p->channels != 1) return fail(VISS_ERR_STATE, "viss_forward_skies: the plan has channels");
+  if (n > 1 && (p->K & 1))
+    return fail(VISS_ERR_ARG, "viss_forward_skies: samples per channel must be even");
+  const cudaStream_t st = as_stream(stream);
+  const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
+  bool three = n == viss::kSkies && !(flags & VISS_FP64);
+  if (three) {
+    bool use = false;
+    if (int s = tracks_ready(p, st, &use)) return s;
+    three = !use || n * viss::tracks_seconds(p->tracks, track_inputs(p), masked, false) >
+                        0.95 * kSkiesSeconds[masked] * static_cast<double>(p->K) * static_cast<double>(p->J);
+  }
+  if (!three) {
+    for (int c = 0; c < n; ++c)
+      if (int s = forward_impl(p, sky + c * p->J, V + 2 * c * p->K, flags, st, p->fwd_shape, true, c == 0)) return s;
+    p->last_total = n * p->K * p->J;
+    return VISS_OK;
+  }
+  const long long per = viss::forward_skies_samples_per_block();
+  const long long blocks = (p->K + per - 1) / per;
+  long long c = (static_cast<long long>(p->fwd_waves) * p->nsm * viss::forward_skies_ctas_per_sm() + blocks - 1) / blocks;
+  c = std::max<long long>(1, std::min<long long>(c, p->ntiles));
+  viss::FwdParams fp;
+  fp.tiles_per_chunk = static_cast<int>((p->ntiles + c - 1) / c);
+  const int nchunk = (p->ntiles + fp.tiles_per_chunk - 1) / fp.tiles_per_chunk;
+  if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * n * p->K)) return s;
+  if (int s = ensure(p->skies, p->skies_cap, sizeof(float4) * p->Jpad, "sky records")) return s;
+  VISS_CUDA(viss::launch_stage_skies(p->J, p->Jpad, p->perm, sky, p->skies, p->dev_words, st), "viss_forward_skies: sky");
+  fp.samp = p->samp;
+  fp.refs = masked ? p->refs : nullptr;
+  fp.occ = masked ? p->occ : nullptr;
+  fp.occ32 = masked ? p->occ32 : nullptr;
+  fp.pix = p->pix;
+  fp.skies = p->skies;
+  fp.cones = p->cones;
+  fp.K = p->K;
+  fp.ntiles = p->ntiles;
+  fp.part = static_cast<double2 *>(p->part);
+  fp.counter = p->dev_words;
+  fp.err = reinterpret_cast<int *>(p->dev_words + 1);
+  fp.use_off = (flags & VISS_NO_OFFSET) ? 0 : 1;
+  fp.channels = 1;
+  fp.Kc = p->K;
+  fp.pix_stride = p->Jpad;
+  fp.drop_tile = p->drop_tile;
+  p->drop_tile = -1;
+  VISS_CUDA(viss::launch_forward_skies(fp, nchunk, masked, st), "viss_forward_skies: kernel");
+  VISS_CUDA(viss::launch_reduce_fwd(n * p->K, nchunk, fp.part, reinterpret_cast<float2 *>(V),
+                                    (flags & VISS_ACCUMULATE) ? 1 : 0, false, st),
+            "viss_forward_skies: reduce");
+  p->last_total = n * p->K * p->J;
+  p->last_stream = st;
+  return VISS_OK;
 }
 
 // fcones non-null: the hybrid instance (occulted, split precision), which

@@ -140,6 +140,26 @@ __device__ __forceinline__ void fwd_term(double t, float I, float &re, float &im
   }
 }
 
+// The same for NS skies (split precision): one exponential, NS sums.
+template <int NS>
+__device__ __forceinline__ void fwd_term_skies(double t, const float (&I)[NS], float (&re)[NS], float (&im)[NS]) {
+  float sn, cs;
+  sfu_sincos(turn_angle(t), sn, cs);
+#pragma unroll
+  for (int c = 0; c < NS; ++c) {
+    re[c] = fmaf(I[c], cs, re[c]);
+    im[c] = fmaf(-I[c], sn, im[c]);
+  }
+}
+
+// A pixel's NS sky values, zero where it is hidden; odd records negated.
+template <int NS>
+__device__ __forceinline__ void skies_of(const float4 &w, bool seen, bool odd, float (&I)[NS]) {
+  const float v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int c = 0; c < NS; ++c) I[c] = seen ? (odd ? -v[c] : v[c]) : 0.f;
+}
+
 // Pixels per forward sub-tile (the span a mixed sample row is refined to).
 constexpr int kSubPix = 32;
 
@@ -163,6 +183,22 @@ __device__ __forceinline__ void fwd_span(const double4 *tp, double ux, double uy
     fwd_term<FP64>(ta, Ia, re, im, dre, dim);
     const double tb = fma(uz, b.z, fma(uy, b.y, fma(ux, b.x, mk2)));
     fwd_term<FP64>(tb, Ib, re, im, dre, dim);
+  }
+}
+
+// fwd_span for NS skies, whose values stand beside the records.
+template <int NROWS, int NS>
+__device__ __forceinline__ void fwd_span_skies(const double4 *tp, const float4 *wp, double ux, double uy, double uz,
+                                               double mk, double mk2, const double4 &q0, const double4 &q1,
+                                               const double4 &q2, float (&re)[NS], float (&im)[NS]) {
+#pragma unroll 2
+  for (int j = 0; j < kSubPix; j += 2) {
+    const double4 a = tp[j], b = tp[j + 1];
+    float Ia[NS], Ib[NS];
+    skies_of<NS>(wp[j], visible_rows<NROWS>(q0, q1, q2, a.x, a.y, a.z), false, Ia);
+    skies_of<NS>(wp[j + 1], visible_rows<NROWS>(q0, q1, q2, b.x, b.y, b.z), true, Ib);
+    fwd_term_skies<NS>(fma(uz, a.z, fma(uy, a.y, fma(ux, a.x, mk))), Ia, re, im);
+    fwd_term_skies<NS>(fma(uz, b.z, fma(uy, b.y, fma(ux, b.x, mk2))), Ib, re, im);
   }
 }
 

@@ -354,6 +354,26 @@ cudaError_t launch_stage_sky(long long J, long long Jpad, const double4 *pix, co
   return cudaGetLastError();
 }
 
+// Staging of kSkies skies: out[i] = their values at record i (zero past J).
+__global__ void k_stage_skies(long long J, long long Jpad, const int *perm, const float *sky, float4 *out,
+                              unsigned long long *zero) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x < 3) zero[threadIdx.x] = 0;
+  if (i >= Jpad) return;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < J) {
+    const long long j = perm[i];
+    v = make_float4(sky[j], sky[J + j], sky[2 * J + j], 0.f);
+  }
+  out[i] = v;
+}
+
+cudaError_t launch_stage_skies(long long J, long long Jpad, const int *perm, const float *sky, float4 *out,
+                               unsigned long long *zero, cudaStream_t st) {
+  k_stage_skies<<<nblk(Jpad, 256), 256, 0, st>>>(J, Jpad, perm, sky, out, zero);
+  return cudaGetLastError();
+}
+
 // Coefficient staging for the adjoint: a 16-byte aligned copy padded to an
 // even count (bulk copies move whole 16-byte units); biased: for k_adjoint's
 // split-precision terms.  zero: the call's three status words, which it clears

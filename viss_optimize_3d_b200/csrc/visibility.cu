@@ -38,6 +38,8 @@
 // long baselines is ~700x smaller.  The split path therefore evaluates odd
 // pixel records half a turn further on and negates them (e^{i(x+pi)} = -e^{ix}),
 // so a constant SFU error cancels between neighbouring pixels.
+#include <type_traits>
+
 #include "direct.cuh"
 #include "visibility.cuh"
 
@@ -46,15 +48,21 @@ namespace viss {
 // ======================================================================
 // forward
 // ======================================================================
-template <int NT, int R, int MINB, bool MASKED, bool FP64>
+// NS > 1: that many skies over the same samples (the phase derivative's three),
+// split precision.  A term costs 21 issue slots with one sky and 2 more (an FFMA
+// per part) for each further one, so three take 1.3 times the time of one: 23.0 ms
+// at 194,400 samples x Nside 128 with the Moon, 54 ms as three channels.
+template <int NT, int R, int MINB, bool MASKED, bool FP64, int NS = 1>
 __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
+  static_assert(NS == 1 || !FP64, "several skies: split precision");
   constexpr int S = kFwdStages;
   constexpr int kWarps = NT / 32;
   __shared__ __align__(128) double4 s_pix[S][kTilePix];
+  __shared__ __align__(128) float4 s_sky[NS > 1 ? S : 1][NS > 1 ? kTilePix : 1];
   __shared__ __align__(16) int4 s_refs[MASKED ? R : 1][MASKED ? NT : 1];
   // Kahan (sum, comp) of re and im per sample, kept in shared memory (touched
   // once per tile) so the registers hold only what the inner loop needs
-  __shared__ float s_kahan[FP64 ? 1 : 4][FP64 ? 1 : R][FP64 ? 1 : NT];
+  __shared__ float s_kahan[FP64 ? 1 : 4 * NS][FP64 ? 1 : R][FP64 ? 1 : NT];
   __shared__ __align__(8) uint64_t s_full[S], s_empty[S];
   __shared__ int s_abort;
   volatile int *abort_flag = &s_abort;
@@ -89,18 +97,20 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     d_re[r] = d_im[r] = 0.0;
-    if (!FP64) s_kahan[0][r][tid] = s_kahan[1][r][tid] = s_kahan[2][r][tid] = s_kahan[3][r][tid] = 0.f;
+#pragma unroll
+    for (int c = 0; c < (FP64 ? 0 : 4 * NS); ++c) s_kahan[c][r][tid] = 0.f;
   }
 
   const int t0 = blockIdx.y * p.tiles_per_chunk;
   const int ntile = max(0, min(t0 + p.tiles_per_chunk, p.ntiles) - t0);
-  constexpr uint32_t kTileBytes = kTilePix * sizeof(double4);
+  constexpr uint32_t kTileBytes = kTilePix * sizeof(double4), kSkyBytes = NS > 1 ? kTilePix * sizeof(float4) : 0;
   // test hook (viss_plan_debug_drop_copy): the first CTA never stages one
   // tile, so its bounded waits run out and the error flag is raised
   const int drop = (blockIdx.x == 0 && blockIdx.y == 0) ? min(p.drop_tile, ntile - 1) : -1;
   auto issue = [&](int i, int stage) {
     if (i == drop) return;
-    mbar_expect_tx(&s_full[stage], kTileBytes);
+    mbar_expect_tx(&s_full[stage], kTileBytes + kSkyBytes);
+    if (NS > 1) bulk_g2s(s_sky[stage], p.skies + static_cast<long long>(t0 + i) * kTilePix, kSkyBytes, &s_full[stage]);
     bulk_g2s(s_pix[stage], pix + static_cast<long long>(t0 + i) * kTilePix, kTileBytes,
              &s_full[stage]);
   };
@@ -165,22 +175,33 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
     }
     const double4 *tp = s_pix[stage];
     if (mode != 0) {
-      float t_re[R], t_im[R];
+      float t_re[R][NS], t_im[R][NS];
       double e_re[R], e_im[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) { t_re[r] = t_im[r] = 0.f; e_re[r] = e_im[r] = 0.0; }
+      for (int r = 0; r < R; ++r) {
+        e_re[r] = e_im[r] = 0.0;
+#pragma unroll
+        for (int c = 0; c < NS; ++c) t_re[r][c] = t_im[r][c] = 0.f;
+      }
       if (mode == 2) {
         if ((tid & 31) == 0) evaluated += static_cast<unsigned long long>(nval_warp) * kTilePix;
         for (int j = 0; j < kTilePix; j += 2) {
           const double4 q0 = tp[j], q1 = tp[j + 1];
           const float I0 = sky_of(q0);
           const float I1 = FP64 ? sky_of(q1) : -sky_of(q1);
+          float W0[NS], W1[NS];
+          if (NS > 1) {
+            skies_of<NS>(s_sky[stage][j], true, false, W0);
+            skies_of<NS>(s_sky[stage][j + 1], true, true, W1);
+          }
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const double t0 = fma(uz[r], q0.z, fma(uy[r], q0.y, fma(ux[r], q0.x, mk[r])));
-            fwd_term<FP64>(t0, I0, t_re[r], t_im[r], e_re[r], e_im[r]);
+            if (NS > 1) fwd_term_skies<NS>(t0, W0, t_re[r], t_im[r]);
+            else fwd_term<FP64>(t0, I0, t_re[r][0], t_im[r][0], e_re[r], e_im[r]);
             const double t1 = fma(uz[r], q1.z, fma(uy[r], q1.y, fma(ux[r], q1.x, mk2[r])));
-            fwd_term<FP64>(t1, I1, t_re[r], t_im[r], e_re[r], e_im[r]);
+            if (NS > 1) fwd_term_skies<NS>(t1, W1, t_re[r], t_im[r]);
+            else fwd_term<FP64>(t1, I1, t_re[r][0], t_im[r][0], e_re[r], e_im[r]);
           }
         }
       } else {
@@ -217,14 +238,19 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
             }
             if (sst == 0) continue;
             const double4 *sp = tp + b * kSubPix;
-            if (wn == 0)
-              fwd_span<0, FP64>(sp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r], t_im[r], e_re[r], e_im[r]);
-            else if (wn == 1)
-              fwd_span<1, FP64>(sp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r], t_im[r], e_re[r], e_im[r]);
-            else if (wn == 2)
-              fwd_span<2, FP64>(sp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r], t_im[r], e_re[r], e_im[r]);
-            else
-              fwd_span<3, FP64>(sp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r], t_im[r], e_re[r], e_im[r]);
+            const float4 *wp = s_sky[NS > 1 ? stage : 0] + (NS > 1 ? b * kSubPix : 0);
+            const auto span = [&](auto rows) {
+              constexpr int N = decltype(rows)::value;
+              if (NS > 1)
+                fwd_span_skies<N, NS>(sp, wp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r], t_im[r]);
+              else
+                fwd_span<N, FP64>(sp, ux[r], uy[r], uz[r], mk[r], mk2[r], q0, q1, q2, t_re[r][0], t_im[r][0], e_re[r],
+                                  e_im[r]);
+            };
+            if (wn == 0) span(std::integral_constant<int, 0>());
+            else if (wn == 1) span(std::integral_constant<int, 1>());
+            else if (wn == 2) span(std::integral_constant<int, 2>());
+            else span(std::integral_constant<int, 3>());
           }
         }
       }
@@ -234,12 +260,15 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
           d_re[r] += e_re[r];
           d_im[r] += e_im[r];
         } else {
-          float s0 = s_kahan[0][r][tid], c0 = s_kahan[1][r][tid];
-          float s1 = s_kahan[2][r][tid], c1 = s_kahan[3][r][tid];
-          kahan_add(s0, c0, t_re[r]);
-          kahan_add(s1, c1, t_im[r]);
-          s_kahan[0][r][tid] = s0; s_kahan[1][r][tid] = c0;
-          s_kahan[2][r][tid] = s1; s_kahan[3][r][tid] = c1;
+#pragma unroll
+          for (int c = 0; c < NS; ++c) {
+            float s0 = s_kahan[4 * c][r][tid], c0 = s_kahan[4 * c + 1][r][tid];
+            float s1 = s_kahan[4 * c + 2][r][tid], c1 = s_kahan[4 * c + 3][r][tid];
+            kahan_add(s0, c0, t_re[r][c]);
+            kahan_add(s1, c1, t_im[r][c]);
+            s_kahan[4 * c][r][tid] = s0; s_kahan[4 * c + 1][r][tid] = c0;
+            s_kahan[4 * c + 2][r][tid] = s1; s_kahan[4 * c + 3][r][tid] = c1;
+          }
         }
       }
     }
@@ -248,23 +277,23 @@ __global__ void __launch_bounds__(NT, MINB) k_forward(const FwdParams p) {
   if (tid == 0) ring_drain<S>(s_full, next);
 
   if (p.counter && (tid & 31) == 0) {
-    if (evaluated) atomicAdd(p.counter, evaluated);
-    if (mixed_terms) atomicAdd(p.counter + 2, mixed_terms);
+    if (evaluated) atomicAdd(p.counter, evaluated * NS);
+    if (mixed_terms) atomicAdd(p.counter + 2, mixed_terms * NS);
   }
-  double2 *out = p.part + static_cast<long long>(blockIdx.y) * p.K;
+  double2 *out = p.part + static_cast<long long>(blockIdx.y) * NS * p.K;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const long long k = kb + r * NT + tid;
     if (!kval[r]) continue;
-    double2 v;
     if (FP64) {
-      v.x = d_re[r];
-      v.y = d_im[r];
+      out[k] = make_double2(d_re[r], d_im[r]);
     } else {
-      v.x = static_cast<double>(s_kahan[0][r][tid]) - static_cast<double>(s_kahan[1][r][tid]);
-      v.y = static_cast<double>(s_kahan[2][r][tid]) - static_cast<double>(s_kahan[3][r][tid]);
+#pragma unroll
+      for (int c = 0; c < NS; ++c)
+        out[c * p.K + k] = make_double2(
+            static_cast<double>(s_kahan[4 * c][r][tid]) - static_cast<double>(s_kahan[4 * c + 1][r][tid]),
+            static_cast<double>(s_kahan[4 * c + 2][r][tid]) - static_cast<double>(s_kahan[4 * c + 3][r][tid]));
     }
-    out[k] = v;
   }
 }
 
@@ -604,6 +633,22 @@ cudaError_t launch_forward(const FwdParams &p, int shape, int nchunk, bool maske
     default: return fwd_m<4, 2>(p, nchunk, masked, st);
   }
 }
+
+// Several skies: 128 threads of two samples, whose sums (12 floats per sample) and
+// staged skies fit beside the pixel ring.
+constexpr int kSkiesNT = 128, kSkiesR = 2, kSkiesCtas = 5;
+
+cudaError_t launch_forward_skies(const FwdParams &p, int nchunk, bool masked, cudaStream_t st) {
+  if (p.K <= 0 || p.ntiles <= 0) return cudaSuccess;
+  if (p.channels != 1) return cudaErrorInvalidValue;
+  const long long per = static_cast<long long>(kSkiesNT) * kSkiesR;
+  const dim3 grid(static_cast<unsigned>((p.K + per - 1) / per), nchunk);
+  if (masked) k_forward<kSkiesNT, kSkiesR, kSkiesCtas, true, false, kSkies><<<grid, kSkiesNT, 0, st>>>(p);
+  else k_forward<kSkiesNT, kSkiesR, kSkiesCtas, false, false, kSkies><<<grid, kSkiesNT, 0, st>>>(p);
+  return cudaGetLastError();
+}
+int forward_skies_samples_per_block() { return kSkiesNT * kSkiesR; }
+int forward_skies_ctas_per_sm() { return kSkiesCtas; }
 
 int forward_samples_per_block(int shape, bool fp64) {
   if (fp64) return kFwdNT * 2;

@@ -10,6 +10,8 @@ constexpr int kSampTile = 128;  // samples per adjoint staging tile
 constexpr int kFwdStages = 3;   // shared-memory ring depth: forward pixel tiles
 constexpr int kAdjStages = 4;   // shared-memory ring depth: adjoint sample tiles
 
+constexpr int kSkies = 3;       // skies of one launch_forward_skies
+
 constexpr int kTrackT = 128;    // samples per track block (tracks.cu)
 
 struct FwdParams {
@@ -30,6 +32,7 @@ struct FwdParams {
   long long Kc;                 // samples per channel
   long long pix_stride;         // pixel records per channel's sky (Jpad)
   int drop_tile;                // test hook: CTA (0, 0) skips this tile's copy (-1: none)
+  const float4 *skies = nullptr;   // [Jpad] kSkies values per record (launch_forward_skies; part: [nchunk][kSkies][K])
 };
 
 struct AdjParams {
@@ -112,6 +115,9 @@ constexpr int kNumAdjShapes = 4;
 extern const FwdShape kFwdShapes[kNumFwdShapes];
 extern const AdjShape kAdjShapes[kNumAdjShapes];
 
+cudaError_t launch_forward_skies(const FwdParams &p, int nchunk, bool masked, cudaStream_t st);
+int forward_skies_samples_per_block();
+int forward_skies_ctas_per_sm();
 cudaError_t launch_forward(const FwdParams &p, int shape, int nchunk, bool masked, bool fp64,
                            cudaStream_t st);
 int forward_samples_per_block(int shape, bool fp64);
