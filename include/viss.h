@@ -135,9 +135,9 @@ int viss_plan_set_samples(viss_plan *plan, int64_t K, const double *uvw, const d
  * staged builds them (a few waits for the device, 1-3 ms) and every call then
  * uses device buffers of the plan, about 1 GiB and 1 KiB per sample; without
  * that memory, under stream capture, and for other samples every term is
- * evaluated.  Asynchronous: VISS_OK means the work was launched.  A bounded device-side wait that gave up inside the
- * kernel (V then incomplete) is reported only by the next
- * viss_plan_last_stats / viss_plan_last_counts on this plan, which return
+ * evaluated.  Asynchronous: VISS_OK means the work was launched.  A bounded
+ * device-side wait that gave up inside the kernel (V then incomplete) is
+ * reported only by the next viss_plan_last_stats / viss_plan_last_counts on this plan, which return
  * VISS_ERR_TIMEOUT; callers that need the guarantee check it after the call. */
 int viss_forward(viss_plan *plan, const float *sky, float *V, int flags, void *stream);
 
@@ -177,7 +177,8 @@ int viss_plan_tune(viss_plan *plan, const float *sky, const float *coef, float *
  * frequency grid in the facet's local frame ("exponential of semicircle"
  * kernel, width 7, oversampling 2), one FFT (cuFFT, oversampling 1.5),
  * interpolation at its pixels (width 9).
- * With facet_pixels = 0 and samples on smooth tracks, track blocks (see
+ * With facet_pixels = 0 the direct sum (few samples: a facet's grid costs the
+ * same for any number) or, for samples on smooth tracks, track blocks (see
  * viss_forward) make the image instead where they are modelled faster; the
  * facet choice is reported all the same.
  * Unmasked (VISS_NO_MASK, or no occulter refs): computeC of the noblockage
@@ -204,7 +205,7 @@ int viss_adjoint_gridded(viss_plan *plan, const float *coef, float *image, float
  * shared-memory box (summed over the facets).  Any pointer may be NULL. */
 int viss_plan_gridded_info(viss_plan *plan, int64_t *facet_pixels, int32_t *grid_dims, int64_t *hbm_blocks);
 
-/* Frequency channels:the plan's K samples are `channels` consecutive blocks
+/* Frequency channels: the plan's K samples are `channels` consecutive blocks
  * of K/channels samples (the same baselines at each frequency; K/channels even
  * when channels > 1).  viss_forward then takes sky as channels x J (one map
  * per channel) and viss_adjoint writes image as channels x J; V and coef stay

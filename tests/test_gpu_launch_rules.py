@@ -94,3 +94,34 @@ def test_skies_refuse_odd_counts(cuda_device):
     plan = api.Plan(lmn, torch.ones(3, 3, dtype=torch.float64, device=cuda_device))
     with pytest.raises(RuntimeError, match="must be even"):
         plan._forward_skies(torch.ones(3, len(lmn), device=cuda_device))
+
+
+@pytest.mark.parametrize("masked,accumulate", [(False, False), (True, False), (False, True)])
+def test_gridded_goes_direct_where_that_is_faster(cuda_device, masked, accumulate):
+    """Few samples: the library's choice is the direct sum (the same bits), its
+    facets are reported, a facet size that is asked for is gridded, and gridding's
+    refusal of non-finite coefficients stays."""
+    nside, K = 32, 3001
+    lmn = api.pix2lmn(nside, "ring", device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    uvw = 20 * torch.randn(K, 3, generator=g, device=cuda_device, dtype=torch.float64)
+    refs = occ = None
+    if masked:
+        occ = torch.tensor([[0.0, 0.0, 1.0, -0.5]], device=cuda_device, dtype=torch.float64)
+        refs = torch.tensor([[0, -1, -1]], device=cuda_device, dtype=torch.int32).repeat(K, 1)
+    coef = torch.randn(K, generator=g, device=cuda_device, dtype=torch.complex64)
+    plan = api.Plan(lmn, uvw, None, refs, occ)
+    direct = plan.adjoint(coef, scale=0.5)
+    if accumulate:
+        got = plan.adjoint_gridded(coef, scale=0.5, out=direct.clone(), accumulate=True)
+        assert bool(((got - 2 * direct).abs() <= 2.0 ** -22 * direct.abs()).all())   # the two roundings
+    else:
+        assert torch.equal(plan.adjoint_gridded(coef, scale=0.5), direct)
+    facet = plan.gridded_info()["facet_pixels"]
+    assert facet >= 64
+    gridded = plan.adjoint_gridded(coef, scale=0.5, facet_pixels=facet)
+    assert plan.gridded_info()["facet_pixels"] == facet
+    assert not torch.equal(gridded, direct) and float((gridded - direct).norm()) <= 5e-6 * float(direct.norm())
+    coef[7] = float("nan")
+    with pytest.raises(RuntimeError):
+        plan.adjoint_gridded(coef)

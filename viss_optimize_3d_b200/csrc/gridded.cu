@@ -695,6 +695,11 @@ constexpr double kSecPerCell = 1.6e-11;
 // and per (sample, pixel) pair of a mixed facet left to the direct kernel
 // (tile culling inside the facet included)
 constexpr double kSecPerMixedPair = 3.0e-13;
+// What a mixed pair takes beyond that against another way to the image: the hybrid
+// kernel measured 1.0e-12 s per pair at facets of 4,096 pixels (52 ms of 78 at Nside
+// 256 x 388,800 samples, 0.1 MHz, Moon; 108 of 235 at Nside 512 x 360,000, 0.3 MHz),
+// where the choice between facet sizes was fitted with the figure above.
+constexpr double kSecPerMixedMore = 7.0e-13;
 
 // Grid shape for targets within |x_d| <= X[d] and |u| <= umax.
 GridGeom grid_geom(const double X_in[3], double umax) {
@@ -848,7 +853,7 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
     // every candidate's real extents (and, with occultation, its share of
     // wholly visible and of mixed sample-facet pairs), then the least
     // modelled time
-    double best_t = 1e300;
+    double best_t = 1e300, best_mixed = 0;
     long long last = 0;
     S.choice_version = -1;
     for (long long c = masked ? kHybridAlign : 64;; c *= 4) {
@@ -863,7 +868,7 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
         const double t = nf * (static_cast<double>(K) * open * kGridW * kGridW * kGridW * kSecPerUpdate +
                                cells * kSecPerCell) +
                          static_cast<double>(K) * J * mixed * kSecPerMixedPair;
-        if (t < best_t) best_t = t, fp = c;
+        if (t < best_t) best_t = t, best_mixed = mixed, fp = c;
       }
       if (c >= J) break;
     }
@@ -874,7 +879,7 @@ int gridded_adjoint(void **statep, long long J, const double4 *pix, const int *p
     S.choice_version = geom_version;
     S.choice_masked = masked;
     S.choice_fp = fp;
-    S.choice_seconds = best_t;
+    S.choice_seconds = best_t + static_cast<double>(K) * J * best_mixed * kSecPerMixedMore;
     for (int d = 0; d < 3; ++d) S.choice_dims[d] = chosen.M[d];
     if (other_way()) {
       if (facet_used) *facet_used = fp;
