@@ -27,6 +27,7 @@ import argparse
 import json
 import math
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -96,6 +97,30 @@ ADJ_INSTANCES = ["k_adjoint<128, 8, 4, {m}, 0, 0>", "k_adjoint<128, 8, 5, {m}, 0
                  "k_adjoint<128, 4, 5, {m}, 0, 0>", "k_adjoint<128, 4, 6, {m}, 0, 0>"]
 
 
+def launched_kernels(step):
+    """{name: (launches, device us)} of the library's kernels in one call of
+    `step`, by the profiler, outside the timed region (the counts and the names
+    are used, not the times)."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        step()
+        torch.cuda.synchronize()
+    found = {}
+    for e in prof.key_averages():
+        if "viss::" in e.key:
+            name = re.sub(r"^void |viss::|\(anonymous namespace\)::|\(viss.*$|\((long|int|double|float|unsigned).*$", "", e.key)
+            found[name] = (e.count, e.device_time_total)
+    return found
+
+
+def dominant(kernels, which):
+    """The kernel of that direction ("fwd" / "adj") with the most device time."""
+    names = [k for k in kernels if which in k or {"fwd": "forward", "adj": "adjoint"}[which] in k]
+    return max(names, key=lambda k: kernels[k][1]) if names else None
+
+
 def measured_traffic(workload: str, kernel: str):
     """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum)
     of the kernel instance `kernel` (e.g. "k_adjoint<128, 8, 4, 1, 0, 0>", the
@@ -121,7 +146,6 @@ def record_traffic(csv_path: str, workload: str, command: str, commit: str = "")
     metrics log (dram__bytes_read.sum, dram__bytes_write.sum) into the traffic
     record, keyed by the current kernel sources' sha256."""
     import csv
-    import re
     per = {}
     with open(csv_path) as f:
         lines = [ln for ln in f if ln.startswith('"')]
@@ -339,6 +363,15 @@ def run_ours(args, rank, world, local_rank):
     fwd_ms = [a.elapsed_time(b) for a, b in fwd_ev]
     adj_ms = [a.elapsed_time(b) for a, b in adj_ev]
     total_s = sum(step_ms) / 1e3
+    def plain_step():
+        V1 = g.plan.forward(g.sky)
+        gs1, _c1, dcf1 = api.dcf(g.bll, g.nr, multiplicity=2)
+        _dg1, wt1 = api.weights(g.w, g.bll, gs1, dcf1, g.nr)
+        replicas.add_day_image(day_sum, g.plan.adjoint(api.scale_coef(wt1, V1), scale=2.0, mask=cfg.imaging_mask))
+
+    day_sum_kept = day_sum.clone()
+    kernels = launched_kernels(plain_step)
+    day_sum.copy_(day_sum_kept)
     # culled fraction of the last forward/adjoint (device counters); also
     # raises if a bounded device-side wait gave up in either kernel
     g.plan.forward(g.sky)
@@ -458,6 +491,9 @@ def run_ours(args, rank, world, local_rank):
                  "adjoint": J * 32 + K * 48 + G * 48 + K * 8 + J * 4}[dom]
     masked = 1 if obs.refs is not None else 0
     inst = (FWD_INSTANCES[shapes[0]] if dom == "forward" else ADJ_INSTANCES[shapes[1]]).format(m=masked)
+    by_tracks = any(k.startswith("k_track_") for k in kernels)
+    if by_tracks:    # most exponentials interpolated: the slowest kernel of the direction stands for it
+        inst = dominant(kernels, "fwd" if dom == "forward" else "adj")
     traffic, traffic_src = measured_traffic(args.workload, inst)
     res = {
         "metric": METRIC,
@@ -478,7 +514,9 @@ def run_ours(args, rank, world, local_rank):
                 "path": "pinned host sky/uvw/refs/satellite positions/Earth rows -> viss_occulters -> "
                         "viss_plan_set_samples -> viss_forward -> viss_dcf/viss_weights -> viss_adjoint "
                         "-> pinned host V/image"},
-        "roofline": {"bound": "sfu", "kernel": f"k_{dom}",
+        "roofline": {"bound": "sfu", "kernel": inst.split("<")[0] if by_tracks else f"k_{dom}",
+                     **({"note": "track blocks: frac counts every term, most of them interpolated (no "
+                                 "exponential); frac_of_evaluated the exponentials"} if by_tracks else {}),
                      "achieved": round(achieved / 1e9, 2), "peak": round(peak_terms / 1e9, 1),
                      "unit": "Gterms/s", "frac": round(achieved / peak_terms, 4),
                      "peak_source": f"8 terms/clk/SM x {nsm} SMs x sm_max_mhz ({pk_kind})",
@@ -492,11 +530,13 @@ def run_ours(args, rank, world, local_rank):
                     "adjoint_evaluated": round(ev_a / tot, 4), "adjoint_mixed": round(mx_a / tot, 4)},
         "day_sum": {"ranks": world, "reduction": "NCCL all-reduce (SUM) of the FP64 day sums"
                     if world > 1 else "single rank: device day sum only", "finite": day_sum_ok},
-        "gpu_launches": 11 * args.steps,
+        "gpu_launches": sum(n for n, _t in kernels.values()) * args.steps,
         "fp64_path": fp64,
         "tuning": {"chosen": {"forward": shapes[0], "adjoint": shapes[1]},
                    "forward_shapes": "(samples/thread, CTAs/SM) = (4,2) (4,3) (2,3) (2,4)",
                    "adjoint_shapes": "(pixels/lane, CTAs/SM), 128-thread CTAs = (8,4) (8,5) (4,5) (4,6)",
+                   **({"track_blocks": "the calls go through track blocks, which have no launch shapes"}
+                      if by_tracks else {}),
                    **({"note": "fixed at the headline size's choice (no sweep at this size)"} if big else sweep)},
         "clocks": clk,
     }
@@ -571,6 +611,7 @@ def run_formation(args, rank, world, local_rank):
     total_s = sum(e[0].elapsed_time(e[3]) for e in ev) / 1e3
     fwd_s = statistics.mean(e[0].elapsed_time(e[1]) for e in ev) / 1e3
     adj_s = statistics.mean(e[2].elapsed_time(e[3]) for e in ev) / 1e3
+    kernels = launched_kernels(lambda: image(plan.forward_formation(g.sky)))
     plan.forward_formation(g.sky)
     ev_f, mx_f, tot = plan.last_stats()
     plan.adjoint_formation(coef, scale=2.0, mask=cfg.imaging_mask)
@@ -630,12 +671,14 @@ def run_formation(args, rank, world, local_rank):
     total_s, e2e_s = replicas.max_over_ranks([total_s, e2e_s], device=dev)
     if rank != 0:
         return None
-    traffic, traffic_src = measured_traffic(
-        args.workload, f"k_form_{'forward' if fwd_s >= adj_s else 'adjoint'}<{plan.form_S}>")
+    dom = "forward" if fwd_s >= adj_s else "adjoint"
+    by_tracks = any(k.startswith("k_track_") for k in kernels)
+    inst = dominant(kernels, "fwd" if dom == "forward" else "adj") if by_tracks else f"k_form_{dom}<{plan.form_S}>"
+    traffic, traffic_src = measured_traffic(args.workload, inst)
     pk, pk_kind = peaks()
     nsm = torch.cuda.get_device_properties(dev).multi_processor_count
-    peak_terms = 128 / FORM_FFMA_PER_TERM * nsm * pk["sm_max_mhz"] * 1e6
-    dom = "forward" if fwd_s >= adj_s else "adjoint"
+    per_clk = MUFU_TERMS_PER_CLK_PER_SM if by_tracks else 128 / FORM_FFMA_PER_TERM
+    peak_terms = per_clk * nsm * pk["sm_max_mhz"] * 1e6
     dom_s = max(fwd_s, adj_s)
     dom_eval = ev_f if dom == "forward" else ev_a
     achieved = K * J / dom_s
@@ -658,11 +701,12 @@ def run_formation(args, rank, world, local_rank):
                 "path": "pinned host sky/satellite positions/Earth rows -> U and viss_occulters on the "
                         "device -> viss_plan_set_formation -> viss_forward_formation -> "
                         "viss_dcf/viss_weights -> viss_adjoint_formation -> pinned host V/image"},
-        "roofline": {"bound": "fp32", "kernel": f"k_form_{dom}",
+        "roofline": {"bound": "sfu" if by_tracks else "fp32", "kernel": inst.split("<")[0],
                      "achieved": round(achieved / 1e9, 2), "peak": round(peak_terms / 1e9, 1),
                      "unit": "Gterms/s", "frac": round(achieved / peak_terms, 4),
-                     "peak_source": f"128 FP32 lanes/clk/SM / {FORM_FFMA_PER_TERM} FFMA per term x {nsm} SMs "
-                                    f"x sm_max_mhz ({pk_kind})",
+                     "peak_source": ("8 terms/clk/SM (track blocks)" if by_tracks else
+                                     f"128 FP32 lanes/clk/SM / {FORM_FFMA_PER_TERM} FFMA per term")
+                                    + f" x {nsm} SMs x sm_max_mhz ({pk_kind})",
                      "evaluated_frac": round(dom_eval / (K * J), 4),
                      "traffic": traffic, "traffic_unit": "DRAM bytes per launch",
                      "traffic_source": traffic_src},
@@ -670,7 +714,7 @@ def run_formation(args, rank, world, local_rank):
         "culling": {"forward_evaluated": round(ev_f / tot, 4), "forward_general_path": round(mx_f / tot, 4),
                     "adjoint_evaluated": round(ev_a / tot, 4), "adjoint_general_path": round(mx_a / tot, 4)},
         "forward_rel_l2_vs_direct": float(f"{rel_v:.3e}"),
-        "gpu_launches": 10 * args.steps,
+        "gpu_launches": sum(n for n, _t in kernels.values()) * args.steps,
         "clocks": clk,
     }
     return res

@@ -973,7 +973,7 @@ static int form_tracks_ready(viss_plan *p, bool masked, bool adjoint, cudaStream
   }
   const viss::TrackInputs in = form_track_inputs(p);
   *use = p->form_tracks_usable &&
-         viss::tracks_seconds(p->form_tracks, in, masked, adjoint) < 0.95 * per_term * static_cast<double>(in.K) * in.J;
+         viss::tracks_seconds(p->form_tracks, in, masked, adjoint) < per_term * static_cast<double>(in.K) * in.J;
   return VISS_OK;
 }
 

@@ -26,11 +26,13 @@
 // block stops when its mean squared prediction error, node errors included, is
 // below 1.8 kNodeNoise^2 (no sample above 4.5): (2.7e-7)^2, where a term that
 // k_forward evaluates is off by 3.7e-7 (a phase of 23 bits).  Measured against
-// FP64 on 1 and 10 MHz Nside 256 observations: V 2.6e-7 - 3.7e-7 and images of
-// random coefficients 4.2e-7, the direct kernels 3.6e-7 - 5.2e-7 and 5.6e-7.
+// FP64 on 1 and 10 MHz Nside 256 observations: V 2.4e-7 - 3.5e-7, images of random
+// coefficients 4.2e-7 and of the observations 3.0e-7 - 4.5e-7; the direct kernels
+// 2.5e-7 - 4.6e-7, 5.0e-7 and 2.6e-7 - 5.4e-7.
 // Stopping at 0.85 (3e-7)^2 with the same node error costs 25 % more nodes
-// for 8 % less error, stopping at 2.5 saves 1 %.  Blocks that need more than kTrackRankMax nodes, or
-// three quarters of their samples, are left to the remainder kernels.
+// for 8 % less error, stopping at 2.5 saves 1 %.  Blocks that need more than
+// kTrackRankMax nodes, or three quarters of their samples, are left to the
+// remainder kernels.
 //
 // Group size.  Long baselines turn faster: every block takes the group size
 // (64, 128, 256 or 1024 pixels) with the least modelled time, and blocks of one
