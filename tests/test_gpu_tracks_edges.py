@@ -1,0 +1,57 @@
+"""Track blocks (csrc/tracks*.cu) on the inputs at the edge of their rules.
+Tolerances as in test_gpu_tracks.py; every case says which path evaluated it.
+"""
+import pytest
+import torch
+
+from viss_optimize_3d_b200 import api, synth
+
+from test_gpu_tracks import close, observation, tables
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(plan, dev, seed=3):
+    g = torch.Generator(device=dev).manual_seed(seed)
+    return (torch.rand(plan.J, generator=g, device=dev) + 0.1,
+            torch.randn(plan.K, generator=g, device=dev, dtype=torch.complex64))
+
+
+def by_blocks(plan):
+    """The last call evaluated far fewer exponentials than terms."""
+    evaluated, _, total = plan.last_stats()
+    return evaluated < total // 2
+
+
+def two_patches(n, dev):
+    """n directions in two caps of 8 degrees, far apart."""
+    g = torch.Generator(device=dev).manual_seed(11)
+    c = torch.tensor([[0.36, 0.48, 0.8], [-0.8, 0.6, 0.0]], device=dev, dtype=torch.float64)
+    d = c[torch.arange(n, device=dev) % 2] + 0.08 * (2 * torch.rand(n, 3, generator=g, device=dev, dtype=torch.float64) - 1)
+    return torch.nn.functional.normalize(d, dim=1)
+
+
+@pytest.mark.parametrize("pixels,n_sat,n_snap,f_hz,moon", [
+    (57, 10, 6000, 2e4, False),     # a tile across two base faces, wider than every group of 1,024
+    (57, 10, 6000, 2e4, True),      # the same of a plan with occulters, unmasked
+    (55, 10, 6200, 2e4, False),
+    ("patches", 10, 6000, 2e4, False),
+])
+def test_tiles_wider_than_their_group(cuda_device, pixels, n_sat, n_snap, f_hz, moon):
+    """Unocculted calls of slow tracks: no tile is left out."""
+    obs = observation(64 if pixels == "patches" else pixels, n_sat, n_snap, f_hz, moon, False)
+    lmn = two_patches(40000, cuda_device) if pixels == "patches" else api.pix2lmn(pixels, "ring", device=cuda_device)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(lmn, torch.as_tensor(obs.uvw(f_hz), device=cuda_device), None, refs, occ)
+    assert plan.K * plan.J >= 1e10
+    sky, coef = inputs(plan, cuda_device)
+    V, img = plan.forward(sky, fp64=True, mask=False), plan.adjoint(coef, fp64=True, mask=False)
+    close(plan.forward(sky, mask=False), V)
+    assert by_blocks(plan)
+    close(plan.adjoint(coef, mask=False), img)
+    assert by_blocks(plan)
+    P = torch.as_tensor(obs.positions, device=cuda_device)
+    plan.set_formation((P - P.mean(dim=1, keepdim=True)) / (synth.C_LIGHT / f_hz))
+    close(plan.forward_formation(sky), V)
+    assert by_blocks(plan)
+    close(plan.adjoint_formation(coef), img)

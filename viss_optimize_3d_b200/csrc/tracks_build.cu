@@ -252,13 +252,14 @@ __device__ __forceinline__ unsigned valid_tiles(int w, int ntiles) {
 
 // Rows of class c (kClasses: blocks without nodes) for unocculted sums: the
 // tiles whose group is within the class's radius (radius: per class, its
-// groups', concatenated from at[c]), merged tiles, and the others.
+// groups', concatenated from at[c]), merged tiles, and the others.  left: bit c
+// set where class c leaves a tile.
 struct ClassSet {
   double rho[kClasses];
   int at[kClasses];
 };
 __global__ void k_track_class_rows(int W, int ntiles, const float *radius, ClassSet cs, unsigned *full,
-                                   unsigned *merged, unsigned *rest) {
+                                   unsigned *merged, unsigned *rest, unsigned long long *left) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
   if (w >= W) return;
   const unsigned valid = valid_tiles(w, ntiles);
@@ -278,6 +279,7 @@ __global__ void k_track_class_rows(int W, int ntiles, const float *radius, Class
   full[c * W + w] = ok;
   merged[c * W + w] = merged_tiles(ok, valid, c);
   rest[c * W + w] = valid & ~ok;
+  if (valid & ~ok) atomicOr(left, 1ull << c);
 }
 
 // A sample's three classification rows (absent: sees everything), and its
@@ -440,13 +442,13 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   int *trial_rank_d;
   unsigned long long *counts_d;
   if (!S.trial.reset(TrackArena::bytes<double4>(total) + TrackArena::bytes<float>(total) + TrackArena::bytes<float>(lags) +
-                     TrackArena::bytes<int>(kRadii * kRankSamples) + TrackArena::bytes<unsigned long long>(3)))
+                     TrackArena::bytes<int>(kRadii * kRankSamples) + TrackArena::bytes<unsigned long long>(4)))
     return 0;
   S.trial.take(S.gcen, total);
   S.trial.take(radius_d, total);
   S.trial.take(score_d, lags);
   S.trial.take(trial_rank_d, kRadii * kRankSamples);
-  S.trial.take(counts_d, 3);
+  S.trial.take(counts_d, 4);
   for (int c = 0; c < kClasses; ++c) {
     k_track_groups<<<blks(ngs[c], 8), 256, 0, st>>>(ngs[c], group_pix(c), in.Jpad, in.pix, S.gcen + S.gat[c],
                                                     radius_d + S.gat[c]);
@@ -546,14 +548,11 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   chosen[kHalf] = true;
   RadiusSet radii{}, some{};
   ClassSet cs{};
-  bool wide[kClasses + 1] = {};
-  wide[kClasses] = true;
   int nclass = 0, class_of[kClasses];
   for (int c = 0; c < kClasses; ++c) {
     cs.rho[c] = radii.rho[c] = trial.rho[pick_q[c]];
     radii.most[c] = trial.most[pick_q[c]];
     cs.at[c] = S.gat[c];
-    wide[c] = within[pick_q[c]] < 1.0;
     if (!chosen[c]) continue;
     some.rho[nclass] = radii.rho[c];
     some.most[nclass] = radii.most[c];
@@ -651,30 +650,30 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   k_track_weights<<<nb, kTrackT, sizeof(TrackFactor), st>>>(S.slot, S.samp, radii, S.cls, S.rank, S.noff, S.node,
                                                            S.nodeblk, S.P);
   TRACK_CUDA(cudaGetLastError(), "weights");
+  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 4 * sizeof(unsigned long long), st), "counts");
   k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, radius_d, cs, S.crow[0],
-                                                                         S.crow[1], S.crow[2]);
+                                                                         S.crow[1], S.crow[2], counts_d + 2);
   TRACK_CUDA(cudaGetLastError(), "class rows");
-  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 3 * sizeof(unsigned long long), st), "counts");
   const unsigned by = static_cast<unsigned>(std::max(1, std::min(S.W / 8, (4 * in.nsm * 8) / nb + 1)));
   if (masked) {
     k_track_bits<<<dim3(nb, by), 128, 0, st>>>(S.W, in.ntiles, S.slot, S.refs, in.occ32, in.cones, S.cls, S.crow[0],
                                                S.brow[0], S.brow[1], S.brow[2], S.brow[3], counts_d);
     TRACK_CUDA(cudaGetLastError(), "pair bits");
   }
-  unsigned long long pairs_of[2] = {0, 0};         // rest, part
+  unsigned long long pairs_of[3] = {0, 0, 0};      // rest, part, classes that leave tiles
   TRACK_CUDA(cudaMemcpyAsync(pairs_of, counts_d, sizeof(pairs_of), cudaMemcpyDeviceToHost, st), "counts");
   TRACK_CUDA(cudaStreamSynchronize(st), "build");
   if (masked) {
     if (pairs_of[1] > INT_MAX || !S.masks.reset(TrackArena::bytes<uint4>(pairs_of[1]))) return 0;
     S.masks.take(S.mask, pairs_of[1]);
     k_track_masks<<<dim3(nb, by), 128, 0, st>>>(S.W, S.slot, S.refs, in.occ32, in.cones, S.brow[1], S.mask_at, S.mask,
-                                                counts_d + 2);
+                                                counts_d + 3);
     TRACK_CUDA(cudaGetLastError(), "sample masks");
     TRACK_CUDA(cudaStreamSynchronize(st), "build");  // later calls may come on other streams
   }
   S.has_rest[1] = pairs_of[0] != 0;
-  S.has_rest[0] = false;                           // unocculted: wide groups, blocks without nodes
-  for (const TrackSlab &sl : S.slabs) S.has_rest[0] = S.has_rest[0] || wide[sl.cls] || wide[kTile];
+  S.has_rest[0] = false;                           // unocculted: tiles a used class leaves
+  for (const TrackSlab &sl : S.slabs) S.has_rest[0] = S.has_rest[0] || (pairs_of[2] >> sl.cls & 1u);
   S.cost = mean;
   *usable = true;
   return 0;
