@@ -55,3 +55,20 @@ def test_tiles_wider_than_their_group(cuda_device, pixels, n_sat, n_snap, f_hz, 
     close(plan.forward_formation(sky), V)
     assert by_blocks(plan)
     close(plan.adjoint_formation(coef), img)
+
+
+def test_pixel_that_is_no_direction(cuda_device):
+    """A NaN pixel stays in its own terms: every other image pixel is what it
+    was, through blocks and without them."""
+    obs = observation(57, 10, 6000, 2e4, False, False)
+    lmn = api.pix2lmn(57, "ring", device=cuda_device).clone()
+    bad = 12345
+    lmn[bad] = float("nan")
+    plan = api.Plan(lmn, torch.as_tensor(obs.uvw(2e4), device=cuda_device))
+    _, coef = inputs(plan, cuda_device)
+    keep = torch.arange(plan.J, device=cuda_device) != bad
+    want = plan.adjoint(coef, fp64=True)
+    got = plan.adjoint(coef)
+    assert by_blocks(plan)
+    assert bool(torch.isfinite(want[keep]).all())
+    close(got[keep], want[keep])

@@ -487,7 +487,8 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   // A class's radius: a percentile of its groups' (wider groups are left) with
   // the least time over some blocks.  On a power-of-two HEALPix grid all groups
   // are alike and the largest wins; elsewhere a few are far wider than the rest.
-  // A group of more than 64 pixels is only worth it with few nodes.
+  // A group of more than 64 pixels is only worth it with few nodes.  A share that
+  // takes in a group with a NaN pixel (radius +inf) is no radius: nothing within it.
   const double share[kShares] = {1.0, 0.99, 0.97, 0.9};
   RadiusSet trial{};
   double within[kRadii];
@@ -496,6 +497,8 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     for (int q = 0; q < kShares; ++q) {
       const int i = std::min(ngs[c] - 1, static_cast<int>(share[q] * ngs[c])), at = c * kShares + q;
       std::nth_element(b, b + i, e);
+      within[at] = 0;
+      if (!std::isfinite(b[i])) continue;            // at most 0 nodes: every block's rank is 0
       trial.rho[at] = b[i] * (1.0 + 1e-6);
       trial.most[at] = c == kHalf ? kTrackRankMax : kTrackRankMax / 2;
       within[at] = std::count_if(b, e, [&](float v) { return v <= static_cast<float>(trial.rho[at]); }) /
