@@ -72,3 +72,19 @@ def test_pixel_that_is_no_direction(cuda_device):
     assert by_blocks(plan)
     assert bool(torch.isfinite(want[keep]).all())
     close(got[keep], want[keep])
+
+
+def test_pixels_beyond_the_unit_sphere(cuda_device):
+    """Vectors that are no directions (a few of length 4) and baselines near the
+    blocks' bound: their phases do not fit the blocks' fixed point."""
+    n = 44000
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+    lmn = torch.nn.functional.normalize(torch.randn(n, 3, generator=g, device=cuda_device, dtype=torch.float64), dim=1)
+    lmn[::1000] *= 4.0
+    # one baseline that stays where it is: a single node serves a block, whatever the group's width
+    uvw = torch.tensor([[1.5e5, -5e4, 4e4]], device=cuda_device, dtype=torch.float64).repeat(240000, 1)
+    plan = api.Plan(lmn, uvw)
+    sky, coef = inputs(plan, cuda_device)
+    # 44 terms of a wrong phase move a value by a few percent, and their pixels by all of it
+    for got, want in ((plan.forward(sky), plan.forward(sky, fp64=True)), (plan.adjoint(coef), plan.adjoint(coef, fp64=True))):
+        assert float((got - want).abs().max()) <= 1e-4 * float(want.abs().square().mean().sqrt())

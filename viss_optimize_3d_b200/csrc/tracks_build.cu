@@ -29,7 +29,9 @@ constexpr int kRadii = kClasses * kShares;
 constexpr size_t kSlabBytes = 1ull << 28;
 
 // Pixel groups of gp pixels: centre (normalised mean direction) and the largest
-// chord from it to a pixel, rounded up; a NaN pixel makes the radius +inf.
+// chord from it to a pixel, rounded up; +inf with a pixel that is NaN or longer
+// than 2 (its phases could reach 2^19 turns: tracks_build bounds those of unit
+// vectors by 2^18).
 __global__ void k_track_groups(int ng, int gp, long long Jpad, const double4 *pix, double4 *gcen, float *radius) {
   const int g = static_cast<int>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
   if (g >= ng) return;
@@ -53,7 +55,7 @@ __global__ void k_track_groups(int ng, int gp, long long Jpad, const double4 *pi
     const double4 p = pix[i];
     const double dx = p.x - c.x, dy = p.y - c.y, dz = p.z - c.z;
     const double d = sqrt(dx * dx + dy * dy + dz * dz);
-    bad = bad || !(d == d);
+    bad = bad || !(d == d) || !(p.x * p.x + p.y * p.y + p.z * p.z <= 4.0);
     r = fmax(r, d);
   }
   for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
@@ -423,7 +425,7 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   if (!*statep) *statep = new (std::nothrow) TrackState();
   if (!*statep) return 0;
   TrackState &S = *static_cast<TrackState *>(*statep);
-  if (!(in.max_turns < 262144.0)) return 0;        // fine_cis: |u.s + off| < 2^19 turns
+  if (!(in.max_turns < 262144.0)) return 0;        // fine_cis: |u.s + off| < 2^19 turns, |s| <= 2
   if (in.K > INT_MAX / 2 || in.ntiles < 8 || in.ntiles > INT_MAX / 16) return 0;
   const int lags = static_cast<int>(std::min<long long>(kLagMax, in.Kc / 32));
   if (lags < 1) return 0;
@@ -488,7 +490,7 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   // the least time over some blocks.  On a power-of-two HEALPix grid all groups
   // are alike and the largest wins; elsewhere a few are far wider than the rest.
   // A group of more than 64 pixels is only worth it with few nodes.  A share that
-  // takes in a group with a NaN pixel (radius +inf) is no radius: nothing within it.
+  // takes in a group that has none (radius +inf) is no radius: nothing within it.
   const double share[kShares] = {1.0, 0.99, 0.97, 0.9};
   RadiusSet trial{};
   double within[kRadii];
