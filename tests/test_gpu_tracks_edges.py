@@ -88,3 +88,26 @@ def test_pixels_beyond_the_unit_sphere(cuda_device):
     # 44 terms of a wrong phase move a value by a few percent, and their pixels by all of it
     for got, want in ((plan.forward(sky), plan.forward(sky, fp64=True)), (plan.adjoint(coef), plan.adjoint(coef, fp64=True))):
         assert float((got - want).abs().max()) <= 1e-4 * float(want.abs().square().mean().sqrt())
+
+
+def test_skies_through_the_blocks(cuda_device):
+    """Three skies a block at a time, and the same call captured afterwards
+    (which evaluates every term, in buffers that are there already)."""
+    obs = observation(57, 10, 6000, 2e4, False, False)
+    plan = api.Plan(api.pix2lmn(57, "ring", device=cuda_device), torch.as_tensor(obs.uvw(2e4), device=cuda_device))
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    sky = torch.randn(3, plan.J, generator=g, device=cuda_device) + 0.5
+    want = plan._forward_skies(sky, fp64=True)
+    got = plan._forward_skies(sky)
+    evaluated, _, total = plan.last_stats()
+    assert total == 3 * plan.K * plan.J and evaluated < total // 2
+    for c in range(3):
+        close(got[c], want[c])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = plan._forward_skies(sky)
+    graph.replay()
+    assert plan.last_stats()[0] >= total            # and the padding of the last tiles
+    for c in range(3):
+        close(out[c], want[c])

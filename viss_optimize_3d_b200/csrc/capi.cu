@@ -655,7 +655,18 @@ int viss_forward_skies(viss_plan *p, int n, const float *sky, float *V, int flag
   const cudaStream_t st = as_stream(stream);
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
   bool three = n == viss::kSkies && !(flags & VISS_FP64);
+  viss::FwdParams fp;
+  int nchunk = 0;
   if (three) {
+    const long long per = viss::forward_skies_samples_per_block();
+    const long long blocks = (p->K + per - 1) / per;
+    long long c = (static_cast<long long>(p->fwd_waves) * p->nsm * viss::forward_skies_ctas_per_sm() + blocks - 1) / blocks;
+    c = std::max<long long>(1, std::min<long long>(c, p->ntiles));
+    fp.tiles_per_chunk = static_cast<int>((p->ntiles + c - 1) / c);
+    nchunk = (p->ntiles + fp.tiles_per_chunk - 1) / fp.tiles_per_chunk;
+    // before the choice: a captured call evaluates every term, whatever the calls before it took
+    if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * n * p->K)) return s;
+    if (int s = ensure(p->skies, p->skies_cap, sizeof(float4) * p->Jpad, "sky records")) return s;
     bool use = false;
     if (int s = tracks_ready(p, st, &use)) return s;
     three = !use || n * viss::tracks_seconds(p->tracks, track_inputs(p), masked, false) >
@@ -667,15 +678,6 @@ int viss_forward_skies(viss_plan *p, int n, const float *sky, float *V, int flag
     p->last_total = n * p->K * p->J;
     return VISS_OK;
   }
-  const long long per = viss::forward_skies_samples_per_block();
-  const long long blocks = (p->K + per - 1) / per;
-  long long c = (static_cast<long long>(p->fwd_waves) * p->nsm * viss::forward_skies_ctas_per_sm() + blocks - 1) / blocks;
-  c = std::max<long long>(1, std::min<long long>(c, p->ntiles));
-  viss::FwdParams fp;
-  fp.tiles_per_chunk = static_cast<int>((p->ntiles + c - 1) / c);
-  const int nchunk = (p->ntiles + fp.tiles_per_chunk - 1) / fp.tiles_per_chunk;
-  if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * n * p->K)) return s;
-  if (int s = ensure(p->skies, p->skies_cap, sizeof(float4) * p->Jpad, "sky records")) return s;
   VISS_CUDA(viss::launch_stage_skies(p->J, p->Jpad, p->perm, sky, p->skies, p->dev_words, st), "viss_forward_skies: sky");
   fp.samp = p->samp;
   fp.refs = masked ? p->refs : nullptr;
