@@ -125,3 +125,30 @@ def test_gridded_goes_direct_where_that_is_faster(cuda_device, masked, accumulat
     coef[7] = float("nan")
     with pytest.raises(RuntimeError):
         plan.adjoint_gridded(coef)
+
+
+@pytest.mark.parametrize("nside,K", [(64, 20001), (48, 30000)])
+def test_captured_calls_outlive_other_calls(cuda_device, nside, K):
+    """A captured unocculted call keeps its workspace when occulted calls, which
+    take other launch shapes, follow on the same samples."""
+    lmn = api.pix2lmn(nside, "ring", device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(7)
+    uvw = 40 * torch.randn(K, 3, generator=g, device=cuda_device, dtype=torch.float64)
+    occ = torch.tensor([[0.0, 0.6, 0.8, -0.3]], device=cuda_device, dtype=torch.float64)
+    refs = torch.tensor([[0, -1, -1]], device=cuda_device, dtype=torch.int32).repeat(K, 1)
+    sky = torch.rand(len(lmn), generator=g, device=cuda_device) + 0.1
+    coef = torch.randn(K, generator=g, device=cuda_device, dtype=torch.complex64)
+    plan = api.Plan(lmn, uvw, None, refs, occ)
+    V, img = torch.empty(K, dtype=torch.complex64, device=cuda_device), torch.empty(len(lmn), device=cuda_device)
+    for call, out in ((lambda **kw: plan.forward(sky, **kw), V), (lambda **kw: plan.adjoint(coef, **kw), img)):
+        want = call(mask=False)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call(mask=False, out=out)
+        masked = call()
+        others = [torch.full((1 << 18,), 7.0, device=cuda_device) for _ in range(8)]   # over what was freed
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and not torch.equal(masked, want)
+        assert all(bool((o == 7.0).all()) for o in others)

@@ -275,6 +275,21 @@ int auto_adj_shape(const viss_plan *p, bool masked) {
   return adj_load(p, 3) < 0.93 * adj_load(p, 1) ? 3 : 1;
 }
 
+// Bytes of the workspace for any forward or adjoint call on the plan's samples,
+// with the plan's shapes or (-1) any that it may pick, occulted or not: a call must
+// not move the workspace that captured calls hold the address of.
+size_t call_workspace(const viss_plan *p, int fwd_shape, int adj_shape, bool fp64) {
+  size_t bytes = 0;
+  int spc = 0;
+  for (int s = 0; s < viss::kNumFwdShapes; ++s)
+    if (fwd_shape == s || (fwd_shape < 0 && s != 1 && s != 3))
+      bytes = std::max(bytes, sizeof(double2) * static_cast<size_t>(fwd_chunks(p, s, fp64)) * p->K);
+  for (int s = 0; s < viss::kNumAdjShapes; ++s)
+    if (adj_shape == s || (adj_shape < 0 && s != 2))
+      bytes = std::max(bytes, sizeof(double) * static_cast<size_t>(adj_chunks(p, s, fp64, &spc)) * p->channels * p->Jpad);
+  return bytes;
+}
+
 cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 
 }  // namespace
@@ -567,9 +582,9 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                         int shape, bool tracks = true, bool first = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
+  if (int s = workspace(p, call_workspace(p, shape, p->adj_shape, fp64))) return s;
   if (shape < 0) shape = auto_fwd_shape(p, masked);
   const int nchunk = fwd_chunks(p, shape, fp64);
-  if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * p->K)) return s;
   if (int s = ensure(p->pixsky, p->pixsky_cap, sizeof(double4) * p->Jpad * p->channels,
                      "pixel+sky records"))
     return s;
@@ -715,11 +730,10 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
                         bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
+  if (int s = workspace(p, call_workspace(p, p->fwd_shape, shape, fp64))) return s;
   if (shape < 0) shape = fcones ? 0 : auto_adj_shape(p, masked);
   int spc = 0;
   const int nchunk = adj_chunks(p, shape, fp64, &spc);
-  if (int s = workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * p->channels * p->Jpad))
-    return s;
   VISS_CUDA(viss::launch_stage_coef(p->K, p->Kpad, reinterpret_cast<const float2 *>(coef), p->coef, !fp64, p->dev_words,
                                     st),
             "viss_adjoint: coef");
