@@ -283,10 +283,10 @@ size_t call_workspace(const viss_plan *p, int fwd_shape, int adj_shape, bool fp6
   int spc = 0;
   for (int s = 0; s < viss::kNumFwdShapes; ++s)
     if (fwd_shape == s || (fwd_shape < 0 && s != 1 && s != 3))
-      bytes = std::max(bytes, sizeof(double2) * static_cast<size_t>(fwd_chunks(p, s, fp64)) * p->K);
+      bytes = std::max<size_t>(bytes, sizeof(double2) * static_cast<size_t>(fwd_chunks(p, s, fp64)) * p->K);
   for (int s = 0; s < viss::kNumAdjShapes; ++s)
     if (adj_shape == s || (adj_shape < 0 && s != 2))
-      bytes = std::max(bytes, sizeof(double) * static_cast<size_t>(adj_chunks(p, s, fp64, &spc)) * p->channels * p->Jpad);
+      bytes = std::max<size_t>(bytes, sizeof(double) * static_cast<size_t>(adj_chunks(p, s, fp64, &spc)) * p->channels * p->Jpad);
   return bytes;
 }
 
