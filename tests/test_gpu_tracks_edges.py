@@ -4,7 +4,7 @@ Tolerances as in test_gpu_tracks.py; every case says which path evaluated it.
 import pytest
 import torch
 
-from viss_optimize_3d_b200 import api, synth
+from viss_optimize_3d_b200 import _capi, api, synth
 
 from test_gpu_tracks import close, observation, tables
 
@@ -111,3 +111,22 @@ def test_skies_through_the_blocks(cuda_device):
     assert plan.last_stats()[0] >= total            # and the padding of the last tiles
     for c in range(3):
         close(out[c], want[c])
+
+
+@pytest.mark.parametrize("tile", [1, 10 ** 6])
+@pytest.mark.parametrize("call", ["forward", "adjoint"])
+@pytest.mark.parametrize("f_hz", [2e4, 2e6])      # groups of 1,024 pixels; of 64 among others
+def test_wait_that_gives_up(cuda_device, call, tile, f_hz):
+    """A staging copy that never comes (a tile past the last one stands for the
+    last): the call ends, the next status read reports it, the plan goes on."""
+    obs = observation(57, 10, 6000, f_hz, False, False)
+    plan = api.Plan(api.pix2lmn(57, "ring", device=cuda_device), torch.as_tensor(obs.uvw(f_hz), device=cuda_device))
+    sky, coef = inputs(plan, cuda_device)
+    run = (lambda **kw: plan.forward(sky, **kw)) if call == "forward" else (lambda **kw: plan.adjoint(coef, **kw))
+    run()
+    assert by_blocks(plan)
+    _capi.check(_capi.lib.viss_plan_debug_drop_copy(plan._h, tile), "viss_plan_debug_drop_copy")
+    run()
+    with pytest.raises(_capi.VissError, match="gave up"):
+        plan.last_stats()
+    close(run(), run(fp64=True))

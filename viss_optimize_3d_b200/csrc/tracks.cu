@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
   }
   const int t0 = blockIdx.y * p.per_chunk, ntile = max(0, min(t0 + p.per_chunk, p.ntiles) - t0);
   const int gt = group_tiles(p.cls);
-  const int drop = (blockIdx.x == 0 && blockIdx.y == 0) ? p.drop_tile : -1;
+  const int drop = (blockIdx.x == 0 && blockIdx.y == 0) ? min(p.drop_tile, ntile - 1) : -1;   // test hook (k_forward)
   constexpr uint32_t kTileBytes = kTilePix * sizeof(double4);
   auto issue = [&](int i, int stage) {
     if (i == drop) return;
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
   const int ntile = max(0, (n1 - n0 + kAdjNodeTile - 1) / kAdjNodeTile);
   const int unit0 = HALF ? 2 * ctile : ctile, units = min(U, (HALF ? 2 : 1) * (p.ntiles - ctile));
   const int group_unit = p.cls == 2 ? 2 * warp : 0;   // a merged group's unit, for both of the warp's tiles
-  const int drop = (blockIdx.x == 0 && blockIdx.y == 0) ? p.drop_tile : -1;
+  const int drop = (blockIdx.x == 0 && blockIdx.y == 0) ? min(p.drop_tile, ntile - 1) : -1;   // test hook (k_forward)
   auto issue = [&](int i, int stage) {
     if (i == drop) return;
     const int at = n0 + i * kAdjNodeTile, n = min(kAdjNodeTile, n1 - at), ne = (n + 1) & ~1;   // ld is even
