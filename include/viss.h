@@ -249,10 +249,12 @@ int viss_adjoint_formation(viss_plan *plan, const float *coef, float *image, flo
 /* Test hook for the failure path: the next viss_forward or viss_adjoint on
  * this plan has its first thread block skip the staging copy of its `tile`-th
  * tile (a pixel tile in the forward, a sample tile in the adjoint; its last
- * one if it has fewer), so that block's bounded waits give up (about 1 s each, no fault, no trap), the
- * kernel ends, and viss_plan_last_stats / viss_plan_last_counts then return
+ * one if it has fewer), so that block's bounded waits give up (about 1 s each,
+ * no fault, no trap), the kernel ends, and viss_plan_last_stats / viss_plan_last_counts then return
  * VISS_ERR_TIMEOUT; the plan and the context stay usable.  The results of
- * that one call are incomplete.  With plan == NULL the hook arms the next
+ * that one call are incomplete.  In a call through track blocks a `tile` of 2^30
+ * or more leaves the first tensor-core product of their interpolation without
+ * its signal instead.  With plan == NULL the hook arms the next
  * viss_forward_noalloc call instead (process-wide), which then returns
  * VISS_ERR_TIMEOUT itself.  No counterpart in the reference. */
 int viss_plan_debug_drop_copy(viss_plan *plan, int tile);

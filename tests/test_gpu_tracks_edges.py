@@ -113,12 +113,13 @@ def test_skies_through_the_blocks(cuda_device):
         close(out[c], want[c])
 
 
-@pytest.mark.parametrize("tile", [1, 10 ** 6])
+@pytest.mark.parametrize("tile", [1, 10 ** 6, 1 << 30])
 @pytest.mark.parametrize("call", ["forward", "adjoint"])
 @pytest.mark.parametrize("f_hz", [2e4, 2e6])      # groups of 1,024 pixels; of 64 among others
 def test_wait_that_gives_up(cuda_device, call, tile, f_hz):
     """A staging copy that never comes (a tile past the last one stands for the
-    last): the call ends, the next status read reports it, the plan goes on."""
+    last) or a product whose end is never signalled (2^30): the call ends, the
+    next status read reports it, the plan goes on."""
     obs = observation(57, 10, 6000, f_hz, False, False)
     plan = api.Plan(api.pix2lmn(57, "ring", device=cuda_device), torch.as_tensor(obs.uvw(f_hz), device=cuda_device))
     sky, coef = inputs(plan, cuda_device)

@@ -258,8 +258,16 @@ struct TrackInterpParams {
   long long vstride;
   const float2 *coef;          // adjoint: slots
   int *err;
+  bool drop;                   // test hook: block (0, 0) never signals its first product
 };
 
+// A wait that gave up ends an interpolation block at its next barrier (all threads
+// together, `broken`); before its tensor memory is freed, the products issued and
+// not waited for get another bounded wait.
+__device__ __forceinline__ bool broken(bool ok) { return __syncthreads_or(!ok) != 0; }
+__device__ __forceinline__ void drain_products(uint64_t *done, int issued) {
+  for (int i = max(issued - 2, 0); i < issued; ++i) mbar_wait_bounded(&done[i & 1], static_cast<uint32_t>(i >> 1) & 1u);
+}
 
 // A unit of one pass: its group's centre, its row of node sums, and which of
 // the block's samples see it (bit k mod 32 of word k / 32).
@@ -441,8 +449,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   umma_fence_after();
   const uint32_t tmem = s_tmem;
   if (passes > 0) fetch(0);
+  const bool drop = p.drop && blockIdx.x == 0 && blockIdx.y == 0;
   double vre = 0.0, vim = 0.0;
   bool ok = true;
+  int issued = passes;                             // products, when the loop ends
   for (int pass = -1; pass < passes; ++pass) {
     const int next = pass + 1;
     if (next < passes) {
@@ -475,7 +485,11 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
       fence_async_smem();
       umma_fence_before();
     }
-    __syncthreads();
+    if (broken(ok)) {
+      ok = false;
+      issued = next;
+      break;
+    }
     umma_fence_after();
     prepare(pass + 3);                             // over the units every thread is done with
     if (next < passes && tid == 0) {
@@ -486,7 +500,7 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
         for (int ks = 0; ks < kc; ks += 2, add = true)
           umma_tf32(d, umma_desc(a + ((q == 1 ? kc : 0) + ks) * kFwdLboA, kFwdLboA),
                     umma_desc(bn + ((q == 0 ? kc : 0) + ks) * kFwdLboB, kFwdLboB), idesc, add);
-      umma_commit(&s_done[next & 1]);
+      if (next > 0 || !drop) umma_commit(&s_done[next & 1]);
     }
     if (pass + 2 < passes) fetch(pass + 2);
     if (pass < 0) continue;
@@ -512,7 +526,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
     vim += static_cast<double>(sim);
     umma_fence_before();                           // the next product but one writes these columns
   }
-  if (!ok && lane == 0) atomicOr(p.err, kErrTimeout);
+  if (!ok) {
+    if (lane == 0) atomicOr(p.err, kErrTimeout);
+    drain_products(s_done, issued);
+  }
   // the two halves of the units meet
   if (half == 1) s_meet[row] = make_double2(vre, vim);
   umma_fence_before();
@@ -865,7 +882,8 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
   const long long slot0 = static_cast<long long>(b) * kTrackT + ks;
   double4 u = p.samp[slot0];
   float2 a = p.coef[slot0];
-  int step = 0;
+  const bool drop = p.drop && blockIdx.x == 0 && blockIdx.y == 0;
+  int step = 0;                                    // products issued
   bool ok = true;
   for (int base = 0, buf = 0; base < count; base += kAdjUnits, buf ^= 1) {
     const int nu = min(kAdjUnits, count - base);
@@ -898,7 +916,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
       if (s == 0) prepare(base + kAdjUnits, buf ^ 1);
       fence_async_smem();
       umma_fence_before();
-      __syncthreads();
+      if (broken(ok)) {
+        ok = false;
+        break;
+      }
       umma_fence_after();
       if (tid == 0) {
         const uint32_t ah = smem_addr(An), al = ah + (kAdjStep / 4) * kAdjLboA;
@@ -913,9 +934,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
           umma_tf32(dl, dal, dbh, idesc, true);
           umma_tf32(dh, dah, dbh, idesc, !first || q > 0);
         }
-        umma_commit(&s_done[step & 1]);
+        if (step > 0 || !drop) umma_commit(&s_done[step & 1]);
       }
     }
+    if (!ok) break;                                // at a barrier of the steps: the same for all
     // the pass's last two products (the commit of the last covers both buffers' reads)
     ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&s_done[step & 1], ((step >> 1) + 1) & 1));
     ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&s_done[(step + 1) & 1], (((step + 1) >> 1) + 1) & 1));
@@ -924,7 +946,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
     float *red = reinterpret_cast<float *>(A);       // [2 kAdjUnits][np + 1]
     const int row = (warp & 3) * 32 + lane;
     const uint32_t my = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    __syncthreads();
+    if (broken(ok)) {
+      ok = false;
+      break;
+    }
     for (int c = (warp >> 2) * 16; c < at.np; c += 32) {
       float sum[16], d[16];
       tmem_load16(my + c, sum);
@@ -955,7 +980,10 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
     }
     __syncthreads();
   }
-  if (!ok && lane == 0) atomicOr(p.err, kErrTimeout);
+  if (!ok) {
+    if (lane == 0) atomicOr(p.err, kErrTimeout);
+    drain_products(s_done, step);
+  }
   umma_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, at.cols);
@@ -1155,8 +1183,10 @@ TrackRestParams rest_params(const TrackState &S, const TrackInputs &in, bool mas
 }
 
 TrackInterpParams interp_params(const TrackState &S, const TrackInputs &in, const TrackSlab &sl, bool masked,
-                                bool use_off) {
+                                bool use_off, int &drop_tile) {
   TrackInterpParams ip{};
+  ip.drop = drop_tile >= kDropProduct;
+  if (ip.drop) drop_tile = -1;
   ip.samp = S.samp;
   ip.slot = S.slot;
   ip.refs = masked ? S.refs : nullptr;
@@ -1200,8 +1230,12 @@ TrackNodeParams node_params(const TrackState &S, const TrackInputs &in, const Tr
   np.Jpad = in.Jpad;
   np.counter = counter;
   np.err = err;
-  np.drop_tile = drop_tile;
-  drop_tile = -1;
+  if (drop_tile < kDropProduct) {
+    np.drop_tile = drop_tile;
+    drop_tile = -1;
+  } else {
+    np.drop_tile = -1;
+  }
   return np;
 }
 
@@ -1250,7 +1284,7 @@ int tracks_forward(void *state, const TrackInputs &in, const double4 *pixsky, fl
       if (sl.cls == kHalf) k_track_fwd_nodes<true><<<grid, kNodeNT, 0, st>>>(np);
       else k_track_fwd_nodes<false><<<grid, kNodeNT, 0, st>>>(np);
       TRACK_CUDA(cudaGetLastError(), "node sums");
-      TrackInterpParams ip = interp_params(S, in, sl, masked, use_off);
+      TrackInterpParams ip = interp_params(S, in, sl, masked, use_off, drop_tile);
       ip.per_chunk = interp_tiles(in, nblk);
       nv = static_cast<int>(blks(in.ntiles, ip.per_chunk));
       ip.vacc = vacc_d;
@@ -1325,7 +1359,7 @@ int tracks_adjoint(void *state, const TrackInputs &in, const float2 *coef, float
       const TrackSlab &sl = S.slabs[si];
       if (sl.cls == kClasses) continue;
       const int nblk = sl.b1 - sl.b0;
-      TrackInterpParams ip = interp_params(S, in, sl, masked, use_off);
+      TrackInterpParams ip = interp_params(S, in, sl, masked, use_off, drop_tile);
       ip.coef = coef_d;
       ip.per_chunk = interp_tiles(in, nblk);
       ip.err = err;

@@ -38,6 +38,9 @@ void tracks_free(void *state);
 // and not (9.6e-14 to 3.4e-13 s per term).
 double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint);
 
+// drop_tile from here on: the interpolation's first product instead of a tile's copy.
+constexpr int kDropProduct = 1 << 30;
+
 // V (channel-major, caller's order) and images of the built blocks.  pixsky:
 // the staged pixel + sky records of every channel; coef: the caller's
 // coefficients.  masked selects the occulted or the unmasked pair bits.
