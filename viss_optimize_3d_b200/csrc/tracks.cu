@@ -248,7 +248,7 @@ struct TrackInterpParams {
   TrackBits bits;
   const double4 *gcen[3];      // centres of the half tiles, the tiles, the class's groups
   int cls, ntiles;
-  int b0;                      // the slab's first block
+  int b0;                      // the slab's first block; every block of it has nodes
   int n0;                      // and node
   int per_chunk;               // tiles per blockIdx.y, a multiple of 32, at most kChunkTiles
   long long ld;
@@ -396,7 +396,6 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   __shared__ __align__(8) uint64_t s_done[2];
   __shared__ double2 s_meet[kTrackT];
   const int b = p.b0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = p.rank[b];
-  if (r == 0) return;                              // its sums in vacc stay zero
   const int kp = round_up(r, 8), kc = kp / 4, n0 = p.noff[b];
   const FwdInterpSmem at(r);
   unsigned char *A = smem + at.a, *B = smem + at.b;
@@ -844,7 +843,6 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
   __shared__ uint32_t s_tmem;
   __shared__ __align__(8) uint64_t s_done[2];
   const int b = p.b0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = p.rank[b];
-  if (r == 0) return;
   const int n0 = p.noff[b];
   const AdjInterpSmem at(r);
   unsigned char *A = smem + at.a, *B = smem + at.b;

@@ -196,10 +196,12 @@ __global__ void __launch_bounds__(kTrackT) k_track_ranks(TrackShape s, int nb, c
 }
 
 // Nodes and weights of every block: node n of block b is record noff[b] + n,
-// its weights for the block's 128 slots P[(noff[b] + n) * 128 + k].
+// its weights for the block's 128 slots P[(noff[b] + n) * 128 + k].  The factorisation
+// is k_track_ranks's; should it ever end at another rank, *differ says so and the
+// blocks are not used.
 __global__ void __launch_bounds__(kTrackT) k_track_weights(const int *slot, const double4 *samp_s, RadiusSet radii,
                                                            const int *cls, const int *rank, const int *noff, double4 *node,
-                                                           int *nodeblk, float *P) {
+                                                           int *nodeblk, float *P, unsigned long long *differ) {
   extern __shared__ __align__(128) unsigned char smem[];
   TrackFactor &f = *reinterpret_cast<TrackFactor *>(smem);
   const int b = blockIdx.x, k = threadIdx.x;
@@ -208,7 +210,10 @@ __global__ void __launch_bounds__(kTrackT) k_track_weights(const int *slot, cons
   const double4 u = samp_s[i];
   const bool valid = slot[i] >= 0;
   const int r = track_factor(f, valid, u, radii.rho[cls[b]], radii.most[cls[b]]);
-  if (r != rank[b]) return;                       // the same arithmetic: cannot happen
+  if (r != rank[b]) {
+    if (k == 0) atomicOr(differ, 1ull);
+    return;
+  }
   const long long n0 = noff[b];
   if (k < r) {
     const int p = f.piv[k];
@@ -444,13 +449,13 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   int *trial_rank_d;
   unsigned long long *counts_d;
   if (!S.trial.reset(TrackArena::bytes<double4>(total) + TrackArena::bytes<float>(total) + TrackArena::bytes<float>(lags) +
-                     TrackArena::bytes<int>(kRadii * kRankSamples) + TrackArena::bytes<unsigned long long>(4)))
+                     TrackArena::bytes<int>(kRadii * kRankSamples) + TrackArena::bytes<unsigned long long>(5)))
     return 0;
   S.trial.take(S.gcen, total);
   S.trial.take(radius_d, total);
   S.trial.take(score_d, lags);
   S.trial.take(trial_rank_d, kRadii * kRankSamples);
-  S.trial.take(counts_d, 4);
+  S.trial.take(counts_d, 5);
   for (int c = 0; c < kClasses; ++c) {
     k_track_groups<<<blks(ngs[c], 8), 256, 0, st>>>(ngs[c], group_pix(c), in.Jpad, in.pix, S.gcen + S.gat[c],
                                                     radius_d + S.gat[c]);
@@ -652,10 +657,10 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   TRACK_CUDA(cudaGetLastError(), "slots");
   TRACK_CUDA(cudaMemsetAsync(S.node, 0, sizeof(double4) * nodes, st), "nodes");
   TRACK_CUDA(cudaMemsetAsync(S.nodeblk, 0xff, sizeof(int) * nodes, st), "nodes");
+  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 5 * sizeof(unsigned long long), st), "counts");
   k_track_weights<<<nb, kTrackT, sizeof(TrackFactor), st>>>(S.slot, S.samp, radii, S.cls, S.rank, S.noff, S.node,
-                                                           S.nodeblk, S.P);
+                                                           S.nodeblk, S.P, counts_d + 3);
   TRACK_CUDA(cudaGetLastError(), "weights");
-  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 4 * sizeof(unsigned long long), st), "counts");
   k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, radius_d, cs, S.crow[0],
                                                                          S.crow[1], S.crow[2], counts_d + 2);
   TRACK_CUDA(cudaGetLastError(), "class rows");
@@ -665,14 +670,15 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
                                                S.brow[0], S.brow[1], S.brow[2], S.brow[3], counts_d);
     TRACK_CUDA(cudaGetLastError(), "pair bits");
   }
-  unsigned long long pairs_of[3] = {0, 0, 0};      // rest, part, classes that leave tiles
+  unsigned long long pairs_of[4] = {0, 0, 0, 0};   // rest, part, classes that leave tiles, ranks that differ
   TRACK_CUDA(cudaMemcpyAsync(pairs_of, counts_d, sizeof(pairs_of), cudaMemcpyDeviceToHost, st), "counts");
   TRACK_CUDA(cudaStreamSynchronize(st), "build");
+  if (pairs_of[3]) return 0;
   if (masked) {
     if (pairs_of[1] > INT_MAX || !S.masks.reset(TrackArena::bytes<uint4>(pairs_of[1]))) return 0;
     S.masks.take(S.mask, pairs_of[1]);
     k_track_masks<<<dim3(nb, by), 128, 0, st>>>(S.W, S.slot, S.refs, in.occ32, in.cones, S.brow[1], S.mask_at, S.mask,
-                                                counts_d + 3);
+                                                counts_d + 4);
     TRACK_CUDA(cudaGetLastError(), "sample masks");
     TRACK_CUDA(cudaStreamSynchronize(st), "build");  // later calls may come on other streams
   }
