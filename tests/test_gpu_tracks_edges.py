@@ -131,3 +131,24 @@ def test_wait_that_gives_up(cuda_device, call, tile, f_hz):
     with pytest.raises(_capi.VissError, match="gave up"):
         plan.last_stats()
     close(run(), run(fp64=True))
+
+
+@pytest.mark.parametrize("seed", [1, 5, 12])
+@pytest.mark.parametrize("f_hz,n_sat", [(1e6, 8), (3e6, 10)])
+def test_no_further_off_than_evaluated_terms(cuda_device, seed, f_hz, n_sat):
+    """A term that the direct kernels evaluate is off by up to 3.7e-7 (a phase of
+    23 bits); V, an image of random coefficients and one of V itself (whose terms
+    share their errors) stay below that through blocks."""
+    obs = observation(128, n_sat, 8640, f_hz, False, False)
+    plan = api.Plan(api.pix2lmn(128, "ring", device=cuda_device), torch.as_tensor(obs.uvw(f_hz), device=cuda_device))
+    g = torch.Generator(device=cuda_device).manual_seed(seed)
+    sky = torch.exp(torch.randn(plan.J, generator=g, device=cuda_device))
+    coef = torch.randn(plan.K, generator=g, device=cuda_device, dtype=torch.complex64)
+    rel = lambda a, b: float((a.to(torch.complex128) - b.to(torch.complex128)).norm() / b.to(torch.complex128).norm())
+    V = plan.forward(sky, fp64=True)
+    assert rel(plan.forward(sky), V) <= 3.7e-7
+    assert by_blocks(plan)
+    for c in (coef, V):
+        img = plan.adjoint(c)
+        assert by_blocks(plan)
+        assert rel(img, plan.adjoint(c, fp64=True)) <= 3.7e-7

@@ -26,9 +26,9 @@
 // block stops when its mean squared prediction error, node errors included, is
 // below 1.8 kNodeNoise^2 (no sample above 4.5): (2.7e-7)^2, where a term that
 // k_forward evaluates is off by 3.7e-7 (a phase of 23 bits).  Measured against
-// FP64 on 1 and 10 MHz Nside 256 observations: V 2.4e-7 - 3.5e-7, images of random
-// coefficients 4.2e-7 and of the observations 3.0e-7 - 4.5e-7; the direct kernels
-// 2.5e-7 - 4.6e-7, 5.0e-7 and 2.6e-7 - 5.4e-7.
+// FP64 on four inputs each of 1 to 10 MHz observations at Nside 128 and 256: V 2.0e-7 -
+// 3.0e-7, images of random coefficients 2.8e-7 - 3.0e-7 and of the observations 2.2e-7
+// - 3.1e-7; the direct kernels 2.5e-7 - 4.6e-7, 5.0e-7 and 2.6e-7 - 5.4e-7.
 // Stopping at 0.85 (3e-7)^2 with the same node error costs 25 % more nodes
 // for 8 % less error, stopping at 2.5 saves 1 %.  Blocks that need more than
 // kTrackRankMax nodes, or three quarters of their samples, are left to the
@@ -97,6 +97,11 @@ __device__ __forceinline__ float turn_angle32(double t) {
 
 constexpr int kNodeNT = 256;
 constexpr int kNodeR = 4;
+// Terms added in plain FP32 before a run's sum joins the others, in both directions.
+// A run of 128 (256 additions in the adjoint) left 1.9e-7 (2.7e-7) of the sum's own
+// size; with 32, images of random coefficients went from 3.75e-7 to 2.85e-7 of error
+// at 1 MHz, V from 3.0e-7 to 2.75e-7 at 10 MHz, in the same time.
+constexpr int kNodeRun = 32;
 
 // G of the slab's nodes (R per thread) over a chunk of tiles: the inner loop
 // and the stage ring of k_forward, a value written per (unit, node) instead of
@@ -183,31 +188,42 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
         float t_re[R], t_im[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) t_re[r] = t_im[r] = 0.f;
-        auto term = [&](int r, const double4 &q, float I, double magic) {
+        auto term = [&](int r, const double4 &q, float I, double magic, float &re, float &im) {
           float sn, cs;
           sfu_sincos(turn_angle32(fma(uz[r], q.z, fma(uy[r], q.y, fma(ux[r], q.x, magic)))), sn, cs);
-          t_re[r] = fmaf(I, cs, t_re[r]);
-          t_im[r] = fmaf(-I, sn, t_im[r]);
+          re = fmaf(I, cs, re);
+          im = fmaf(-I, sn, im);
         };
-        if (rows == (1u << R) - 1) {
-          for (int j = 0; j < kSpan; j += 2) {
-            const double4 q0 = tp[j], q1 = tp[j + 1];
-            const float I0 = sky_of(q0), I1 = -sky_of(q1);
+#pragma unroll 1
+        for (int j0 = 0; j0 < kSpan; j0 += kNodeRun) {
+          if (rows == (1u << R) - 1) {
+            float re[R], im[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) re[r] = im[r] = 0.f;
+            for (int j = j0; j < j0 + kNodeRun; j += 2) {
+              const double4 q0 = tp[j], q1 = tp[j + 1];
+              const float I0 = sky_of(q0), I1 = -sky_of(q1);
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                term(r, q0, I0, kTurn32, re[r], im[r]);
+                term(r, q1, I1, kTurn32 + 0.5, re[r], im[r]);   // odd records half a turn on (k_forward)
+              }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) t_re[r] += re[r], t_im[r] += im[r];
+          } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              term(r, q0, I0, kTurn32);
-              term(r, q1, I1, kTurn32 + 0.5);         // odd records half a turn on (k_forward)
-            }
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if (!((rows >> r) & 1u)) continue;
+              if (!((rows >> r) & 1u)) continue;
+              float re = 0.f, im = 0.f;
 #pragma unroll 4
-            for (int j = 0; j < kSpan; j += 2) {
-              const double4 q0 = tp[j], q1 = tp[j + 1];
-              term(r, q0, sky_of(q0), kTurn32);
-              term(r, q1, -sky_of(q1), kTurn32 + 0.5);
+              for (int j = j0; j < j0 + kNodeRun; j += 2) {
+                const double4 q0 = tp[j], q1 = tp[j + 1];
+                term(r, q0, sky_of(q0), kTurn32, re, im);
+                term(r, q1, -sky_of(q1), kTurn32 + 0.5, re, im);
+              }
+              t_re[r] += re;
+              t_im[r] += im;
             }
           }
         }
@@ -451,8 +467,8 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   const bool drop = p.drop && blockIdx.x == 0 && blockIdx.y == 0;
   double vre = 0.0, vim = 0.0;
   bool ok = true;
-  int issued = passes;                             // products, when the loop ends
-  for (int pass = -1; pass < passes; ++pass) {
+  int pass = -1;
+  for (; pass < passes; ++pass) {
     const int next = pass + 1;
     if (next < passes) {
       // the next pass's operand; its buffer was read by the product before the last one
@@ -486,7 +502,6 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
     }
     if (broken(ok)) {
       ok = false;
-      issued = next;
       break;
     }
     umma_fence_after();
@@ -527,7 +542,7 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   }
   if (!ok) {
     if (lane == 0) atomicOr(p.err, kErrTimeout);
-    drain_products(s_done, issued);
+    drain_products(s_done, min(pass + 1, passes));
   }
   // the two halves of the units meet
   if (half == 1) s_meet[row] = make_double2(vre, vim);
@@ -973,7 +988,9 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
       for (int n = tid & 3; n < r; n += 4) {
         const double4 w = un[n];
         const float2 c = fine_cis(fma(w.z, gz, fma(w.y, gy, fma(w.x, gx, kFine))));
-        out[n] = make_float2(sre[n] * c.x + sim[n] * c.y, sim[n] * c.x - sre[n] * c.y);
+        const float re = sre[n] * c.x + sim[n] * c.y, im = sim[n] * c.x - sre[n] * c.y;
+        const float sign = ((n0 - p.n0 + n) & 32) ? -1.f : 1.f;   // half a turn on (k_track_adj_nodes)
+        out[n] = make_float2(sign * re, sign * im);
       }
     }
     __syncthreads();
@@ -1044,6 +1061,7 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
   __syncthreads();
   const bool odd_lane = (lane & 1) != 0;             // half a turn on, negated at the end (k_adjoint)
   const double magic = odd_lane ? kTurn32 + 0.5 : kTurn32;
+  static_assert(kNodeRun == 32, "a run is a group of nodes below");
   unsigned long long evaluated = 0;
   int next = 0;
   for (int it = 0; it < ntile; ++it) {
@@ -1073,12 +1091,13 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
       break;
     }
     const AdjNodeStage<HALF> &st = stages[buf];
-    float acc[P];
+    float acc[P], sum[P];
 #pragma unroll
-    for (int q = 0; q < P; ++q) acc[q] = 0.f;
+    for (int q = 0; q < P; ++q) sum[q] = 0.f;
+    double from = magic;
     auto term = [&](int q, const double4 &u, const float2 &c) {
       float sn, cs;
-      sfu_sincos(turn_angle32(fma(u.z, sz[q], fma(u.y, sy[q], fma(u.x, sx[q], magic)))), sn, cs);
+      sfu_sincos(turn_angle32(fma(u.z, sz[q], fma(u.y, sy[q], fma(u.x, sx[q], from)))), sn, cs);
       acc[q] = fmaf(-c.y, sn, fmaf(c.x, cs, acc[q]));
     };
 #pragma unroll 1
@@ -1088,6 +1107,13 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
       for (int q = 1; q < kAdjNodeTile / 32; ++q) b3 = g == q ? three[q] : b3;
       const unsigned m0 = __ballot_sync(0xffffffffu, b3 & 1u), m1 = __ballot_sync(0xffffffffu, b3 & 2u);
       const unsigned mg = HALF ? 0u : __ballot_sync(0xffffffffu, b3 & 4u);
+      // every other 32 nodes half a turn on, their coefficients negated: an SFU error that
+      // the terms of a coherent sum share cancels (as k_forward's over pixels; odd lanes alone
+      // do not do it for one pixel's sum).  Images of 1 MHz observations: 3.7-4.2e-7 of error
+      // -> 2.2-2.5e-7, for 1.3 % of the 10 MHz adjoint's time.
+      from = (g & 1) ? magic + 0.5 : magic;
+#pragma unroll
+      for (int q = 0; q < P; ++q) acc[q] = 0.f;
       evaluated += static_cast<unsigned>(__popc(m0) + __popc(m1)) * static_cast<unsigned>(kTilePix);
       for (unsigned m = m0 & m1; m; m &= m - 1) {
         const int j = __ffs(m) - 1, i = 32 * g + j;
@@ -1120,11 +1146,13 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
 #pragma unroll
         for (int q = 4; q < 8; ++q) term(q, u, q < 6 ? c0 : c1);
       }
+#pragma unroll
+      for (int q = 0; q < P; ++q) sum[q] += acc[q];
     }
 #pragma unroll
     for (int q = 0; q < P; ++q) {
       float s = s_kahan[0][q][tid], c = s_kahan[1][q][tid];
-      kahan_add(s, c, acc[q]);
+      kahan_add(s, c, sum[q]);
       s_kahan[0][q][tid] = s;
       s_kahan[1][q][tid] = c;
     }
