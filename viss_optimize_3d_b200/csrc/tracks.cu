@@ -377,6 +377,21 @@ __device__ __forceinline__ double fine_phase(double ux, double uy, double uz, co
 // (the accumulator truncates, so it should be small while they are added).
 // Measured against FP64 on random 128 x K by K x 64 products: 1.1e-7 at K = 32,
 // 1.8e-7 at K = 64, where FP32 multiply-adds give 1.0e-7 and 1.5e-7.
+//
+// What that leaves out in scale, on average, is put back (interp_scale; not for one
+// node: identical samples, whose sums stay exact).  The SFU's sine and cosine are
+// 7.6e-8 short over a turn.  Every product added into an accumulator truncates it:
+// with the kernels' own order of products and the weights of 1 and 10 MHz
+// observations, sums of n = ceil(r / 8) steps (forward) came out 3.8, 5.7, 7.4,
+// 10.1, 12.9, 14.3e-8 short for n = 1 to 6, those of the adjoint's runs of 6 steps
+// 1.04e-7 to 1.16e-7 at ranks of 10 to 37.  One factor of 1.5e-7 for all of them left
+// V up to 5.8e-8 too large and images 3.0e-8 to 4.2e-8 too small; now 1.4e-8 of
+// incoherent sums at most either way.
+__device__ __forceinline__ float interp_scale(int r, bool adjoint) {
+  if (r == 1) return 0.f;
+  return 7.6e-8f + (adjoint ? 1.1e-7f : 1.7e-8f + 2.1e-8f * static_cast<float>((r + 7) / 8));
+}
+
 constexpr int kInterpNT = 256;
 constexpr int kFwdUnits = 32;          // units per pass, forward: 64 columns of the product
 constexpr int kFwdLboA = 2048, kFwdLboB = 2 * kFwdUnits * 16 + 16;
@@ -551,8 +566,9 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   if (warp == 0) tmem_free(tmem, 128);
   if (half == 0) {
     const double2 o = s_meet[row];
+    const double scale = 1.0 + static_cast<double>(interp_scale(r, false));
     p.vacc[blockIdx.y * p.vstride + static_cast<long long>(blockIdx.x) * kTrackT + row] =
-        make_double2(vre + o.x, vim + o.y);
+        make_double2(scale * (vre + o.x), scale * (vim + o.y));
   }
 }
 
@@ -985,12 +1001,13 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_adj_interp(const TrackIn
       const double gx = g.x, gy = g.y, gz = g.z;
       float2 *out = p.sums + g.row * p.ld + (n0 - p.n0);
       const float *sre = red + q * (at.np + 1), *sim = red + (kAdjUnits + q) * (at.np + 1);
+      const float scale = interp_scale(r, true);
       for (int n = tid & 3; n < r; n += 4) {
         const double4 w = un[n];
         const float2 c = fine_cis(fma(w.z, gz, fma(w.y, gy, fma(w.x, gx, kFine))));
         const float re = sre[n] * c.x + sim[n] * c.y, im = sim[n] * c.x - sre[n] * c.y;
         const float sign = ((n0 - p.n0 + n) & 32) ? -1.f : 1.f;   // half a turn on (k_track_adj_nodes)
-        out[n] = make_float2(sign * re, sign * im);
+        out[n] = make_float2(sign * fmaf(scale, re, re), sign * fmaf(scale, im, im));
       }
     }
     __syncthreads();

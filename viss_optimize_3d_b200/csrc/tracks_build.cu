@@ -14,11 +14,6 @@ namespace viss {
 namespace {
 
 constexpr double kNodeNoise2 = 4e-14;            // kNodeNoise^2
-// What the sums lack in scale: the tensor cores' accumulators truncate and the SFU's
-// sine and cosine are 7.7e-8 short.  Without it V came out 0.8e-7 to 1.5e-7 and
-// images 1.85e-7 too small (Nside 256, 1 and 10 MHz, 90,000 and 388,800 samples),
-// a coherent part of errors of 2.5e-7 to 4.8e-7.
-constexpr double kTrackScale = 1.5e-7;
 constexpr int kLagMax = 1024;                    // tracks interleaved in the caller's order, at most
 constexpr int kLagSamples = 128;
 constexpr int kRankSamples = 48;                 // blocks that decide whether nodes pay at all
@@ -229,8 +224,7 @@ __global__ void __launch_bounds__(kTrackT) k_track_weights(const int *slot, cons
     for (int q = j + 1; q < r; ++q) v = fma(-x[q], f.L[j * kTrackT + f.piv[q]], v);
     x[j] = v / f.ld[j];
   }
-  const double scale = r > 1 ? 1.0 + kTrackScale : 1.0;     // one node: identical samples, sums of them stay exact
-  for (int j = 0; j < r; ++j) P[(n0 + j) * kTrackT + k] = valid ? static_cast<float>(x[j] * scale) : 0.f;
+  for (int j = 0; j < r; ++j) P[(n0 + j) * kTrackT + k] = valid ? static_cast<float>(x[j]) : 0.f;
 }
 
 // A tile is merged with the others of its group of class c (2 or 3) when all
