@@ -46,6 +46,7 @@ extern "C" {
 #define VISS_NO_MASK 0x2     /* ignore occultation references */
 #define VISS_NO_OFFSET 0x4   /* ignore the per-sample phase offset */
 #define VISS_ACCUMULATE 0x8  /* add into the output instead of overwriting */
+#define VISS_ALL_TERMS 0x10  /* evaluate every term, as captured calls do: no track blocks */
 
 /* HEALPix schemes */
 #define VISS_RING 0
@@ -135,9 +136,11 @@ int viss_plan_set_samples(viss_plan *plan, int64_t K, const double *uvw, const d
  * staged builds them (a few waits for the device, 1-3 ms) and every call then
  * uses device buffers of the plan, about 1 GiB and 1 KiB per sample; without
  * that memory, under stream capture, and for other samples every term is
- * evaluated.  Asynchronous: VISS_OK means the work was launched.  A bounded
- * device-side wait that gave up inside the kernel (V then incomplete) is
- * reported only by the next viss_plan_last_stats / viss_plan_last_counts on this plan, which return
+ * evaluated.  The two ways agree to their accuracy, not bit by bit:
+ * VISS_ALL_TERMS asks for the second, with the same bits as a captured call.
+ * Asynchronous: VISS_OK means the work was launched.  A bounded device-side wait
+ * that gave up inside the kernel (V then incomplete) is reported only by the
+ * next viss_plan_last_stats / viss_plan_last_counts on this plan, which return
  * VISS_ERR_TIMEOUT; callers that need the guarantee check it after the call. */
 int viss_forward(viss_plan *plan, const float *sky, float *V, int flags, void *stream);
 
@@ -151,8 +154,8 @@ int viss_forward_skies(viss_plan *plan, int n, const float *sky, float *V, int f
 /* Imaging adjoint, replaces computeC (vissgen3d_blockage.cu:167-192):
  *   image_j = scale * sum_k Re(coef_k exp(+2 pi i (u_k . s_j + off_k))) vis_kj
  * coef: K complex64 (the weighted visibilities w_k V_k); image: J FP32.  Track
- * blocks as in viss_forward.  Asynchronous; a timed-out wait is reported as for viss_forward, only
- * through viss_plan_last_stats / viss_plan_last_counts. */
+ * blocks as in viss_forward.  Asynchronous; a timed-out wait is reported as for
+ * viss_forward, only through viss_plan_last_stats / viss_plan_last_counts. */
 int viss_adjoint(viss_plan *plan, const float *coef, float *image, float scale, int flags,
                  void *stream);
 
@@ -160,7 +163,9 @@ int viss_adjoint(viss_plan *plan, const float *coef, float *image, float scale, 
  * this plan's problem (CUDA events on `stream`, one warm-up and one timed
  * launch each) and keeps the fastest for later calls.  sky (channels x J
  * FP32) and coef (K complex64) are representative inputs; V_scratch (K
- * complex64) and img_scratch (channels x J FP32) receive throw-away outputs.  Synchronous.  The chosen
+ * complex64) and img_scratch (channels x J FP32) receive throw-away outputs.
+ * Every term is evaluated: the shapes serve the calls that do so (captured ones,
+ * VISS_ALL_TERMS, all that do not go through track blocks).  Synchronous.  The chosen
  * shape indices are returned through fwd_shape / adj_shape (may be NULL).
  * No counterpart in the reference (it launches one fixed shape from
  * cudaOccupancyMaxPotentialBlockSize, vissgen3d_blockage.cu:412-413). */
@@ -264,7 +269,8 @@ int viss_plan_debug_drop_copy(viss_plan *plan, int tile);
 int viss_plan_set_shapes(viss_plan *plan, int fwd_shape, int adj_shape);
 
 /* Terms evaluated by the last viss_forward / viss_adjoint on this plan
- * (visible-or-mixed pairs actually exponentiated) and the total K*J, read
+ * (visible-or-mixed pairs actually exponentiated; through track blocks the
+ * exponentials of the nodes and of the remainder) and the total K*J, read
  * back from the device (synchronises the plan's last stream). */
 int viss_plan_last_counts(viss_plan *plan, int64_t *evaluated, int64_t *total);
 /* The same plus the terms evaluated in "mixed" tiles (per-term occultation

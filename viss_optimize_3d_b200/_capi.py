@@ -38,6 +38,7 @@ VISS_FP64 = 0x1
 VISS_NO_MASK = 0x2
 VISS_NO_OFFSET = 0x4
 VISS_ACCUMULATE = 0x8
+VISS_ALL_TERMS = 0x10
 VISS_RING = 0
 VISS_NESTED = 1
 

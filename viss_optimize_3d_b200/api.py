@@ -179,7 +179,7 @@ class Plan:
         self.channels = int(channels)
 
     @staticmethod
-    def _flags(fp64, mask, use_offset, accumulate=False):
+    def _flags(fp64, mask, use_offset, accumulate=False, all_terms=False):
         f = 0
         if fp64:
             f |= capi.VISS_FP64
@@ -189,14 +189,17 @@ class Plan:
             f |= capi.VISS_NO_OFFSET
         if accumulate:
             f |= capi.VISS_ACCUMULATE
+        if all_terms:
+            f |= capi.VISS_ALL_TERMS
         return f
 
     def forward(self, sky, fp64: bool = False, mask: bool = True, use_offset: bool = True,
-                out: torch.Tensor | None = None) -> torch.Tensor:
+                out: torch.Tensor | None = None, all_terms: bool = False) -> torch.Tensor:
         """healpix_moonback_viss (vissgen3d_blockage.cu:76-102):
         V_k = sum_j sky_j vis_kj exp(-2 pi i (u_k.s_j + off_k)), complex64.
         Asynchronous; a bounded device-side wait that gave up inside the
-        kernel is raised by the next last_stats() / last_counts()."""
+        kernel is raised by the next last_stats() / last_counts().  all_terms
+        evaluates every term (no track blocks), as a captured call does."""
         sky = _cuda(sky, torch.float32, self.device)
         if sky.numel() != self.channels * self.J:
             raise ValueError(f"sky must hold {self.channels} x {self.J} values")
@@ -205,24 +208,27 @@ class Plan:
         elif (out.dtype != torch.complex64 or not out.is_contiguous() or out.numel() != self.K
               or out.device != self.device):
             raise ValueError(f"out must be a contiguous complex64 tensor of {self.K} values on {self.device}")
-        check(lib.viss_forward(self._h, _p(sky), _p(out), self._flags(fp64, mask, use_offset),
+        check(lib.viss_forward(self._h, _p(sky), _p(out), self._flags(fp64, mask, use_offset, all_terms=all_terms),
                                _stream(sky)), "viss_forward")
         return out
 
-    def _forward_skies(self, sky, fp64: bool = False) -> torch.Tensor:
+    def _forward_skies(self, sky, fp64: bool = False, all_terms: bool = False) -> torch.Tensor:
         """V (n x K complex64) of n skies (n x J) over the plan's samples; an
         even K, one channel."""
         sky = _cuda(sky, torch.float32, self.device)
         out = torch.empty((sky.shape[0], self.K), dtype=torch.complex64, device=self.device)
-        check(lib.viss_forward_skies(self._h, sky.shape[0], _p(sky), _p(out), self._flags(fp64, True, True),
-                                     _stream(sky)), "viss_forward_skies")
+        check(lib.viss_forward_skies(self._h, sky.shape[0], _p(sky), _p(out),
+                                     self._flags(fp64, True, True, all_terms=all_terms), _stream(sky)),
+              "viss_forward_skies")
         return out
 
     def adjoint(self, coef, scale: float = 1.0, fp64: bool = False, mask: bool = True,
-                use_offset: bool = True, out: torch.Tensor | None = None) -> torch.Tensor:
+                use_offset: bool = True, out: torch.Tensor | None = None,
+                all_terms: bool = False) -> torch.Tensor:
         """computeC (vissgen3d_blockage.cu:167-192):
         img_j = scale * sum_k Re(coef_k exp(+2 pi i (u_k.s_j + off_k))) vis_kj.
-        Asynchronous, like forward (a timed-out wait surfaces in last_stats())."""
+        Asynchronous, like forward (a timed-out wait surfaces in last_stats());
+        all_terms as there."""
         coef = _cuda(coef, torch.complex64, self.device)
         if coef.shape != (self.K,):
             raise ValueError(f"coef must have shape ({self.K},)")
@@ -234,7 +240,8 @@ class Plan:
             raise ValueError(f"out must be a contiguous float32 tensor of {self.channels} x {self.J} "
                              f"values on {self.device}")
         check(lib.viss_adjoint(self._h, _p(coef), _p(out), float(scale),
-                               self._flags(fp64, mask, use_offset), _stream(coef)), "viss_adjoint")
+                               self._flags(fp64, mask, use_offset, all_terms=all_terms), _stream(coef)),
+              "viss_adjoint")
         return out
 
     def adjoint_gridded(self, coef, scale: float = 1.0, mask: bool = True, use_offset: bool = True,
@@ -314,7 +321,7 @@ class Plan:
             check(lib.viss_plan_set_formation_channels(self._h, C), "viss_plan_set_formation_channels")
 
     def forward_formation(self, sky, mask: bool = True, use_offset: bool = True,
-                          out: torch.Tensor | None = None, accumulate: bool = False):
+                          out: torch.Tensor | None = None, accumulate: bool = False, all_terms: bool = False):
         """V (T * B complex64) of the formation's samples (channel-major with
         channels: sky then holds C x J values)."""
         sky = _cuda(sky, torch.float32, self.device)
@@ -326,12 +333,13 @@ class Plan:
         elif (out.dtype != torch.complex64 or not out.is_contiguous() or out.numel() != n
               or out.device != self.device):
             raise ValueError(f"out must be a contiguous complex64 tensor of {n} values on {self.device}")
-        check(lib.viss_forward_formation(self._h, _p(sky), _p(out), self._flags(False, mask, use_offset, accumulate),
-                                         _stream(sky)), "viss_forward_formation")
+        check(lib.viss_forward_formation(self._h, _p(sky), _p(out),
+                                         self._flags(False, mask, use_offset, accumulate, all_terms), _stream(sky)),
+              "viss_forward_formation")
         return out
 
     def adjoint_formation(self, coef, scale: float = 1.0, mask: bool = True, use_offset: bool = True,
-                          out: torch.Tensor | None = None, accumulate: bool = False):
+                          out: torch.Tensor | None = None, accumulate: bool = False, all_terms: bool = False):
         """img (J FP32, or C x J with channels) = scale * the adjoint of the
         formation's samples."""
         n = self.form_T * self.form_B
@@ -346,7 +354,7 @@ class Plan:
               or out.device != self.device):
             raise ValueError(f"out must be a contiguous float32 tensor of {nimg} values on {self.device}")
         check(lib.viss_adjoint_formation(self._h, _p(coef), _p(out), float(scale),
-                                         self._flags(False, mask, use_offset, accumulate), _stream(coef)),
+                                         self._flags(False, mask, use_offset, accumulate, all_terms), _stream(coef)),
               "viss_adjoint_formation")
         return out
 

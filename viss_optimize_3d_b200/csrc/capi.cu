@@ -561,9 +561,9 @@ static bool tracks_allowed(double terms, cudaStream_t st) {
   return cap == cudaStreamCaptureStatusNone;
 }
 
-static int tracks_ready(viss_plan *p, cudaStream_t st, bool *use) {
+static int tracks_ready(viss_plan *p, int flags, cudaStream_t st, bool *use) {
   *use = false;
-  if (!tracks_allowed(static_cast<double>(p->K) * p->J, st)) return VISS_OK;
+  if ((flags & VISS_ALL_TERMS) || !tracks_allowed(static_cast<double>(p->K) * p->J, st)) return VISS_OK;
   if (p->tracks_version != p->geom_version) {
     bool ok = false;
     if (int s = viss::tracks_build(&p->tracks, track_inputs(p), st, &ok)) return s;
@@ -593,7 +593,7 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
             "viss_forward: sky");
   bool use = false;
   if (tracks && !fp64)
-    if (int s = tracks_ready(p, st, &use)) return s;
+    if (int s = tracks_ready(p, flags, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_forward(p->tracks, track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V), masked,
                                        !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
@@ -683,7 +683,7 @@ int viss_forward_skies(viss_plan *p, int n, const float *sky, float *V, int flag
     if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * n * p->K)) return s;
     if (int s = ensure(p->skies, p->skies_cap, sizeof(float4) * p->Jpad, "sky records")) return s;
     bool use = false;
-    if (int s = tracks_ready(p, st, &use)) return s;
+    if (int s = tracks_ready(p, flags, st, &use)) return s;
     three = !use || n * viss::tracks_seconds(p->tracks, track_inputs(p), masked, false) >
                         0.95 * kSkiesSeconds[masked] * static_cast<double>(p->K) * static_cast<double>(p->J);
   }
@@ -739,7 +739,7 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
             "viss_adjoint: coef");
   bool use = false;
   if (tracks && !fp64 && !fcones)
-    if (int s = tracks_ready(p, st, &use)) return s;
+    if (int s = tracks_ready(p, flags, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_adjoint(p->tracks, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
                                        !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
@@ -969,8 +969,9 @@ static viss::TrackInputs form_track_inputs(const viss_plan *p) {
 // 256 x 388,800 samples, Moon + Earth; measured 94.1 against 55 ms and 74.5
 // against 63 ms at 10 MHz).  Per pair S exponentials serve S - 1 / 2: with fewer
 // satellites a pair costs the formation kernels more, which only favours the blocks.
-static int form_tracks_ready(viss_plan *p, bool masked, bool adjoint, cudaStream_t st, bool *use) {
+static int form_tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint, cudaStream_t st, bool *use) {
   *use = false;
+  if (flags & VISS_ALL_TERMS) return VISS_OK;
   const double per_term = adjoint ? 2.43e-13 : 3.07e-13;
   const long long K = p->form_T * viss::form_pairs(p->form_S);
   if (!tracks_allowed(static_cast<double>(K) * p->J, st) || !(3.0 * p->form_turns < 262144.0)) return VISS_OK;
@@ -1016,7 +1017,7 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
             "viss_forward_formation: sky");
   bool use = false;
   const bool masked = (fp.sat_rows || fp.snap_rows);
-  if (int s = form_tracks_ready(p, masked, false, st, &use)) return s;
+  if (int s = form_tracks_ready(p, flags, masked, false, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_forward(p->form_tracks, form_track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V),
                                        masked, !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
@@ -1069,7 +1070,7 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
   viss::FormParams fp = form_params(p, flags);
   bool use = false;
   const bool masked = (fp.sat_rows || fp.snap_rows);
-  if (int s = form_tracks_ready(p, masked, true, st, &use)) return s;
+  if (int s = form_tracks_ready(p, flags, masked, true, st, &use)) return s;
   if (use) {
     const int s = viss::tracks_adjoint(p->form_tracks, form_track_inputs(p), reinterpret_cast<const float2 *>(coef),
                                        image, scale, masked, !(flags & VISS_NO_OFFSET),
@@ -1127,7 +1128,7 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   double other = 0;
   bool by_tracks = false;
   if (facet_pixels == 0) {
-    if (int s = tracks_ready(p, st, &by_tracks)) return s;
+    if (int s = tracks_ready(p, flags, st, &by_tracks)) return s;
     if (by_tracks) other = viss::tracks_seconds(p->tracks, track_inputs(p), masked, true);
     if (p->max_turns < viss::kMaxTurns) {
       const double direct = kDirectSeconds[masked] * static_cast<double>(p->K) * static_cast<double>(p->J);
