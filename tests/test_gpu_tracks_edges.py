@@ -166,3 +166,22 @@ def test_scale_of_the_image(cuda_device, f_hz, n_sat):
     assert by_blocks(plan)
     want = plan.adjoint(coef, fp64=True).double()
     assert abs(float(((got - want) * want).sum() / want.square().sum())) <= 2e-8
+
+
+@pytest.mark.parametrize("nside,n_sat,n_snap,f_hz,blocks", [
+    (256, 10, 600, 3e6, False),      # few snapshots: a limb crosses many tiles within a block
+    (256, 10, 600, 1e6, False),
+    (128, 10, 4600, 3e6, True),
+])
+def test_occulted_calls_take_the_faster_way(cuda_device, nside, n_sat, n_snap, f_hz, blocks):
+    """Sparse snapshots make the remainder of the blocks dear (measured: the first
+    two forwards 16.5 and 10.6 ms through blocks, 10.1 term by term; the third 9.9
+    against 19.5)."""
+    obs = observation(nside, n_sat, n_snap, f_hz, True, True)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(api.pix2lmn(nside, "ring", device=cuda_device), torch.as_tensor(obs.uvw(f_hz), device=cuda_device),
+                    None, refs, occ)
+    sky, _ = inputs(plan, cuda_device)
+    got = plan.forward(sky)
+    assert by_blocks(plan) == blocks
+    close(got, plan.forward(sky, fp64=True))

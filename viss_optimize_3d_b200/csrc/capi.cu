@@ -188,14 +188,14 @@ struct viss_plan {
   long long gridded_facet = 0;
   long long gridded_hbm_blocks = 0;
   long long geom_version = 0;   // bumped by every call that restages pixels or samples
-  // track blocks of the staged samples (tracks.cu), for geometry tracks_version
-  void *tracks = nullptr;
-  long long tracks_version = -1;
-  bool tracks_usable = false;
-  // the same for the formation's pairs, as samples u = U_a - U_b
-  void *form_tracks = nullptr;
-  long long form_version = 0, form_tracks_version = -1;
-  bool form_tracks_usable = false;
+  // track blocks (tracks.cu) of the staged samples, and of the formation's pairs as
+  // samples u = U_a - U_b; form_version as geom_version
+  struct Blocks {
+    void *state = nullptr;
+    long long version = -1;       // of the geometry that was looked at
+    bool promising = false, built = false, usable = false;
+  } tracks, form_tracks;
+  long long form_version = 0;
   double form_turns = 0;        // bound on |U.s| and |off|
   float4 *skies = nullptr;      size_t skies_cap = 0;   // viss_forward_skies
   double4 *form_samp = nullptr; size_t form_samp_cap = 0;
@@ -435,8 +435,8 @@ int viss_plan_destroy(viss_plan *p) {
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->gridded) viss::gridded_free(p->gridded);
-  if (p->tracks) viss::tracks_free(p->tracks);
-  if (p->form_tracks) viss::tracks_free(p->form_tracks);
+  if (p->tracks.state) viss::tracks_free(p->tracks.state);
+  if (p->form_tracks.state) viss::tracks_free(p->form_tracks.state);
   delete p;
   return VISS_OK;
 }
@@ -545,14 +545,42 @@ static viss::TrackInputs track_inputs(const viss_plan *p) {
   return in;
 }
 
-// Whether a split-precision call goes through the track blocks, built here for
-// newly staged samples.  From kTrackMinTerms terms on: the build takes 1-2 ms
-// (a few waits for the device among it), so a single call has to be longer.
+// Shares of the (sample, tile) pairs that a call sees, and sees in part: counted on
+// some blocks where those were looked at, else those of the Moon and the Earth seen
+// from a 300 km orbit (.048, .097 and .20 in part at Nside 256, 128 and 64).
+static void visible_shares(const viss_plan::Blocks &b, long long version, long long J, bool masked, double *seen,
+                           double *mixed) {
+  *seen = 1.0;
+  *mixed = 0.0;
+  if (!masked) return;
+  if (b.promising && b.version == version) return viss::tracks_shares(b.state, seen, mixed);
+  *seen = 0.8;
+  *mixed = std::min(0.8, 42.0 / std::sqrt(static_cast<double>(J)));
+}
+
+// The direct kernels, seconds per call: 5.35e-13 (forward) and 5.41e-13 s per visible
+// (sample, pixel) at every size measured, and what the exact tests add per pair of a
+// tile seen in part; within 4 % of 47 occulted observations of 1e10 to 8e10 terms.
+static double direct_seconds(const viss_plan *p, bool masked, bool adjoint) {
+  double seen, mixed;
+  visible_shares(p->tracks, p->geom_version, p->J, masked, &seen, &mixed);
+  const double per = adjoint ? 5.41e-13 * seen + 15.2e-13 * mixed : 5.35e-13 * seen + 4.5e-13 * mixed;
+  return per * static_cast<double>(p->K) * static_cast<double>(p->J);
+}
+
+// Blocks are taken where they are modelled below this share of what else would do the
+// call.  Of 1,172 calls measured (1e10 to 3e11 terms, plain and formation, occulted and
+// not) 879 took them, none of which is slower than term by term.
+constexpr double kTrackMargin = 0.95;
+// Fewer terms are not looked at: that takes 0.2 to 0.5 ms of a call's first pass on
+// newly staged samples, and the build 1 to 4.5 ms, more with a plan's first allocations.
+constexpr double kTrackMinTerms = 1e10;
+constexpr double kTrackMinSeconds = 3e-3;          // likewise, of the formation kernels (1e10 terms: 2.7 to 4.6 ms)
+
 // Not under stream capture: a captured call is replayed after the samples were
 // staged again, and the blocks' launch sizes depend on the samples.
-constexpr double kTrackMinTerms = 1e10;
-static bool tracks_allowed(double terms, cudaStream_t st) {
-  if (terms < kTrackMinTerms) return false;
+static bool tracks_allowed(int flags, cudaStream_t st) {
+  if (flags & (VISS_ALL_TERMS | VISS_FP64)) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
     cudaGetLastError();
@@ -561,17 +589,34 @@ static bool tracks_allowed(double terms, cudaStream_t st) {
   return cap == cudaStreamCaptureStatusNone;
 }
 
-static int tracks_ready(viss_plan *p, int flags, cudaStream_t st, bool *use) {
-  *use = false;
-  if ((flags & VISS_ALL_TERMS) || !tracks_allowed(static_cast<double>(p->K) * p->J, st)) return VISS_OK;
-  if (p->tracks_version != p->geom_version) {
-    bool ok = false;
-    if (int s = viss::tracks_build(&p->tracks, track_inputs(p), st, &ok)) return s;
-    p->tracks_usable = ok;
-    p->tracks_version = p->geom_version;
-  }
-  *use = p->tracks_usable;
+// Looks at newly staged samples; b.promising says what came of it.
+static int tracks_look(viss_plan::Blocks &b, const viss::TrackInputs &in, long long version, cudaStream_t st) {
+  if (b.version == version) return VISS_OK;
+  b.promising = b.built = b.usable = false;
+  if (int s = viss::tracks_try(&b.state, in, st, &b.promising)) return s;
+  b.version = version;
   return VISS_OK;
+}
+
+static int tracks_built(viss_plan::Blocks &b, const viss::TrackInputs &in, cudaStream_t st, bool *use) {
+  if (!b.built) {
+    if (int s = viss::tracks_build(b.state, in, st, &b.usable)) return s;
+    b.built = true;
+  }
+  *use = b.usable;
+  return VISS_OK;
+}
+
+// Whether a split-precision call goes through the track blocks.
+static int tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint, cudaStream_t st, bool *use) {
+  *use = false;
+  if (static_cast<double>(p->K) * p->J < kTrackMinTerms || !tracks_allowed(flags, st)) return VISS_OK;
+  const viss::TrackInputs in = track_inputs(p);
+  if (int s = tracks_look(p->tracks, in, p->geom_version, st)) return s;
+  if (!p->tracks.promising || viss::tracks_seconds(p->tracks.state, in, masked, adjoint) >=
+                                  kTrackMargin * direct_seconds(p, masked, adjoint))
+    return VISS_OK;
+  return tracks_built(p->tracks, in, st, use);
 }
 
 // Three skies at once, seconds per (sample, pixel): measured 6.0e-13 to 6.3e-13
@@ -592,10 +637,10 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                                    p->channels, first ? p->dev_words : nullptr, st),
             "viss_forward: sky");
   bool use = false;
-  if (tracks && !fp64)
-    if (int s = tracks_ready(p, flags, st, &use)) return s;
+  if (tracks)
+    if (int s = tracks_ready(p, flags, masked, false, st, &use)) return s;
   if (use) {
-    const int s = viss::tracks_forward(p->tracks, track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V), masked,
+    const int s = viss::tracks_forward(p->tracks.state, track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V), masked,
                                        !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                        reinterpret_cast<int *>(p->dev_words + 1), p->drop_tile, st);
     if (s != VISS_ERR_ALLOC) {   // short of memory for its sums: the direct kernel has its workspace
@@ -682,10 +727,12 @@ int viss_forward_skies(viss_plan *p, int n, const float *sky, float *V, int flag
     // before the choice: a captured call evaluates every term, whatever the calls before it took
     if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * n * p->K)) return s;
     if (int s = ensure(p->skies, p->skies_cap, sizeof(float4) * p->Jpad, "sky records")) return s;
-    bool use = false;
-    if (int s = tracks_ready(p, flags, st, &use)) return s;
-    three = !use || n * viss::tracks_seconds(p->tracks, track_inputs(p), masked, false) >
-                        0.95 * kSkiesSeconds[masked] * static_cast<double>(p->K) * static_cast<double>(p->J);
+    if (static_cast<double>(p->K) * p->J >= kTrackMinTerms && tracks_allowed(flags, st)) {
+      const viss::TrackInputs in = track_inputs(p);
+      if (int s = tracks_look(p->tracks, in, p->geom_version, st)) return s;
+      three = !p->tracks.promising || n * viss::tracks_seconds(p->tracks.state, in, masked, false) >=
+                                          kTrackMargin * kSkiesSeconds[masked] * static_cast<double>(p->K) * p->J;
+    }
   }
   if (!three) {
     for (int c = 0; c < n; ++c)
@@ -738,10 +785,10 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
                                     st),
             "viss_adjoint: coef");
   bool use = false;
-  if (tracks && !fp64 && !fcones)
-    if (int s = tracks_ready(p, flags, st, &use)) return s;
+  if (tracks && !fcones)
+    if (int s = tracks_ready(p, flags, masked, true, st, &use)) return s;
   if (use) {
-    const int s = viss::tracks_adjoint(p->tracks, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
+    const int s = viss::tracks_adjoint(p->tracks.state, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
                                        !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                        reinterpret_cast<int *>(p->dev_words + 1), p->drop_tile, st);
     if (s != VISS_ERR_ALLOC) {
@@ -963,19 +1010,28 @@ static viss::TrackInputs form_track_inputs(const viss_plan *p) {
   return in;
 }
 
+// The formation kernels, 1e-13 s per sample and pixel with S satellites, measured
+// unocculted at Nside 64 and 128 (S exponentials serve S (S - 1) / 2 samples); occulted
+// calls cost that of what is seen, and more for tiles seen in part (kFormPart: constant,
+// per share): the least of what was measured at S = 4, 6 and 10, Nside 64 to 256.
+constexpr double kFormSeconds[2][11] = {{0, 0, 24.0, 12.2, 7.5, 5.4, 6.3, 4.9, 4.3, 3.85, 3.5},
+                                        {0, 0, 18.9, 9.6, 6.4, 4.77, 3.91, 3.44, 3.12, 2.8, 2.65}};
+constexpr double kFormPart[2][2] = {{0.0, 1.7}, {0.06, 1.35}};
+
 // Whether a formation call goes through track blocks of its pairs (u = U_a -
-// U_b, the same rows): when they are modelled faster than the formation kernels'
-// seconds (forward 3.07e-13, adjoint 2.43e-13 per sample and pixel at S = 10, Nside
-// 256 x 388,800 samples, Moon + Earth; measured 94.1 against 55 ms and 74.5
-// against 63 ms at 10 MHz).  Per pair S exponentials serve S - 1 / 2: with fewer
-// satellites a pair costs the formation kernels more, which only favours the blocks.
+// U_b, the same rows).
 static int form_tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint, cudaStream_t st, bool *use) {
   *use = false;
-  if (flags & VISS_ALL_TERMS) return VISS_OK;
-  const double per_term = adjoint ? 2.43e-13 : 3.07e-13;
   const long long K = p->form_T * viss::form_pairs(p->form_S);
-  if (!tracks_allowed(static_cast<double>(K) * p->J, st) || !(3.0 * p->form_turns < 262144.0)) return VISS_OK;
-  if (p->form_tracks_version != p->form_version) {
+  viss_plan::Blocks &b = p->form_tracks;
+  auto other = [&]() {
+    double seen, mixed;
+    visible_shares(b, p->form_version, p->J, masked, &seen, &mixed);
+    if (masked) seen += kFormPart[adjoint][0] + kFormPart[adjoint][1] * mixed;
+    return 1e-13 * kFormSeconds[adjoint][p->form_S] * seen * static_cast<double>(K) * p->J;
+  };
+  if (other() < kTrackMinSeconds || !(3.0 * p->form_turns < 262144.0) || !tracks_allowed(flags, st)) return VISS_OK;
+  if (b.version != p->form_version) {
     const bool rows = p->form_sat || p->form_snap;
     if (ensure(p->form_samp, p->form_samp_cap, sizeof(double4) * K, "formation samples") ||
         (rows && ensure(p->form_refs, p->form_refs_cap, sizeof(int4) * K, "formation samples")))
@@ -983,15 +1039,11 @@ static int form_tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint,
     VISS_CUDA(viss::launch_pair_samples(p->form_T, p->form_S, p->form_U, p->form_has_off ? p->form_off : nullptr,
                                         p->form_sat, p->form_snap, p->form_samp, rows ? p->form_refs : nullptr, st),
               "formation samples");
-    bool ok = false;
-    if (int s = viss::tracks_build(&p->form_tracks, form_track_inputs(p), st, &ok)) return s;
-    p->form_tracks_usable = ok;
-    p->form_tracks_version = p->form_version;
   }
   const viss::TrackInputs in = form_track_inputs(p);
-  *use = p->form_tracks_usable &&
-         viss::tracks_seconds(p->form_tracks, in, masked, adjoint) < per_term * static_cast<double>(in.K) * in.J;
-  return VISS_OK;
+  if (int s = tracks_look(b, in, p->form_version, st)) return s;
+  if (!b.promising || viss::tracks_seconds(b.state, in, masked, adjoint) >= kTrackMargin * other()) return VISS_OK;
+  return tracks_built(b, in, st, use);
 }
 
 int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, void *stream) {
@@ -1019,7 +1071,7 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
   const bool masked = (fp.sat_rows || fp.snap_rows);
   if (int s = form_tracks_ready(p, flags, masked, false, st, &use)) return s;
   if (use) {
-    const int s = viss::tracks_forward(p->form_tracks, form_track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V),
+    const int s = viss::tracks_forward(p->form_tracks.state, form_track_inputs(p), p->pixsky, reinterpret_cast<float2 *>(V),
                                        masked, !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                        reinterpret_cast<int *>(p->dev_words + 1), -1, st);
     if (s != VISS_ERR_ALLOC) {
@@ -1072,7 +1124,7 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
   const bool masked = (fp.sat_rows || fp.snap_rows);
   if (int s = form_tracks_ready(p, flags, masked, true, st, &use)) return s;
   if (use) {
-    const int s = viss::tracks_adjoint(p->form_tracks, form_track_inputs(p), reinterpret_cast<const float2 *>(coef),
+    const int s = viss::tracks_adjoint(p->form_tracks.state, form_track_inputs(p), reinterpret_cast<const float2 *>(coef),
                                        image, scale, masked, !(flags & VISS_NO_OFFSET),
                                        (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                        reinterpret_cast<int *>(p->dev_words + 1), -1, st);
@@ -1097,10 +1149,6 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
 }
 
 // ------------------------------------------------------ gridded adjoint
-// The direct adjoint, seconds per (sample, pixel): measured 5.45e-13 unocculted,
-// 5.2e-13 to 5.9e-13 occulted, from 1e9 on.
-constexpr double kDirectSeconds[2] = {5.45e-13, 5.9e-13};
-
 int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float scale, int flags,
                          int64_t facet_pixels, void *stream) {
   const NvtxRange range("viss_adjoint_gridded");
@@ -1128,11 +1176,15 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   double other = 0;
   bool by_tracks = false;
   if (facet_pixels == 0) {
-    if (int s = tracks_ready(p, flags, st, &by_tracks)) return s;
-    if (by_tracks) other = viss::tracks_seconds(p->tracks, track_inputs(p), masked, true);
+    if (static_cast<double>(p->K) * p->J >= kTrackMinTerms && tracks_allowed(flags, st)) {
+      const viss::TrackInputs in = track_inputs(p);
+      if (int s = tracks_look(p->tracks, in, p->geom_version, st)) return s;
+      by_tracks = p->tracks.promising;
+      if (by_tracks) other = viss::tracks_seconds(p->tracks.state, in, masked, true);
+    }
     if (p->max_turns < viss::kMaxTurns) {
-      const double direct = kDirectSeconds[masked] * static_cast<double>(p->K) * static_cast<double>(p->J);
-      if (!by_tracks || direct < other) other = direct, by_tracks = false;
+      const double direct = direct_seconds(p, masked, true);
+      if (!by_tracks || kTrackMargin * direct <= other) other = direct, by_tracks = false;
     }
     if (other > 0) {
       VISS_CUDA(cudaMemsetAsync(p->dev_words + 3, 0, sizeof(unsigned long long), st), "viss_adjoint_gridded");
@@ -1153,12 +1205,17 @@ int viss_adjoint_gridded(viss_plan *p, const float *coef, float *image, float sc
   p->gridded_hbm_blocks = info;
   p->last_stream = st;
   if (s == 1) {
-    if (by_tracks) {
+    bool use = by_tracks;
+    if (by_tracks)
+      if (int b = tracks_built(p->tracks, track_inputs(p), st, &use)) return b;
+    if (use) {
       VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint_gridded");
-      s = viss::tracks_adjoint(p->tracks, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
+      s = viss::tracks_adjoint(p->tracks.state, track_inputs(p), reinterpret_cast<const float2 *>(coef), image, scale, masked,
                                !(flags & VISS_NO_OFFSET), (flags & VISS_ACCUMULATE) != 0, p->dev_words,
                                reinterpret_cast<int *>(p->dev_words + 1), -1, st);
       if (s == VISS_OK) p->last_total = p->K * p->J;
+    } else if (by_tracks) {
+      s = VISS_ERR_ALLOC;                          // no room for the blocks
     } else {
       s = adjoint_impl(p, coef, image, scale, flags, st, p->adj_shape, nullptr, 0, 0, nullptr, 0, false);
     }

@@ -23,20 +23,24 @@ struct TrackInputs {
   double max_turns;        // bound on |u.s + off|
 };
 
-// Builds the track blocks of the staged samples into *state (allocated on
-// first use, buffers kept).  *usable = false when the samples are not smooth
-// enough to gain, or memory is short; the direct kernels take the call then.
-// Waits for `st` a few times; must not run under stream capture.
-int tracks_build(void **state, const TrackInputs &in, cudaStream_t st, bool *usable);
+// Looks at a few blocks of the staged samples (*state: allocated on first use,
+// buffers kept).  *promising = false when the samples are not smooth enough for
+// nodes to pay, or memory is short; the direct kernels take the calls then.  Waits
+// for `st` a few times; must not run under stream capture.
+int tracks_try(void **state, const TrackInputs &in, cudaStream_t st, bool *promising);
+// Builds the blocks of the samples that tracks_try found promising; likewise.
+int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usable);
 void tracks_free(void *state);
 
-// Modelled time of one call with the built blocks, in seconds: per (sample, pixel)
-// and modelled issue slot 3.1e-14 (forward) or 3.3e-14 s (adjoint), and in an
-// occulted call 0.85 of that, for what is hidden, plus the pairs at the rims, whose
-// share goes with the width of a tile: 4.3e-11 or 5.5e-11 / sqrt(J).  Within 10 %
-// of nine calls of 1e10 to 3e11 terms at Nside 128 and 256, 1 to 10 MHz, occulted
-// and not (9.6e-14 to 3.4e-13 s per term).
+// Modelled time of one call through the blocks, in seconds, from what tracks_try
+// counted in its blocks.  Fitted to 105 observations of 1e10 to 7e11 terms (Nside 48
+// to 512, 500 to 8,640 snapshots, 4 to 10 satellites, 0.3 to 10 MHz), each occulted and
+// not, those near the direct kernels' time weighted most, and checked on 100 others of
+// 1e10 to 4e10: within 24 % (forward) and 24 % below to 58 % above (adjoint), the
+// largest where blocks are several times faster.
 double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint);
+// Shares of the (sample, tile) pairs that an occulted call sees, and sees in part.
+void tracks_shares(const void *state, double *seen, double *mixed);
 
 // drop_tile from here on: the interpolation's first product instead of a tile's copy.
 constexpr int kDropProduct = 1 << 30;

@@ -16,9 +16,8 @@ namespace {
 constexpr double kNodeNoise2 = 4e-14;            // kNodeNoise^2
 constexpr int kLagMax = 1024;                    // tracks interleaved in the caller's order, at most
 constexpr int kLagSamples = 128;
-constexpr int kRankSamples = 48;                 // blocks that decide whether nodes pay at all
-constexpr int kShares = 4;                       // radii tried per class
-constexpr int kRadii = kClasses * kShares;
+constexpr int kBuckets = kTrackRankMax / 16 + 1; // blocks of similar rank are stored together
+constexpr int kRankSamples = 48;                 // blocks that decide whether nodes pay
 // Node sums of one slab of blocks: large enough that a slab's kernels fill the
 // device several times over.
 constexpr size_t kSlabBytes = 1ull << 28;
@@ -172,18 +171,13 @@ __device__ int track_factor(TrackFactor &f, bool valid, const double4 &u, double
   }
 }
 
-// Ranks of natural blocks (all nb, or gridDim.x scattered ones: an even stride
-// would favour some tracks) for group radius rho[blockIdx.y] and at most
-// most[blockIdx.y] nodes, as rank[blockIdx.y][block] (0: more).
-struct RadiusSet {
-  double rho[kRadii];
-  int most[kRadii];
-};
-__global__ void __launch_bounds__(kTrackT) k_track_ranks(TrackShape s, int nb, const double4 *samp,
+// Ranks of natural blocks (which: of all, if null) for group radius rho[blockIdx.y]
+// and at most most[blockIdx.y] nodes, as rank[blockIdx.y][block] (0: more).
+__global__ void __launch_bounds__(kTrackT) k_track_ranks(TrackShape s, const int *which, const double4 *samp,
                                                          RadiusSet radii, int *rank) {
   extern __shared__ __align__(128) unsigned char smem[];
   TrackFactor &f = *reinterpret_cast<TrackFactor *>(smem);
-  const int b = gridDim.x == nb ? blockIdx.x : static_cast<int>(blockIdx.x * 2654435761u % static_cast<unsigned>(nb));
+  const int b = which ? which[blockIdx.x] : static_cast<int>(blockIdx.x);
   const long long k = block_sample(s, b, threadIdx.x);
   const double4 u = k >= 0 ? samp[k] : make_double4(0, 0, 0, 0);
   const int r = track_factor(f, k >= 0, u, radii.rho[blockIdx.y], radii.most[blockIdx.y]);
@@ -255,10 +249,6 @@ __device__ __forceinline__ unsigned valid_tiles(int w, int ntiles) {
 // tiles whose group is within the class's radius (radius: per class, its
 // groups', concatenated from at[c]), merged tiles, and the others.  left: bit c
 // set where class c leaves a tile.
-struct ClassSet {
-  double rho[kClasses];
-  int at[kClasses];
-};
 __global__ void k_track_class_rows(int W, int ntiles, const float *radius, ClassSet cs, unsigned *full,
                                    unsigned *merged, unsigned *rest, unsigned long long *left) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
@@ -375,6 +365,70 @@ __global__ void k_track_bits(int W, int ntiles, const int *slot, const int4 *ref
   if (lane == 0 && npart) atomicAdd(count + 1, npart);
 }
 
+// Sums over the blocks' tiles of a call's work (TrackEstimate's members in order;
+// refs null: an unocculted call), as k_track_bits classifies them.
+constexpr int kEstimates = 8;
+__global__ void k_track_estimate(int W, int ntiles, const int *slot, const int4 *refs, const float4 *occ32,
+                                 const float4 *cones, const int *cls, const int *rank, const unsigned *crow,
+                                 unsigned long long *sums) {
+  const int b = static_cast<int>(blockIdx.x), lane = threadIdx.x & 31;
+  const int warps = blockDim.x / 32 * gridDim.y, w0 = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32;
+  SampleRows rows[4];
+  bool val[4];
+  int nvalid = 0;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const long long i = static_cast<long long>(b) * kTrackT + 32 * s + lane;
+    val[s] = slot[i] >= 0;
+    rows[s] = sample_rows(val[s] && refs ? refs[i] : make_int4(-1, -1, -1, -1), occ32);
+    nvalid += __popc(__ballot_sync(0xffffffffu, val[s]));
+  }
+  // samples that see part of a cone, and all of it
+  auto count = [&](const float4 &cone, int &part, int &all) {
+    part = all = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int st = val[s] ? cone_rows_state(cone, rows[s]) : 0;
+      part += __popc(__ballot_sync(0xffffffffu, st == 1));
+      all += __popc(__ballot_sync(0xffffffffu, st == 2));
+    }
+  };
+  const int c = cls[b], r = rank[b];
+  unsigned long long sum[kEstimates] = {};
+  for (int w = w0; w < W; w += warps) {
+    const unsigned ok = crow[c * W + w], valid = valid_tiles(w, ntiles);
+    unsigned full = 0, taken = 0;
+    for (int q = 0; q < 32 / kSuperTiles; ++q) {
+      const int t0 = 32 * w + q * kSuperTiles;
+      if (t0 >= ntiles) break;
+      int part, all;
+      count(cones[5LL * ntiles + t0 / kSuperTiles], part, all);
+      const bool refine = part > 0;
+      for (int i = 0; i < kSuperTiles && t0 + i < ntiles; ++i) {
+        const int bit = q * kSuperTiles + i;
+        if (refine) count(cones[t0 + i], part, all);
+        const bool in = (ok >> bit) & 1u;
+        const int rest = part + (in ? 0 : all);
+        full |= static_cast<unsigned>(in && all == nvalid) << bit;
+        taken |= static_cast<unsigned>(in && all > 0) << bit;
+        sum[3] += rest > 0;
+        sum[4] += rest;
+        sum[5] += part + all;
+        sum[6] += part;
+      }
+    }
+    const unsigned first = c == 2 ? 0x55555555u : 0x01010101u;
+    const unsigned units = __popc(taken & ~(merged_tiles(full, valid, c) & ~first)) * (c == kHalf ? 2 : 1);
+    sum[0] += static_cast<unsigned long long>(__popc(taken)) * kTilePix * r;
+    sum[1] += static_cast<unsigned long long>(units) * kTrackT;
+    sum[2] += static_cast<unsigned long long>(units) * kTrackT * r;
+    if (r > kOneCtaRank) sum[7] += static_cast<unsigned long long>(units) * kTrackT;
+  }
+  if (lane == 0)
+    for (int i = 0; i < kEstimates; ++i)
+      if (sum[i]) atomicAdd(sums + i, sum[i]);
+}
+
 // Sample masks of the part tiles: a word's masks stand together, in the order
 // of its tiles, wherever `next` had room (mask_at).
 __global__ void k_track_masks(int W, const int *slot, const int4 *refs, const float4 *occ32, const float4 *cones,
@@ -414,13 +468,56 @@ void tracks_free(void *state) { delete static_cast<TrackState *>(state); }
 
 double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint) {
   const TrackState &S = *static_cast<const TrackState *>(state);
-  double per = (adjoint ? 3.3e-14 : 3.1e-14) * S.cost;
-  if (masked) per = 0.85 * per + (adjoint ? 5.5e-11 : 4.3e-11) / std::sqrt(static_cast<double>(in.J));
-  return static_cast<double>(in.K) * in.J * per;
+  const TrackEstimate &e = S.est[masked];
+  if (!adjoint)                                    // few blocks: short slabs, whose last waves are mostly empty
+    return (5.62e-13 * e.nodes + 1.6e-13 * e.units + 9.6e-14 * e.unit_nodes + 9.64e-12 * e.wide_units +
+            1.26e-8 * e.rest_blocks + 1.22e-4 * S.slab_count + 9.2e-5) * (1.0 + 20.0 / S.nb);
+  // unocculted, the few warps of the tiles that are left walk all samples alone
+  return 2.23e-13 * e.nodes + 8.92e-12 * e.units + 5.4e-14 * e.unit_nodes + 1.85e-10 * e.rest_samples +
+         (!masked && S.leaves_tiles ? 2.0e-9 * static_cast<double>(in.K) : 0.0) + 1.5e-4 * S.slab_count + 1.66e-4;
 }
 
-int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *usable) {
-  *usable = false;
+void tracks_shares(const void *state, double *seen, double *mixed) {
+  const TrackState &S = *static_cast<const TrackState *>(state);
+  *seen = S.est[1].seen;
+  *mixed = S.est[1].mixed;
+}
+
+namespace {
+
+// Modelled time of a block's nodes and interpolation per (sample, pixel), in issue
+// slots of a scheduler, by which classes are chosen: an evaluated exponential term
+// takes 21, an interpolated (sample, unit) about r + 100 (both measured on the 1 and
+// 10 MHz Nside 256 observations), and a term left to the remainder kernels 1.5 times
+// that of k_forward / k_adjoint (one sample per lane, no shared staging).
+constexpr double kTermSlots = 21.0, kLeftSlots = 1.5 * kTermSlots;
+double block_slots(int c, int r, int len) {
+  return r ? kTermSlots * r / len + (r + 100.0) / group_pix(c) : kLeftSlots;
+}
+
+}  // namespace
+
+namespace {
+
+// n natural blocks to look at, spread evenly over tracks and time together (the R2
+// sequence, M. Roberts 2018: multiples of 1/g and 1/g^2, g^3 = g + 1) and the
+// channels in turn: a baseline's length decides its ranks, and 48 blocks picked at
+// random of 200 misjudged some calls by a fifth.
+std::vector<int> spread_blocks(const TrackShape &s, int nb, int n) {
+  std::vector<int> at(n);
+  const int nbc = s.blocks_per_channel();
+  auto part = [](double x, int m) { return std::min(m - 1, static_cast<int>((x - std::floor(x)) * m)); };
+  for (int i = 0; i < n; ++i)
+    at[i] = n == nb ? i
+                    : i % s.channels * nbc + part(0.5 + 0.5698402909980532 * i, s.nbt) * s.lag +
+                          part(0.5 + 0.7548776662466927 * i, s.lag);
+  return at;
+}
+
+}  // namespace
+
+int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *promising) {
+  *promising = false;
   if (!*statep) *statep = new (std::nothrow) TrackState();
   if (!*statep) return 0;
   TrackState &S = *static_cast<TrackState *>(*statep);
@@ -440,16 +537,27 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     total += ngs[c];
   }
   float *radius_d, *score_d;
-  int *trial_rank_d;
-  unsigned long long *counts_d;
+  int *trial_rank_d, *order_d, *cls_d, *slot_d;
+  double4 *samp_d;
+  int4 *refs_d;
+  unsigned long long *sums_d;
+  const size_t slots = static_cast<size_t>(kRankSamples) * kTrackT, crows = static_cast<size_t>(kClasses + 1) * ((in.ntiles + 31) / 32);
   if (!S.trial.reset(TrackArena::bytes<double4>(total) + TrackArena::bytes<float>(total) + TrackArena::bytes<float>(lags) +
-                     TrackArena::bytes<int>(kRadii * kRankSamples) + TrackArena::bytes<unsigned long long>(5)))
+                     TrackArena::bytes<int>(kRadii * kRankSamples) + 2 * TrackArena::bytes<int>(2 * kRankSamples) +
+                     TrackArena::bytes<int>(slots) + TrackArena::bytes<double4>(slots) + TrackArena::bytes<int4>(slots) +
+                     3 * TrackArena::bytes<unsigned>(crows) + TrackArena::bytes<unsigned long long>(1 + 2 * kEstimates)))
     return 0;
   S.trial.take(S.gcen, total);
   S.trial.take(radius_d, total);
   S.trial.take(score_d, lags);
   S.trial.take(trial_rank_d, kRadii * kRankSamples);
-  S.trial.take(counts_d, 5);
+  S.trial.take(order_d, 2 * kRankSamples);
+  S.trial.take(cls_d, 2 * kRankSamples);           // classes, then ranks
+  S.trial.take(slot_d, slots);
+  S.trial.take(samp_d, slots);
+  S.trial.take(refs_d, slots);
+  for (auto &row : S.crow) S.trial.take(row, crows);
+  S.trial.take(sums_d, 1 + 2 * kEstimates);        // classes that leave tiles, unocculted, occulted
   for (int c = 0; c < kClasses; ++c) {
     k_track_groups<<<blks(ngs[c], 8), 256, 0, st>>>(ngs[c], group_pix(c), in.Jpad, in.pix, S.gcen + S.gat[c],
                                                     radius_d + S.gat[c]);
@@ -478,13 +586,6 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   const int nb = static_cast<int>(nbl);
   S.W = (in.ntiles + 31) / 32;
   if (static_cast<double>(nb) * S.W > INT_MAX) return 0;
-  // Modelled time per (sample, pixel), in issue slots of a scheduler: an
-  // evaluated exponential term takes 21, an interpolated (sample, unit) about
-  // r + 100 (both measured on the 1 and 10 MHz Nside 256 observations), and a
-  // term left to the remainder kernels 1.5 times that of k_forward / k_adjoint
-  // (one sample per lane, no shared staging).
-  const double term = 21.0, left = 1.5 * term;
-  auto cost = [&](int c, int r) { return r ? term * r / sh.len + (r + 100.0) / group_pix(c) : left; };
   // A class's radius: a percentile of its groups' (wider groups are left) with
   // the least time over some blocks.  On a power-of-two HEALPix grid all groups
   // are alike and the largest wins; elsewhere a few are far wider than the rest.
@@ -507,15 +608,17 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     }
   }
   const int nsamp = std::min(nb, kRankSamples);
+  const std::vector<int> order = spread_blocks(sh, nb, nsamp);
+  TRACK_CUDA(cudaMemcpyAsync(order_d, order.data(), sizeof(int) * nsamp, cudaMemcpyHostToDevice, st), "order");
   std::vector<int> rk(static_cast<size_t>(kRadii) * nsamp);
   auto block_cost = [&](int at, int i) {
-    return within[at] * cost(at / kShares, rk[static_cast<size_t>(at) * nsamp + i]) + (1.0 - within[at]) * left;
+    return within[at] * block_slots(at / kShares, rk[static_cast<size_t>(at) * nsamp + i], sh.len) + (1.0 - within[at]) * kLeftSlots;
   };
   // first the smallest groups alone: samples too sparse for those end here
   auto ranks_of = [&](int first, int n) -> cudaError_t {
     RadiusSet some{};
     for (int q = 0; q < n; ++q) some.rho[q] = trial.rho[first + q], some.most[q] = trial.most[first + q];
-    k_track_ranks<<<dim3(nsamp, n), kTrackT, sizeof(TrackFactor), st>>>(sh, nb, in.samp, some, trial_rank_d);
+    k_track_ranks<<<dim3(nsamp, n), kTrackT, sizeof(TrackFactor), st>>>(sh, order_d, in.samp, some, trial_rank_d);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = cudaMemcpyAsync(rk.data() + static_cast<size_t>(first) * nsamp, trial_rank_d, sizeof(int) * n * nsamp,
@@ -523,9 +626,10 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);
   };
   int pick_q[kClasses];
-  std::vector<double> least(nsamp, left);          // a block's best class so far
-  double mean = 0;
-  bool chosen[kClasses] = {};
+  std::vector<double> least(nsamp, kLeftSlots);    // a block's best class so far
+  std::vector<int> least_cls(2 * nsamp, kClasses); // that class, and the rank
+  std::fill(least_cls.begin() + nsamp, least_cls.end(), 0);
+  for (bool &c : S.chosen) c = false;
   for (int pass = 0; pass < 2; ++pass) {
     TRACK_CUDA(ranks_of(pass ? kShares : 0, pass ? kRadii - kShares : kShares), "ranks");
     for (int c = pass ? 1 : 0; c < (pass ? kClasses : 1); ++c) {
@@ -537,56 +641,104 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
       }
       for (int i = 0; i < nsamp; ++i) {
         const double v = block_cost(pick_q[c], i);
-        if (v < least[i]) least[i] = v, chosen[c] = true;
+        if (v < least[i]) {
+          least[i] = v, least_cls[i] = c, least_cls[nsamp + i] = rk[static_cast<size_t>(pick_q[c]) * nsamp + i];
+          S.chosen[c] = true;
+        }
       }
     }
-    mean = 0;
+    // the smallest groups alone: samples that even those leave near the cost of a
+    // call without track blocks end here (larger groups only help where those do)
+    double mean = 0;
     for (double v : least) mean += v / nsamp;
-    // against `term`, the cost of a call without track blocks (occultation adds
-    // to both): at .63 to .70 an occulted call takes .81 to .95 of the direct
-    // kernels' time, and a build about 3 % of the smallest call's that gets here.
-    // Larger groups only help where the smallest already do.
-    if (!(mean < (pass ? 0.70 : 0.82) * term)) return 0;
+    if (!(mean < 0.82 * kTermSlots)) return 0;
   }
-  // every block's ranks in the classes some sampled block takes (the smallest always)
-  chosen[kHalf] = true;
-  RadiusSet radii{}, some{};
+  S.chosen[kHalf] = true;
   ClassSet cs{};
-  int nclass = 0, class_of[kClasses];
   for (int c = 0; c < kClasses; ++c) {
-    cs.rho[c] = radii.rho[c] = trial.rho[pick_q[c]];
-    radii.most[c] = trial.most[pick_q[c]];
+    cs.rho[c] = S.radii.rho[c] = trial.rho[pick_q[c]];
+    S.radii.most[c] = trial.most[pick_q[c]];
     cs.at[c] = S.gat[c];
-    if (!chosen[c]) continue;
-    some.rho[nclass] = radii.rho[c];
-    some.most[nclass] = radii.most[c];
-    class_of[nclass++] = c;
   }
-  // a block's class, and the stored order: by channel, class, similar rank, then as they come
   S.nb = nb;
   S.shape = sh;
   S.Ks = nbl * kTrackT;
+  // those blocks' share of a call's work
+  TRACK_CUDA(cudaMemcpyAsync(cls_d, least_cls.data(), sizeof(int) * 2 * nsamp, cudaMemcpyHostToDevice, st), "classes");
+  TRACK_CUDA(cudaMemsetAsync(sums_d, 0, (1 + 2 * kEstimates) * sizeof(unsigned long long), st), "sums");
+  k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, radius_d, cs, S.crow[0],
+                                                                         S.crow[1], S.crow[2], sums_d);
+  TRACK_CUDA(cudaGetLastError(), "class rows");
+  k_track_slots<<<blks(nsamp * kTrackT, 256), 256, 0, st>>>(sh, nsamp * kTrackT, order_d, in.samp, in.refs, slot_d,
+                                                            samp_d, refs_d);
+  TRACK_CUDA(cudaGetLastError(), "slots");
+  const unsigned by = static_cast<unsigned>(std::max(1, std::min((S.W + 3) / 4, (8 * in.nsm + nsamp - 1) / nsamp)));
+  for (int m = 0; m < (in.refs ? 2 : 1); ++m) {
+    k_track_estimate<<<dim3(nsamp, by), 128, 0, st>>>(S.W, in.ntiles, slot_d, m ? refs_d : nullptr, in.occ32, in.cones,
+                                                      cls_d, cls_d + nsamp, S.crow[0], sums_d + 1 + m * kEstimates);
+    TRACK_CUDA(cudaGetLastError(), "estimate");
+  }
+  unsigned long long sums[1 + 2 * kEstimates] = {};
+  TRACK_CUDA(cudaMemcpyAsync(sums, sums_d, sizeof(sums), cudaMemcpyDeviceToHost, st), "estimate");
+  TRACK_CUDA(cudaStreamSynchronize(st), "estimate");
+  const double all = static_cast<double>(nb) / nsamp;
+  for (int m = 0; m < 2; ++m) {
+    const unsigned long long *v = sums + 1 + m * kEstimates;
+    TrackEstimate &e = S.est[m];
+    e.nodes = all * v[0], e.units = all * v[1], e.unit_nodes = all * v[2];
+    e.rest_blocks = all * v[3], e.rest_samples = all * v[4];
+    const double pairs = static_cast<double>(in.K) * in.ntiles;
+    e.seen = all * v[5] / pairs, e.mixed = all * v[6] / pairs;
+    e.wide_units = all * v[7];
+  }
+  S.class_rest = sums[0];
+  S.leaves_tiles = false;
+  bool bucket[kClasses * kBuckets] = {};           // classes and similar ranks that blocks have
+  for (int i = 0; i < nsamp; ++i) {
+    const int c = least_cls[i], r = least_cls[nsamp + i];
+    if (c < kClasses) bucket[c * kBuckets + (r + 15) / 16] = true;
+    S.leaves_tiles = S.leaves_tiles || (S.class_rest >> c & 1u);
+  }
+  S.slab_count = static_cast<double>(sh.channels) * std::count(bucket, bucket + kClasses * kBuckets, true);
+  *promising = true;
+  return 0;
+}
+
+int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usable) {
+  *usable = false;
+  TrackState &S = *static_cast<TrackState *>(state);
+  const TrackShape sh = S.shape;
+  const int nb = S.nb;
+  // every block's ranks in the classes some block looked at takes (the smallest always)
+  RadiusSet some{};
+  int nclass = 0, class_of[kClasses];
+  for (int c = 0; c < kClasses; ++c) {
+    if (!S.chosen[c]) continue;
+    some.rho[nclass] = S.radii.rho[c];
+    some.most[nclass] = S.radii.most[c];
+    class_of[nclass++] = c;
+  }
+  // a block's class, and the stored order: by channel, class, similar rank, then as they come
   const bool masked = in.refs != nullptr;
   const size_t pairs = static_cast<size_t>(nb) * S.W;
   int *all_ranks_d;
   if (!S.masks.reset(TrackArena::bytes<int>(static_cast<size_t>(nclass) * nb))) return 0;
   S.masks.take(all_ranks_d, static_cast<size_t>(nclass) * nb);
-  k_track_ranks<<<dim3(nb, nclass), kTrackT, sizeof(TrackFactor), st>>>(sh, nb, in.samp, some, all_ranks_d);
+  k_track_ranks<<<dim3(nb, nclass), kTrackT, sizeof(TrackFactor), st>>>(sh, nullptr, in.samp, some, all_ranks_d);
   TRACK_CUDA(cudaGetLastError(), "ranks");
-  rk.resize(static_cast<size_t>(nclass) * nb);
+  std::vector<int> rk(static_cast<size_t>(nclass) * nb);
   TRACK_CUDA(cudaMemcpyAsync(rk.data(), all_ranks_d, sizeof(int) * rk.size(), cudaMemcpyDeviceToHost, st), "ranks");
   TRACK_CUDA(cudaStreamSynchronize(st), "ranks");
   const int nbc = sh.blocks_per_channel();
   std::vector<int> pick(nb, kClasses), pick_rank(nb, 0);
   for (int b = 0; b < nb; ++b) {
-    double m = left;
+    double m = kLeftSlots;
     for (int i = 0; i < nclass; ++i) {
       const int r = rk[static_cast<size_t>(i) * nb + b];
-      const double v = cost(class_of[i], r);
+      const double v = block_slots(class_of[i], r, sh.len);
       if (v < m) m = v, pick[b] = class_of[i], pick_rank[b] = r;
     }
   }
-  constexpr int kBuckets = kTrackRankMax / 16 + 1;
   std::vector<std::vector<int>> piles(static_cast<size_t>(sh.channels) * (kClasses + 1) * kBuckets);
   for (int b = 0; b < nb; ++b)
     piles[(static_cast<size_t>(b / nbc) * (kClasses + 1) + pick[b]) * kBuckets + (pick_rank[b] + 15) / 16].push_back(b);
@@ -622,12 +774,12 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   }
   if (n == 0) return 0;
   const size_t nodes = (n + 31) / 32 * 32, rows = masked ? pairs : 0;
-  const size_t crows = static_cast<size_t>(kClasses + 1) * S.W, sums = static_cast<size_t>(in.ntiles) * S.ld_max;
+  const size_t sums = static_cast<size_t>(in.ntiles) * S.ld_max;
   if (!S.plan.reset(TrackArena::bytes<int>(S.Ks) + 4 * TrackArena::bytes<int>(nb) + TrackArena::bytes<int>(nodes) +
                     TrackArena::bytes<double4>(S.Ks) + TrackArena::bytes<double4>(nodes) +
                     TrackArena::bytes<int4>(masked ? S.Ks : 0) + TrackArena::bytes<float>(nodes * kTrackT) +
-                    3 * TrackArena::bytes<unsigned>(crows) + 4 * TrackArena::bytes<unsigned>(rows) +
-                    TrackArena::bytes<int>(rows) + TrackArena::bytes<float2>(sums)))
+                    4 * TrackArena::bytes<unsigned>(rows) + TrackArena::bytes<int>(rows) +
+                    TrackArena::bytes<float2>(sums) + TrackArena::bytes<unsigned long long>(4)))
     return 0;
   S.plan.take(S.slot, S.Ks);
   for (int **p : {&S.order, &S.cls, &S.rank, &S.noff}) S.plan.take(*p, nb);
@@ -636,10 +788,11 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   S.plan.take(S.node, nodes);
   S.plan.take(S.refs, masked ? S.Ks : 0);
   S.plan.take(S.P, nodes * kTrackT);
-  for (auto &row : S.crow) S.plan.take(row, crows);
   for (auto &row : S.brow) S.plan.take(row, rows);
   S.plan.take(S.mask_at, rows);
   S.plan.take(S.sums, sums);
+  unsigned long long *counts_d;                    // rest pairs, part pairs, ranks that differ; masks taken
+  S.plan.take(counts_d, 4);
   auto up = [&](int *dst, const std::vector<int> &v) {
     return cudaMemcpyAsync(dst, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, st);
   };
@@ -651,35 +804,31 @@ int tracks_build(void **statep, const TrackInputs &in, cudaStream_t st, bool *us
   TRACK_CUDA(cudaGetLastError(), "slots");
   TRACK_CUDA(cudaMemsetAsync(S.node, 0, sizeof(double4) * nodes, st), "nodes");
   TRACK_CUDA(cudaMemsetAsync(S.nodeblk, 0xff, sizeof(int) * nodes, st), "nodes");
-  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 5 * sizeof(unsigned long long), st), "counts");
-  k_track_weights<<<nb, kTrackT, sizeof(TrackFactor), st>>>(S.slot, S.samp, radii, S.cls, S.rank, S.noff, S.node,
-                                                           S.nodeblk, S.P, counts_d + 3);
+  TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 4 * sizeof(unsigned long long), st), "counts");
+  k_track_weights<<<nb, kTrackT, sizeof(TrackFactor), st>>>(S.slot, S.samp, S.radii, S.cls, S.rank, S.noff, S.node,
+                                                           S.nodeblk, S.P, counts_d + 2);
   TRACK_CUDA(cudaGetLastError(), "weights");
-  k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, radius_d, cs, S.crow[0],
-                                                                         S.crow[1], S.crow[2], counts_d + 2);
-  TRACK_CUDA(cudaGetLastError(), "class rows");
   const unsigned by = static_cast<unsigned>(std::max(1, std::min(S.W / 8, (4 * in.nsm * 8) / nb + 1)));
   if (masked) {
     k_track_bits<<<dim3(nb, by), 128, 0, st>>>(S.W, in.ntiles, S.slot, S.refs, in.occ32, in.cones, S.cls, S.crow[0],
                                                S.brow[0], S.brow[1], S.brow[2], S.brow[3], counts_d);
     TRACK_CUDA(cudaGetLastError(), "pair bits");
   }
-  unsigned long long pairs_of[4] = {0, 0, 0, 0};   // rest, part, classes that leave tiles, ranks that differ
+  unsigned long long pairs_of[3] = {0, 0, 0};
   TRACK_CUDA(cudaMemcpyAsync(pairs_of, counts_d, sizeof(pairs_of), cudaMemcpyDeviceToHost, st), "counts");
   TRACK_CUDA(cudaStreamSynchronize(st), "build");
-  if (pairs_of[3]) return 0;
+  if (pairs_of[2]) return 0;
   if (masked) {
     if (pairs_of[1] > INT_MAX || !S.masks.reset(TrackArena::bytes<uint4>(pairs_of[1]))) return 0;
     S.masks.take(S.mask, pairs_of[1]);
     k_track_masks<<<dim3(nb, by), 128, 0, st>>>(S.W, S.slot, S.refs, in.occ32, in.cones, S.brow[1], S.mask_at, S.mask,
-                                                counts_d + 4);
+                                                counts_d + 3);
     TRACK_CUDA(cudaGetLastError(), "sample masks");
     TRACK_CUDA(cudaStreamSynchronize(st), "build");  // later calls may come on other streams
   }
   S.has_rest[1] = pairs_of[0] != 0;
   S.has_rest[0] = false;                           // unocculted: tiles a used class leaves
-  for (const TrackSlab &sl : S.slabs) S.has_rest[0] = S.has_rest[0] || (pairs_of[2] >> sl.cls & 1u);
-  S.cost = mean;
+  for (const TrackSlab &sl : S.slabs) S.has_rest[0] = S.has_rest[0] || (S.class_rest >> sl.cls & 1u);
   *usable = true;
   return 0;
 }

@@ -75,13 +75,39 @@ struct TrackArena {
   }
 };
 
+// What a call has to do, estimated from a few blocks: node exponentials, (sample,
+// unit) pairs and those times the rank, (block, tile) and (sample, tile) pairs of
+// the remainder; the share of (sample, tile) pairs that are seen at all and in part;
+// (sample, unit) pairs of ranks whose interpolation leaves room for one CTA per SM.
+struct TrackEstimate {
+  double nodes = 0, units = 0, unit_nodes = 0, rest_blocks = 0, rest_samples = 0, seen = 0, mixed = 0, wide_units = 0;
+};
+constexpr int kOneCtaRank = 52;
+
+constexpr int kShares = 4;                       // radii tried per class
+constexpr int kRadii = kClasses * kShares;
+struct RadiusSet {
+  double rho[kRadii];
+  int most[kRadii];
+};
+struct ClassSet {
+  double rho[kClasses];
+  int at[kClasses];
+};
+
 struct TrackState {
   TrackArena trial, plan, masks, fwd, adj;
+  TrackEstimate est[2];                    // unocculted, occulted
+  double slab_count = 0;                   // slabs, but for those that a class of one rank is cut into by memory
+  unsigned long long class_rest = 0;       // bit c: class c leaves tiles
+  bool leaves_tiles = false;               // a class that blocks take does
+  RadiusSet radii{};                       // per class
+  bool chosen[kClasses] = {};
   int *slot = nullptr, *order = nullptr, *cls = nullptr, *rank = nullptr, *noff = nullptr, *nodeblk = nullptr;
   double4 *samp = nullptr, *node = nullptr, *gcen = nullptr;
   int4 *refs = nullptr;
   float *P = nullptr;
-  unsigned *crow[3] = {};                  // class rows: full, merged, rest
+  unsigned *crow[3] = {};                  // class rows: full, merged, rest (in `trial`)
   unsigned *brow[4] = {};                  // occulted: full, part, merged, rest per block
   int *mask_at = nullptr;
   uint4 *mask = nullptr;
@@ -91,7 +117,6 @@ struct TrackState {
   int gat[kClasses] = {0, 0, 0, 0};        // a class's first centre in gcen
   long long Ks = 0, ld_max = 0;
   bool has_rest[2] = {false, false};       // unocculted, occulted
-  double cost = 0;                         // modelled issue slots per (sample, pixel); an evaluated term is 21
   std::vector<TrackSlab> slabs;
 
   TrackBits bits(bool occulted) const {
