@@ -27,8 +27,8 @@
 // below 1.8 kNodeNoise^2 (no sample above 4.5): (2.7e-7)^2, where a term that
 // k_forward evaluates is off by 3.7e-7 (a phase of 23 bits).  Measured against
 // FP64 on four inputs each of 1 to 10 MHz observations at Nside 128 and 256: V 2.0e-7 -
-// 3.0e-7, images of random coefficients 2.8e-7 - 3.0e-7 and of the observations 2.2e-7
-// - 3.1e-7; the direct kernels 2.5e-7 - 4.6e-7, 5.0e-7 and 2.6e-7 - 5.4e-7.
+// 3.2e-7, images of random coefficients 2.8e-7 - 3.0e-7 and of the observations 2.3e-7
+// - 3.2e-7; the direct kernels 2.5e-7 - 4.6e-7, 5.0e-7 and 2.6e-7 - 5.4e-7.
 // Stopping at 0.85 (3e-7)^2 with the same node error costs 25 % more nodes
 // for 8 % less error, stopping at 2.5 saves 1 %.  Blocks that need more than
 // kTrackRankMax nodes, or three quarters of their samples, are left to the
@@ -97,11 +97,13 @@ __device__ __forceinline__ float turn_angle32(double t) {
 
 constexpr int kNodeNT = 256;
 constexpr int kNodeR = 4;
-// Terms added in plain FP32 before a run's sum joins the others, in both directions.
-// A run of 128 (256 additions in the adjoint) left 1.9e-7 (2.7e-7) of the sum's own
-// size; with 32, images of random coefficients went from 3.75e-7 to 2.85e-7 of error
-// at 1 MHz, V from 3.0e-7 to 2.75e-7 at 10 MHz, in the same time.
-constexpr int kNodeRun = 32;
+// Terms added in plain FP32 before a run's sum joins the others: pixels in the
+// forward, nodes (two additions each) in the adjoint.  Runs of 128 left 1.9e-7 and
+// 2.7e-7 of the sum's own size.  Images of random coefficients went from 3.75e-7 to
+// 2.85e-7 of error at 1 MHz in the same time.  In the forward at 10 MHz runs of 32 took V
+// from 3.0e-7 to 2.75e-7 for 1.2 % of the time, runs of 64 to 2.9e-7 for none (53.3 and
+// 52.6 ms; its images are at 3.1e-7 with either).
+constexpr int kFwdRun = 64, kNodeRun = 32;
 
 // G of the slab's nodes (R per thread) over a chunk of tiles: the inner loop
 // and the stage ring of k_forward, a value written per (unit, node) instead of
@@ -194,13 +196,13 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
           re = fmaf(I, cs, re);
           im = fmaf(-I, sn, im);
         };
-#pragma unroll 1
-        for (int j0 = 0; j0 < kSpan; j0 += kNodeRun) {
-          if (rows == (1u << R) - 1) {
+        if (rows == (1u << R) - 1) {
+          for (int j0 = 0; j0 < kSpan; j0 += kFwdRun) {
             float re[R], im[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) re[r] = im[r] = 0.f;
-            for (int j = j0; j < j0 + kNodeRun; j += 2) {
+#pragma unroll 4
+            for (int j = j0; j < j0 + kFwdRun; j += 2) {
               const double4 q0 = tp[j], q1 = tp[j + 1];
               const float I0 = sky_of(q0), I1 = -sky_of(q1);
 #pragma unroll
@@ -211,13 +213,15 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
             }
 #pragma unroll
             for (int r = 0; r < R; ++r) t_re[r] += re[r], t_im[r] += im[r];
-          } else {
+          }
+        } else {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-              if (!((rows >> r) & 1u)) continue;
+          for (int r = 0; r < R; ++r) {
+            if (!((rows >> r) & 1u)) continue;
+            for (int j0 = 0; j0 < kSpan; j0 += kFwdRun) {
               float re = 0.f, im = 0.f;
 #pragma unroll 4
-              for (int j = j0; j < j0 + kNodeRun; j += 2) {
+              for (int j = j0; j < j0 + kFwdRun; j += 2) {
                 const double4 q0 = tp[j], q1 = tp[j + 1];
                 term(r, q0, sky_of(q0), kTurn32, re, im);
                 term(r, q1, -sky_of(q1), kTurn32 + 0.5, re, im);
