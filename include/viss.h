@@ -132,10 +132,12 @@ int viss_plan_set_samples(viss_plan *plan, int64_t K, const double *uvw, const d
  * VISS_FP64 selects the plain FP64 path.  From 1e10 sample x pixel terms on,
  * samples that lie on smooth tracks (the baselines of a formation) go through
  * track blocks: most exponentials interpolated from a few samples per block, to
- * the same accuracy.  The first split call after the samples or pixels were
- * staged builds them (a few waits for the device, 1-3 ms) and every call then
- * uses device buffers of the plan, about 1 GiB and 1 KiB per sample; without
- * that memory, under stream capture, and for other samples every term is
+ * the same accuracy, where that is modelled faster.  The first split calls after
+ * the samples or pixels were staged look at them and build the blocks (a few
+ * waits for the device, 1 to 4 ms in all), and calls through blocks use device
+ * buffers of the plan: about 1/4 GiB, 1/4 KiB per sample, 1.5e-4 bytes per term and,
+ * above 4 million pixels, 64 bytes per pixel.  Without that memory, under stream
+ * capture, and for other samples every term is
  * evaluated.  The two ways agree to their accuracy, not bit by bit:
  * VISS_ALL_TERMS asks for the second, with the same bits as a captured call.
  * Asynchronous: VISS_OK means the work was launched.  A bounded device-side wait

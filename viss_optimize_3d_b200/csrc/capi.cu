@@ -188,6 +188,7 @@ struct viss_plan {
   long long gridded_facet = 0;
   long long gridded_hbm_blocks = 0;
   long long geom_version = 0;   // bumped by every call that restages pixels or samples
+  long long pix_version = 0;    // by those that restage pixels
   // track blocks (tracks.cu) of the staged samples, and of the formation's pairs as
   // samples u = U_a - U_b; form_version as geom_version
   struct Blocks {
@@ -198,8 +199,6 @@ struct viss_plan {
   long long form_version = 0;
   double form_turns = 0;        // bound on |U.s| and |off|
   float4 *skies = nullptr;      size_t skies_cap = 0;   // viss_forward_skies
-  double4 *form_samp = nullptr; size_t form_samp_cap = 0;
-  int4 *form_refs = nullptr;    size_t form_refs_cap = 0;
 };
 
 namespace {
@@ -431,7 +430,7 @@ int viss_plan_destroy(viss_plan *p) {
   void *bufs[] = {p->pix,    p->pixsky,  p->cones,    p->perm,      p->samp,
                   p->refs,   p->occ,     p->occ32,    p->coef,      p->part,
                   p->dev_words, p->form_U, p->form_off, p->form_occ, p->form_occ32,
-                  p->form_coef, p->form_samp, p->form_refs, p->skies};
+                  p->form_coef, p->skies};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->gridded) viss::gridded_free(p->gridded);
@@ -442,7 +441,7 @@ int viss_plan_destroy(viss_plan *p) {
 }
 
 int viss_plan_set_pixels(viss_plan *p, int64_t J, const double *lmn, void *stream) {
-  if (p) ++p->geom_version, ++p->form_version;
+  if (p) ++p->geom_version, ++p->form_version, ++p->pix_version;
   if (!p || J <= 0 || !lmn) return fail(VISS_ERR_ARG, "viss_plan_set_pixels: bad arguments");
   if (J > (1LL << 31) * viss::kTilePix / 2)
     return fail(VISS_ERR_ARG, "viss_plan_set_pixels: too many pixels");
@@ -542,6 +541,9 @@ static viss::TrackInputs track_inputs(const viss_plan *p) {
   in.channels = p->channels;
   in.nsm = p->nsm;
   in.max_turns = p->max_turns;
+  in.pix_version = p->pix_version;
+  in.work = p->part;
+  in.work_bytes = p->part ? p->part_cap : 0;
   return in;
 }
 
@@ -572,8 +574,11 @@ static double direct_seconds(const viss_plan *p, bool masked, bool adjoint) {
 // call.  Of 1,172 calls measured (1e10 to 3e11 terms, plain and formation, occulted and
 // not) 879 took them, none of which is slower than term by term.
 constexpr double kTrackMargin = 0.95;
-// Fewer terms are not looked at: that takes 0.2 to 0.5 ms of a call's first pass on
-// newly staged samples, and the build 1 to 4.5 ms, more with a plan's first allocations.
+// Fewer terms are not looked at.  On newly staged samples looking takes 0.2 to 0.4 ms
+// and looking and building together 1.2 to 1.6 ms at 1e10 to 2e10 terms, 3.6 ms at 3e11
+// (Nside 256 x 388,800 samples); a plan's first allocations another 0.5 to 1 ms.  A 1e10
+// term forward on restaged samples (Nside 64, 2 MHz, occulted): 5.4 ms with the build, 3.8
+// once built, 5.4 term by term.
 constexpr double kTrackMinTerms = 1e10;
 constexpr double kTrackMinSeconds = 3e-3;          // likewise, of the formation kernels (1e10 terms: 2.7 to 4.6 ms)
 
@@ -999,11 +1004,12 @@ static viss::FormParams form_params(viss_plan *p, int flags) {
 static viss::TrackInputs form_track_inputs(const viss_plan *p) {
   viss::TrackInputs in = track_inputs(p);
   const long long B = viss::form_pairs(p->form_S);
-  in.samp = p->form_samp;
-  in.refs = (p->form_sat || p->form_snap) ? p->form_refs : nullptr;
+  in.K = p->form_T * B;
+  // the pairs' records, while they are looked at and built from, at the front of the workspace
+  in.samp = static_cast<const double4 *>(p->part);
+  in.refs = (p->form_sat || p->form_snap) ? reinterpret_cast<const int4 *>(in.samp + in.K) : nullptr;
   in.occ = p->form_occ;
   in.occ32 = p->form_occ32;
-  in.K = p->form_T * B;
   in.Kc = p->form_T / p->form_C * B;
   in.channels = p->form_C;
   in.max_turns = 3.0 * p->form_turns;              // |U_a.s| + |U_b.s| + |off|
@@ -1018,6 +1024,12 @@ constexpr double kFormSeconds[2][11] = {{0, 0, 24.0, 12.2, 7.5, 5.4, 6.3, 4.9, 4
                                         {0, 0, 18.9, 9.6, 6.4, 4.77, 3.91, 3.44, 3.12, 2.8, 2.65}};
 constexpr double kFormPart[2][2] = {{0.0, 1.7}, {0.06, 1.35}};
 
+// The workspace of a formation call, with room for its pairs' records.
+static int form_workspace(viss_plan *p, size_t bytes) {
+  const size_t K = static_cast<size_t>(p->form_T) * viss::form_pairs(p->form_S);
+  return workspace(p, std::max(bytes, (sizeof(double4) + sizeof(int4)) * K));
+}
+
 // Whether a formation call goes through track blocks of its pairs (u = U_a -
 // U_b, the same rows).
 static int form_tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint, cudaStream_t st, bool *use) {
@@ -1031,19 +1043,26 @@ static int form_tracks_ready(viss_plan *p, int flags, bool masked, bool adjoint,
     return 1e-13 * kFormSeconds[adjoint][p->form_S] * seen * static_cast<double>(K) * p->J;
   };
   if (other() < kTrackMinSeconds || !(3.0 * p->form_turns < 262144.0) || !tracks_allowed(flags, st)) return VISS_OK;
-  if (b.version != p->form_version) {
-    const bool rows = p->form_sat || p->form_snap;
-    if (ensure(p->form_samp, p->form_samp_cap, sizeof(double4) * K, "formation samples") ||
-        (rows && ensure(p->form_refs, p->form_refs_cap, sizeof(int4) * K, "formation samples")))
-      return VISS_OK;                              // without that memory: the formation kernels
-    VISS_CUDA(viss::launch_pair_samples(p->form_T, p->form_S, p->form_U, p->form_has_off ? p->form_off : nullptr,
-                                        p->form_sat, p->form_snap, p->form_samp, rows ? p->form_refs : nullptr, st),
-              "formation samples");
+  // where even the pairs of tiles seen in part cost more, whatever the nodes (the
+  // shares not counted yet: at Nside 64, as a rule)
+  if (masked && adjoint && b.version != p->form_version) {
+    double seen, mixed;
+    visible_shares(b, p->form_version, p->J, masked, &seen, &mixed);
+    if ((1.45e-12 * mixed + 3e-14) * static_cast<double>(K) * p->J >= kTrackMargin * other()) return VISS_OK;
   }
-  const viss::TrackInputs in = form_track_inputs(p);
-  if (int s = tracks_look(b, in, p->form_version, st)) return s;
-  if (!b.promising || viss::tracks_seconds(b.state, in, masked, adjoint) >= kTrackMargin * other()) return VISS_OK;
-  return tracks_built(b, in, st, use);
+  const bool rows = p->form_sat || p->form_snap;
+  auto pairs = [&]() {                             // into the workspace (form_workspace), that nothing uses yet
+    const viss::TrackInputs in = form_track_inputs(p);
+    return viss::launch_pair_samples(p->form_T, p->form_S, p->form_U, p->form_has_off ? p->form_off : nullptr, p->form_sat,
+                                     p->form_snap, const_cast<double4 *>(in.samp), const_cast<int4 *>(in.refs), st);
+  };
+  const bool fresh = b.version != p->form_version;
+  if (fresh) VISS_CUDA(pairs(), "formation samples");
+  if (int s = tracks_look(b, form_track_inputs(p), p->form_version, st)) return s;
+  if (!b.promising || viss::tracks_seconds(b.state, form_track_inputs(p), masked, adjoint) >= kTrackMargin * other())
+    return VISS_OK;
+  if (!b.built && !fresh) VISS_CUDA(pairs(), "formation samples");
+  return tracks_built(b, form_track_inputs(p), st, use);
 }
 
 int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, void *stream) {
@@ -1062,7 +1081,7 @@ int viss_forward_formation(viss_plan *p, const float *sky, float *V, int flags, 
   fp.tiles_per_chunk = static_cast<int>((p->ntiles + c - 1) / c);
   const int nchunk = (p->ntiles + fp.tiles_per_chunk - 1) / fp.tiles_per_chunk;
   fp.nchunk = nchunk;
-  if (int s = workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * T * B)) return s;
+  if (int s = form_workspace(p, sizeof(double2) * static_cast<size_t>(nchunk) * T * B)) return s;
   if (int s = ensure(p->pixsky, p->pixsky_cap, sizeof(double4) * p->Jpad * C, "pixel+sky records"))
     return s;
   VISS_CUDA(viss::launch_stage_sky(p->J, p->Jpad, p->pix, p->perm, sky, 1.0f, p->pixsky, C, p->dev_words, st),
@@ -1117,7 +1136,7 @@ int viss_adjoint_formation(viss_plan *p, const float *coef, float *image, float 
   long long spc = (Tc + c - 1) / c;
   spc = (spc + viss::kFormSnapTile - 1) / viss::kFormSnapTile * viss::kFormSnapTile;
   const int nchunk = static_cast<int>((Tc + spc - 1) / spc);
-  if (int s = workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * C * p->Jpad)) return s;
+  if (int s = form_workspace(p, sizeof(double) * static_cast<size_t>(nchunk) * C * p->Jpad)) return s;
   VISS_CUDA(cudaMemsetAsync(p->dev_words, 0, 3 * sizeof(unsigned long long), st), "viss_adjoint_formation");
   viss::FormParams fp = form_params(p, flags);
   bool use = false;

@@ -1288,6 +1288,25 @@ TrackNodeParams node_params(const TrackState &S, const TrackInputs &in, const Tr
 
 }  // namespace
 
+namespace {
+
+// A call's sums: in the caller's workspace if they fit, else in the blocks' own (at:
+// null without memory).
+struct TrackCut {
+  char *at;
+  template <class T>
+  void take(T *&p, size_t n) {
+    p = reinterpret_cast<T *>(at);
+    at += TrackArena::bytes<T>(n);
+  }
+};
+TrackCut call_sums(TrackState &S, const TrackInputs &in, size_t bytes) {
+  if (in.work && bytes <= in.work_bytes) return {static_cast<char *>(in.work)};
+  return {S.call.reset(bytes) ? S.call.base : nullptr};
+}
+
+}  // namespace
+
 int tracks_forward(void *state, const TrackInputs &in, const double4 *pixsky, float2 *V, bool masked,
                    bool use_off, bool accumulate, unsigned long long *counter, int *err, int drop_tile,
                    cudaStream_t st) {
@@ -1301,10 +1320,11 @@ int tracks_forward(void *state, const TrackInputs &in, const double4 *pixsky, fl
   const int per = ((in.ntiles + y - 1) / y + 31) / 32 * 32;
   const int nrest = S.has_rest[masked] ? static_cast<int>(blks(in.ntiles, per)) : 0;
   double2 *vacc_d, *rest_d;
-  if (!S.fwd.reset(TrackArena::bytes<double2>(vacc) + TrackArena::bytes<double2>(static_cast<size_t>(nrest) * S.Ks)))
-    return record_error(-3, "viss_forward: device allocation failed (track block sums)");
-  S.fwd.take(vacc_d, vacc);
-  S.fwd.take(rest_d, static_cast<size_t>(nrest) * S.Ks);
+  TrackCut sums = call_sums(S, in, TrackArena::bytes<double2>(vacc) +
+                                       TrackArena::bytes<double2>(static_cast<size_t>(nrest) * S.Ks));
+  if (!sums.at) return record_error(-3, "viss_forward: device allocation failed (track block sums)");
+  sums.take(vacc_d, vacc);
+  sums.take(rest_d, static_cast<size_t>(nrest) * S.Ks);
   if (nrest) {
     TrackRestParams rp = rest_params(S, in, masked, use_off, counter);
     rp.pix = pixsky;
@@ -1372,11 +1392,12 @@ int tracks_adjoint(void *state, const TrackInputs &in, const float2 *coef, float
   const size_t nodes = static_cast<size_t>(ny) * in.Jpad, rests = static_cast<size_t>(nrest) * in.channels * in.Jpad;
   float2 *coef_d;
   double *node_d, *rest_d;
-  if (!S.adj.reset(TrackArena::bytes<float2>(S.Ks) + TrackArena::bytes<double>(nodes) + TrackArena::bytes<double>(rests)))
-    return record_error(-3, "viss_adjoint: device allocation failed (track block sums)");
-  S.adj.take(coef_d, S.Ks);
-  S.adj.take(node_d, nodes);
-  S.adj.take(rest_d, rests);
+  TrackCut sums = call_sums(S, in, TrackArena::bytes<float2>(S.Ks) + TrackArena::bytes<double>(nodes) +
+                                       TrackArena::bytes<double>(rests));
+  if (!sums.at) return record_error(-3, "viss_adjoint: device allocation failed (track block sums)");
+  sums.take(coef_d, S.Ks);
+  sums.take(node_d, nodes);
+  sums.take(rest_d, rests);
   k_track_coef<<<blks(S.Ks, 256), 256, 0, st>>>(S.Ks, S.slot, coef, coef_d);
   TRACK_CUDA(cudaGetLastError(), "coefficients");
   if (nrest) {

@@ -21,6 +21,9 @@ struct TrackInputs {
   int channels;
   int nsm;
   double max_turns;        // bound on |u.s + off|
+  long long pix_version;   // another one for newly staged pixels
+  void *work;              // a call's sums go there if they fit
+  size_t work_bytes;
 };
 
 // Looks at a few blocks of the staged samples (*state: allocated on first use,

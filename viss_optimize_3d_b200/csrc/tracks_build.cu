@@ -110,16 +110,20 @@ __global__ void k_track_slots(TrackShape s, long long Ks, const int *order, cons
 // comment): thread = sample; column j of the factor at L[j * kTrackT + k].
 // Returns the rank (0: not worth it), the pivots in piv and the pivots'
 // diagonal entries in ld.
+// RM: ranks up to it; 48 leave room for twice the CTAs per SM.
+template <int RM>
 struct TrackFactor {
-  double L[kTrackRankMax * kTrackT];
+  double L[RM * kTrackT];
   double u[3][kTrackT];
-  double ld[kTrackRankMax], diag[kTrackT];
+  double ld[RM], diag[kTrackT];
   unsigned long long best[kTrackT / 32];
   double sum[kTrackT / 32], top[kTrackT / 32];
-  unsigned char piv[kTrackRankMax];
+  unsigned char piv[RM];
 };
+constexpr int kSmallRank = kTrackRankMax / 2;
 
-__device__ int track_factor(TrackFactor &f, bool valid, const double4 &u, double rho, int rank_max) {
+template <int RM>
+__device__ int track_factor(TrackFactor<RM> &f, bool valid, const double4 &u, double rho, int rank_max) {
   const int k = threadIdx.x, lane = k & 31, w = k >> 5;
   f.u[0][k] = u.x;
   f.u[1][k] = u.y;
@@ -173,10 +177,11 @@ __device__ int track_factor(TrackFactor &f, bool valid, const double4 &u, double
 
 // Ranks of natural blocks (which: of all, if null) for group radius rho[blockIdx.y]
 // and at most most[blockIdx.y] nodes, as rank[blockIdx.y][block] (0: more).
+template <int RM>
 __global__ void __launch_bounds__(kTrackT) k_track_ranks(TrackShape s, const int *which, const double4 *samp,
                                                          RadiusSet radii, int *rank) {
   extern __shared__ __align__(128) unsigned char smem[];
-  TrackFactor &f = *reinterpret_cast<TrackFactor *>(smem);
+  TrackFactor<RM> &f = *reinterpret_cast<TrackFactor<RM> *>(smem);
   const int b = which ? which[blockIdx.x] : static_cast<int>(blockIdx.x);
   const long long k = block_sample(s, b, threadIdx.x);
   const double4 u = k >= 0 ? samp[k] : make_double4(0, 0, 0, 0);
@@ -187,18 +192,19 @@ __global__ void __launch_bounds__(kTrackT) k_track_ranks(TrackShape s, const int
 // Nodes and weights of every block: node n of block b is record noff[b] + n,
 // its weights for the block's 128 slots P[(noff[b] + n) * 128 + k].  The factorisation
 // is k_track_ranks's; should it ever end at another rank, *differ says so and the
-// blocks are not used.
-__global__ void __launch_bounds__(kTrackT) k_track_weights(const int *slot, const double4 *samp_s, RadiusSet radii,
+// blocks are not used.  Blocks of ranks in (above, RM].
+template <int RM>
+__global__ void __launch_bounds__(kTrackT) k_track_weights(int above, const int *slot, const double4 *samp_s, RadiusSet radii,
                                                            const int *cls, const int *rank, const int *noff, double4 *node,
                                                            int *nodeblk, float *P, unsigned long long *differ) {
   extern __shared__ __align__(128) unsigned char smem[];
-  TrackFactor &f = *reinterpret_cast<TrackFactor *>(smem);
+  TrackFactor<RM> &f = *reinterpret_cast<TrackFactor<RM> *>(smem);
   const int b = blockIdx.x, k = threadIdx.x;
-  if (rank[b] == 0) return;
+  if (rank[b] <= above || rank[b] > RM) return;
   const long long i = static_cast<long long>(b) * kTrackT + k;
   const double4 u = samp_s[i];
   const bool valid = slot[i] >= 0;
-  const int r = track_factor(f, valid, u, radii.rho[cls[b]], radii.most[cls[b]]);
+  const int r = track_factor(f, valid, u, radii.rho[cls[b]], min(radii.most[cls[b]], RM));
   if (r != rank[b]) {
     if (k == 0) atomicOr(differ, 1ull);
     return;
@@ -211,7 +217,7 @@ __global__ void __launch_bounds__(kTrackT) k_track_weights(const int *slot, cons
   }
   // x L11 = l_k from the last column back, L11[j][q] = L[q][piv j] (q < j), ld[j] on
   // the diagonal.  The pivots' rows are read by all, so x goes to registers first.
-  double x[kTrackRankMax];
+  double x[RM];
 #pragma unroll 1
   for (int j = r - 1; j >= 0; --j) {
     double v = f.L[j * kTrackT + k];
@@ -499,6 +505,52 @@ double block_slots(int c, int r, int len) {
 
 namespace {
 
+// Pixel groups of newly staged pixels: centres, radii and the radii to try, kept until
+// pixels are staged again.  S.pix_version stays behind if memory is short.
+int track_pixels(TrackState &S, const TrackInputs &in, cudaStream_t st) {
+  if (S.pix_version == in.pix_version) return 0;
+  S.pix_version = -1;
+  int ngs[kClasses], total = 0;
+  for (int c = 0; c < kClasses; ++c) {
+    ngs[c] = static_cast<int>((in.Jpad + group_pix(c) - 1) / group_pix(c));
+    S.gat[c] = total;
+    total += ngs[c];
+  }
+  if (!S.pixels.reset(TrackArena::bytes<double4>(total) + TrackArena::bytes<float>(total))) return 0;
+  S.pixels.take(S.gcen, total);
+  S.pixels.take(S.radius, total);
+  for (int c = 0; c < kClasses; ++c) {
+    k_track_groups<<<blks(ngs[c], 8), 256, 0, st>>>(ngs[c], group_pix(c), in.Jpad, in.pix, S.gcen + S.gat[c],
+                                                    S.radius + S.gat[c]);
+    TRACK_CUDA(cudaGetLastError(), "groups");
+  }
+  std::vector<float> radius(total);
+  TRACK_CUDA(cudaMemcpyAsync(radius.data(), S.radius, sizeof(float) * total, cudaMemcpyDeviceToHost, st), "radii");
+  TRACK_CUDA(cudaStreamSynchronize(st), "groups");
+  // A class's radius: a percentile of its groups' (wider groups are left) with
+  // the least time over some blocks.  On a power-of-two HEALPix grid all groups
+  // are alike and the largest wins; elsewhere a few are far wider than the rest.
+  // A group of more than 64 pixels is only worth it with few nodes.  A share that
+  // takes in a group that has none (radius +inf) is no radius: nothing within it.
+  const double share[kShares] = {1.0, 0.99, 0.97, 0.9};
+  RadiusSet &trial = S.shares;
+  for (int c = 0; c < kClasses; ++c) {
+    auto b = radius.begin() + S.gat[c], e = b + ngs[c];
+    for (int q = 0; q < kShares; ++q) {
+      const int i = std::min(ngs[c] - 1, static_cast<int>(share[q] * ngs[c])), at = c * kShares + q;
+      std::nth_element(b, b + i, e);
+      S.within[at] = 0;
+      if (!std::isfinite(b[i])) continue;            // at most 0 nodes: every block's rank is 0
+      trial.rho[at] = b[i] * (1.0 + 1e-6);
+      trial.most[at] = c == kHalf ? kTrackRankMax : kSmallRank;
+      S.within[at] = std::count_if(b, e, [&](float v) { return v <= static_cast<float>(trial.rho[at]); }) /
+                   static_cast<double>(ngs[c]);
+    }
+  }
+  S.pix_version = in.pix_version;
+  return 0;
+}
+
 // n natural blocks to look at, spread evenly over tracks and time together (the R2
 // sequence, M. Roberts 2018: multiples of 1/g and 1/g^2, g^3 = g + 1) and the
 // channels in turn: a baseline's length decides its ranks, and 48 blocks picked at
@@ -525,30 +577,24 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
   if (in.K > INT_MAX / 2 || in.ntiles < 8 || in.ntiles > INT_MAX / 16) return 0;
   const int lags = static_cast<int>(std::min<long long>(kLagMax, in.Kc / 32));
   if (lags < 1) return 0;
-  TRACK_CUDA(cudaFuncSetAttribute(k_track_ranks, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(sizeof(TrackFactor))), "attributes");
-  TRACK_CUDA(cudaFuncSetAttribute(k_track_weights, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(sizeof(TrackFactor))), "attributes");
-  // pixel groups of each class, and how far samples a lag apart are
-  int ngs[kClasses], total = 0;
-  for (int c = 0; c < kClasses; ++c) {
-    ngs[c] = static_cast<int>((in.Jpad + group_pix(c) - 1) / group_pix(c));
-    S.gat[c] = total;
-    total += ngs[c];
-  }
-  float *radius_d, *score_d;
+  TRACK_CUDA(cudaFuncSetAttribute(k_track_ranks<kTrackRankMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(TrackFactor<kTrackRankMax>))), "attributes");
+  TRACK_CUDA(cudaFuncSetAttribute(k_track_ranks<kSmallRank>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(TrackFactor<kSmallRank>))), "attributes");
+  if (int s = track_pixels(S, in, st)) return s;
+  if (S.pix_version != in.pix_version) return 0;   // no memory
+  // how far samples a lag apart are
+  float *score_d;
   int *trial_rank_d, *order_d, *cls_d, *slot_d;
   double4 *samp_d;
   int4 *refs_d;
   unsigned long long *sums_d;
   const size_t slots = static_cast<size_t>(kRankSamples) * kTrackT, crows = static_cast<size_t>(kClasses + 1) * ((in.ntiles + 31) / 32);
-  if (!S.trial.reset(TrackArena::bytes<double4>(total) + TrackArena::bytes<float>(total) + TrackArena::bytes<float>(lags) +
+  if (!S.trial.reset(TrackArena::bytes<float>(lags) +
                      TrackArena::bytes<int>(kRadii * kRankSamples) + 2 * TrackArena::bytes<int>(2 * kRankSamples) +
                      TrackArena::bytes<int>(slots) + TrackArena::bytes<double4>(slots) + TrackArena::bytes<int4>(slots) +
                      3 * TrackArena::bytes<unsigned>(crows) + TrackArena::bytes<unsigned long long>(1 + 2 * kEstimates)))
     return 0;
-  S.trial.take(S.gcen, total);
-  S.trial.take(radius_d, total);
   S.trial.take(score_d, lags);
   S.trial.take(trial_rank_d, kRadii * kRankSamples);
   S.trial.take(order_d, 2 * kRankSamples);
@@ -558,18 +604,12 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
   S.trial.take(refs_d, slots);
   for (auto &row : S.crow) S.trial.take(row, crows);
   S.trial.take(sums_d, 1 + 2 * kEstimates);        // classes that leave tiles, unocculted, occulted
-  for (int c = 0; c < kClasses; ++c) {
-    k_track_groups<<<blks(ngs[c], 8), 256, 0, st>>>(ngs[c], group_pix(c), in.Jpad, in.pix, S.gcen + S.gat[c],
-                                                    radius_d + S.gat[c]);
-    TRACK_CUDA(cudaGetLastError(), "groups");
-  }
   const double rho_lag = 2.0 / std::sqrt(static_cast<double>(in.ntiles));   // about one tile's radius
   k_track_lags<<<lags, kLagSamples, 0, st>>>(in.Kc, in.channels, in.samp, rho_lag, score_d);
   TRACK_CUDA(cudaGetLastError(), "lags");
-  std::vector<float> radius(total), score(lags);
+  std::vector<float> score(lags);
   TRACK_CUDA(cudaMemcpyAsync(score.data(), score_d, sizeof(float) * lags, cudaMemcpyDeviceToHost, st), "lags");
-  TRACK_CUDA(cudaMemcpyAsync(radius.data(), radius_d, sizeof(float) * total, cudaMemcpyDeviceToHost, st), "radii");
-  TRACK_CUDA(cudaStreamSynchronize(st), "groups");
+  TRACK_CUDA(cudaStreamSynchronize(st), "lags");
   // the tracks: the shortest lag whose samples lie about as close as any lag's
   const float best = *std::min_element(score.begin(), score.end());
   if (!(best < 1.0f)) return 0;                    // neighbours a turn apart: nothing to interpolate
@@ -586,27 +626,8 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
   const int nb = static_cast<int>(nbl);
   S.W = (in.ntiles + 31) / 32;
   if (static_cast<double>(nb) * S.W > INT_MAX) return 0;
-  // A class's radius: a percentile of its groups' (wider groups are left) with
-  // the least time over some blocks.  On a power-of-two HEALPix grid all groups
-  // are alike and the largest wins; elsewhere a few are far wider than the rest.
-  // A group of more than 64 pixels is only worth it with few nodes.  A share that
-  // takes in a group that has none (radius +inf) is no radius: nothing within it.
-  const double share[kShares] = {1.0, 0.99, 0.97, 0.9};
-  RadiusSet trial{};
-  double within[kRadii];
-  for (int c = 0; c < kClasses; ++c) {
-    auto b = radius.begin() + S.gat[c], e = b + ngs[c];
-    for (int q = 0; q < kShares; ++q) {
-      const int i = std::min(ngs[c] - 1, static_cast<int>(share[q] * ngs[c])), at = c * kShares + q;
-      std::nth_element(b, b + i, e);
-      within[at] = 0;
-      if (!std::isfinite(b[i])) continue;            // at most 0 nodes: every block's rank is 0
-      trial.rho[at] = b[i] * (1.0 + 1e-6);
-      trial.most[at] = c == kHalf ? kTrackRankMax : kTrackRankMax / 2;
-      within[at] = std::count_if(b, e, [&](float v) { return v <= static_cast<float>(trial.rho[at]); }) /
-                   static_cast<double>(ngs[c]);
-    }
-  }
+  const RadiusSet &trial = S.shares;
+  const double *within = S.within;
   const int nsamp = std::min(nb, kRankSamples);
   const std::vector<int> order = spread_blocks(sh, nb, nsamp);
   TRACK_CUDA(cudaMemcpyAsync(order_d, order.data(), sizeof(int) * nsamp, cudaMemcpyHostToDevice, st), "order");
@@ -618,7 +639,12 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
   auto ranks_of = [&](int first, int n) -> cudaError_t {
     RadiusSet some{};
     for (int q = 0; q < n; ++q) some.rho[q] = trial.rho[first + q], some.most[q] = trial.most[first + q];
-    k_track_ranks<<<dim3(nsamp, n), kTrackT, sizeof(TrackFactor), st>>>(sh, order_d, in.samp, some, trial_rank_d);
+    if (first == kHalf)
+      k_track_ranks<kTrackRankMax><<<dim3(nsamp, n), kTrackT, sizeof(TrackFactor<kTrackRankMax>), st>>>(
+          sh, order_d, in.samp, some, trial_rank_d);
+    else
+      k_track_ranks<kSmallRank><<<dim3(nsamp, n), kTrackT, sizeof(TrackFactor<kSmallRank>), st>>>(
+          sh, order_d, in.samp, some, trial_rank_d);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = cudaMemcpyAsync(rk.data() + static_cast<size_t>(first) * nsamp, trial_rank_d, sizeof(int) * n * nsamp,
@@ -666,7 +692,7 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
   // those blocks' share of a call's work
   TRACK_CUDA(cudaMemcpyAsync(cls_d, least_cls.data(), sizeof(int) * 2 * nsamp, cudaMemcpyHostToDevice, st), "classes");
   TRACK_CUDA(cudaMemsetAsync(sums_d, 0, (1 + 2 * kEstimates) * sizeof(unsigned long long), st), "sums");
-  k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, radius_d, cs, S.crow[0],
+  k_track_class_rows<<<dim3(blks(S.W, 128), kClasses + 1), 128, 0, st>>>(S.W, in.ntiles, S.radius, cs, S.crow[0],
                                                                          S.crow[1], S.crow[2], sums_d);
   TRACK_CUDA(cudaGetLastError(), "class rows");
   k_track_slots<<<blks(nsamp * kTrackT, 256), 256, 0, st>>>(sh, nsamp * kTrackT, order_d, in.samp, in.refs, slot_d,
@@ -724,8 +750,15 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
   int *all_ranks_d;
   if (!S.masks.reset(TrackArena::bytes<int>(static_cast<size_t>(nclass) * nb))) return 0;
   S.masks.take(all_ranks_d, static_cast<size_t>(nclass) * nb);
-  k_track_ranks<<<dim3(nb, nclass), kTrackT, sizeof(TrackFactor), st>>>(sh, nullptr, in.samp, some, all_ranks_d);
+  k_track_ranks<kTrackRankMax><<<nb, kTrackT, sizeof(TrackFactor<kTrackRankMax>), st>>>(sh, nullptr, in.samp, some,
+                                                                                     all_ranks_d);
   TRACK_CUDA(cudaGetLastError(), "ranks");
+  if (nclass > 1) {                                // the first is kHalf
+    for (int i = 0; i + 1 < nclass; ++i) some.rho[i] = some.rho[i + 1], some.most[i] = some.most[i + 1];
+    k_track_ranks<kSmallRank><<<dim3(nb, nclass - 1), kTrackT, sizeof(TrackFactor<kSmallRank>), st>>>(
+        sh, nullptr, in.samp, some, all_ranks_d + nb);
+    TRACK_CUDA(cudaGetLastError(), "ranks");
+  }
   std::vector<int> rk(static_cast<size_t>(nclass) * nb);
   TRACK_CUDA(cudaMemcpyAsync(rk.data(), all_ranks_d, sizeof(int) * rk.size(), cudaMemcpyDeviceToHost, st), "ranks");
   TRACK_CUDA(cudaStreamSynchronize(st), "ranks");
@@ -775,12 +808,15 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
   if (n == 0) return 0;
   const size_t nodes = (n + 31) / 32 * 32, rows = masked ? pairs : 0;
   const size_t sums = static_cast<size_t>(in.ntiles) * S.ld_max;
-  if (!S.plan.reset(TrackArena::bytes<int>(S.Ks) + 4 * TrackArena::bytes<int>(nb) + TrackArena::bytes<int>(nodes) +
+  // four sample masks per (block, word) are more than most observations need
+  const size_t room = 4 * rows;
+  if (!S.plan.reset(TrackArena::bytes<uint4>(room) + TrackArena::bytes<int>(S.Ks) + 4 * TrackArena::bytes<int>(nb) + TrackArena::bytes<int>(nodes) +
                     TrackArena::bytes<double4>(S.Ks) + TrackArena::bytes<double4>(nodes) +
                     TrackArena::bytes<int4>(masked ? S.Ks : 0) + TrackArena::bytes<float>(nodes * kTrackT) +
                     4 * TrackArena::bytes<unsigned>(rows) + TrackArena::bytes<int>(rows) +
                     TrackArena::bytes<float2>(sums) + TrackArena::bytes<unsigned long long>(4)))
     return 0;
+  S.plan.take(S.mask, room);
   S.plan.take(S.slot, S.Ks);
   for (int **p : {&S.order, &S.cls, &S.rank, &S.noff}) S.plan.take(*p, nb);
   S.plan.take(S.nodeblk, nodes);
@@ -805,9 +841,18 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
   TRACK_CUDA(cudaMemsetAsync(S.node, 0, sizeof(double4) * nodes, st), "nodes");
   TRACK_CUDA(cudaMemsetAsync(S.nodeblk, 0xff, sizeof(int) * nodes, st), "nodes");
   TRACK_CUDA(cudaMemsetAsync(counts_d, 0, 4 * sizeof(unsigned long long), st), "counts");
-  k_track_weights<<<nb, kTrackT, sizeof(TrackFactor), st>>>(S.slot, S.samp, S.radii, S.cls, S.rank, S.noff, S.node,
-                                                           S.nodeblk, S.P, counts_d + 2);
+  TRACK_CUDA(cudaFuncSetAttribute(k_track_weights<kTrackRankMax>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(TrackFactor<kTrackRankMax>))), "attributes");
+  TRACK_CUDA(cudaFuncSetAttribute(k_track_weights<kSmallRank>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(sizeof(TrackFactor<kSmallRank>))), "attributes");
+  k_track_weights<kSmallRank><<<nb, kTrackT, sizeof(TrackFactor<kSmallRank>), st>>>(
+      0, S.slot, S.samp, S.radii, S.cls, S.rank, S.noff, S.node, S.nodeblk, S.P, counts_d + 2);
   TRACK_CUDA(cudaGetLastError(), "weights");
+  if (*std::max_element(rank.begin(), rank.end()) > kSmallRank) {
+    k_track_weights<kTrackRankMax><<<nb, kTrackT, sizeof(TrackFactor<kTrackRankMax>), st>>>(
+        kSmallRank, S.slot, S.samp, S.radii, S.cls, S.rank, S.noff, S.node, S.nodeblk, S.P, counts_d + 2);
+    TRACK_CUDA(cudaGetLastError(), "weights");
+  }
   const unsigned by = static_cast<unsigned>(std::max(1, std::min(S.W / 8, (4 * in.nsm * 8) / nb + 1)));
   if (masked) {
     k_track_bits<<<dim3(nb, by), 128, 0, st>>>(S.W, in.ntiles, S.slot, S.refs, in.occ32, in.cones, S.cls, S.crow[0],
@@ -819,8 +864,11 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
   TRACK_CUDA(cudaStreamSynchronize(st), "build");
   if (pairs_of[2]) return 0;
   if (masked) {
-    if (pairs_of[1] > INT_MAX || !S.masks.reset(TrackArena::bytes<uint4>(pairs_of[1]))) return 0;
-    S.masks.take(S.mask, pairs_of[1]);
+    if (pairs_of[1] > INT_MAX) return 0;
+    if (pairs_of[1] > room) {
+      if (!S.masks.reset(TrackArena::bytes<uint4>(pairs_of[1]))) return 0;
+      S.masks.take(S.mask, pairs_of[1]);
+    }
     k_track_masks<<<dim3(nb, by), 128, 0, st>>>(S.W, S.slot, S.refs, in.occ32, in.cones, S.brow[1], S.mask_at, S.mask,
                                                 counts_d + 3);
     TRACK_CUDA(cudaGetLastError(), "sample masks");

@@ -96,7 +96,11 @@ struct ClassSet {
 };
 
 struct TrackState {
-  TrackArena trial, plan, masks, fwd, adj;
+  TrackArena pixels, trial, plan, masks, call;
+  long long pix_version = -1;              // of the pixels that `pixels` and `shares` are of
+  RadiusSet shares{};                      // radii to try, and the share of groups within each
+  double within[kRadii] = {};
+  float *radius = nullptr;                 // groups', class after class from gat[c]
   TrackEstimate est[2];                    // unocculted, occulted
   double slab_count = 0;                   // slabs, but for those that a class of one rank is cut into by memory
   unsigned long long class_rest = 0;       // bit c: class c leaves tiles
