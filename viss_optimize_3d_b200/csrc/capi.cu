@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <string>
 
 #include "viss.h"
@@ -594,18 +595,28 @@ static bool tracks_allowed(int flags, cudaStream_t st) {
   return cap == cudaStreamCaptureStatusNone;
 }
 
-// Looks at newly staged samples; b.promising says what came of it.
+// Looks at newly staged samples; b.promising says what came of it.  Host memory that
+// runs out (std::bad_alloc of the lists kept meanwhile) leaves it without blocks, as
+// device memory does.
 static int tracks_look(viss_plan::Blocks &b, const viss::TrackInputs &in, long long version, cudaStream_t st) {
   if (b.version == version) return VISS_OK;
   b.promising = b.built = b.usable = false;
-  if (int s = viss::tracks_try(&b.state, in, st, &b.promising)) return s;
+  try {
+    if (int s = viss::tracks_try(&b.state, in, st, &b.promising)) return s;
+  } catch (const std::bad_alloc &) {
+    b.promising = false;
+  }
   b.version = version;
   return VISS_OK;
 }
 
 static int tracks_built(viss_plan::Blocks &b, const viss::TrackInputs &in, cudaStream_t st, bool *use) {
   if (!b.built) {
-    if (int s = viss::tracks_build(b.state, in, st, &b.usable)) return s;
+    try {
+      if (int s = viss::tracks_build(b.state, in, st, &b.usable)) return s;
+    } catch (const std::bad_alloc &) {
+      b.usable = false;
+    }
     b.built = true;
   }
   *use = b.usable;
