@@ -111,6 +111,7 @@ def launched_kernels(step):
     for e in prof.key_averages():
         if "viss::" in e.key:
             name = re.sub(r"^void |viss::|\(anonymous namespace\)::|\(viss.*$|\((long|int|double|float|unsigned).*$", "", e.key)
+            name = name.replace("<true>", "<1>").replace("<false>", "<0>")     # as ncu prints them
             found[name] = (e.count, e.device_time_total)
     return found
 
@@ -156,7 +157,7 @@ def record_traffic(csv_path: str, workload: str, command: str, commit: str = "")
             continue
         unit = row.get("Metric Unit", "byte")
         scale = {"byte": 1, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "KB": 1e3, "MB": 1e6, "GB": 1e9}.get(unit, 1)
-        m = re.search(r"\b((?:k_form_forward|k_form_adjoint|k_forward|k_adjoint)<[^>]*>)", name)
+        m = re.search(r"\b((?:k_form_forward|k_form_adjoint|k_forward|k_adjoint|k_track_\w+)<[^>]*>)", name)
         if m:
             k = m.group(1)     # the template instance, e.g. k_adjoint<128, 8, 4, 1, 0, 0>
             per.setdefault(k, {}).setdefault(row.get("ID"), 0.0)
@@ -309,11 +310,13 @@ def run_ours(args, rank, world, local_rank):
         g.plan.set_shapes(0, 0)
         shapes = (0, 0)
     else:
-        # launch-shape sweep (recorded) and the plan's own tuner (chooses)
+        # launch-shape sweep of the direct kernels (every term evaluated; recorded) and
+        # the plan's own tuner (chooses)
         for shape in range(4):
             g.plan.set_shapes(shape, shape)
-            for key, fn in (("forward_ms", lambda: g.plan.forward(g.sky)),
-                            ("adjoint_ms", lambda: g.plan.adjoint(coef0, scale=2.0, mask=cfg.imaging_mask))):
+            for key, fn in (("forward_ms", lambda: g.plan.forward(g.sky, all_terms=True)),
+                            ("adjoint_ms", lambda: g.plan.adjoint(coef0, scale=2.0, mask=cfg.imaging_mask,
+                                                                  all_terms=True))):
                 fn()
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record(stream)
@@ -494,6 +497,7 @@ def run_ours(args, rank, world, local_rank):
     by_tracks = any(k.startswith("k_track_") for k in kernels)
     if by_tracks:    # most exponentials interpolated: the slowest kernel of the direction stands for it
         inst = dominant(kernels, "fwd" if dom == "forward" else "adj")
+        achieved = dom_eval / dom_s
     traffic, traffic_src = measured_traffic(args.workload, inst)
     res = {
         "metric": METRIC,
@@ -514,9 +518,10 @@ def run_ours(args, rank, world, local_rank):
                 "path": "pinned host sky/uvw/refs/satellite positions/Earth rows -> viss_occulters -> "
                         "viss_plan_set_samples -> viss_forward -> viss_dcf/viss_weights -> viss_adjoint "
                         "-> pinned host V/image"},
-        "roofline": {"bound": "sfu", "kernel": inst.split("<")[0] if by_tracks else f"k_{dom}",
-                     **({"note": "track blocks: frac counts every term, most of them interpolated (no "
-                                 "exponential); frac_of_evaluated the exponentials"} if by_tracks else {}),
+        "roofline": {"bound": "sfu", "kernel": f"track blocks, {dom}" if by_tracks else f"k_{dom}",
+                     **({"note": "track blocks: the exponentials that the whole call evaluates (most terms are "
+                                 "interpolated) over its whole time; traffic is of one launch of its longest kernel",
+                         "terms_rate": round(K * J / dom_s / 1e9, 2)} if by_tracks else {}),
                      "achieved": round(achieved / 1e9, 2), "peak": round(peak_terms / 1e9, 1),
                      "unit": "Gterms/s", "frac": round(achieved / peak_terms, 4),
                      "peak_source": f"8 terms/clk/SM x {nsm} SMs x sm_max_mhz ({pk_kind})",
@@ -535,7 +540,8 @@ def run_ours(args, rank, world, local_rank):
         "tuning": {"chosen": {"forward": shapes[0], "adjoint": shapes[1]},
                    "forward_shapes": "(samples/thread, CTAs/SM) = (4,2) (4,3) (2,3) (2,4)",
                    "adjoint_shapes": "(pixels/lane, CTAs/SM), 128-thread CTAs = (8,4) (8,5) (4,5) (4,6)",
-                   **({"track_blocks": "the calls go through track blocks, which have no launch shapes"}
+                   **({"track_blocks": "the timed calls go through track blocks, which have no launch shapes; the "
+                                       "times here are of the direct kernels (VISS_ALL_TERMS)"}
                       if by_tracks else {}),
                    **({"note": "fixed at the headline size's choice (no sweep at this size)"} if big else sweep)},
         "clocks": clk,
@@ -681,7 +687,7 @@ def run_formation(args, rank, world, local_rank):
     peak_terms = per_clk * nsm * pk["sm_max_mhz"] * 1e6
     dom_s = max(fwd_s, adj_s)
     dom_eval = ev_f if dom == "forward" else ev_a
-    achieved = K * J / dom_s
+    achieved = (dom_eval if by_tracks else K * J) / dom_s
     res = {
         "metric": METRIC,
         "value": round(terms_per_step * args.steps * world / total_s / 1e9, 3),
@@ -701,10 +707,11 @@ def run_formation(args, rank, world, local_rank):
                 "path": "pinned host sky/satellite positions/Earth rows -> U and viss_occulters on the "
                         "device -> viss_plan_set_formation -> viss_forward_formation -> "
                         "viss_dcf/viss_weights -> viss_adjoint_formation -> pinned host V/image"},
-        "roofline": {"bound": "sfu" if by_tracks else "fp32", "kernel": inst.split("<")[0],
+        "roofline": {"bound": "sfu" if by_tracks else "fp32",
+                     "kernel": f"track blocks, {dom}" if by_tracks else inst.split("<")[0],
                      "achieved": round(achieved / 1e9, 2), "peak": round(peak_terms / 1e9, 1),
                      "unit": "Gterms/s", "frac": round(achieved / peak_terms, 4),
-                     "peak_source": ("8 terms/clk/SM (track blocks)" if by_tracks else
+                     "peak_source": ("8 terms/clk/SM (the exponentials that track blocks evaluate)" if by_tracks else
                                      f"128 FP32 lanes/clk/SM / {FORM_FFMA_PER_TERM} FFMA per term")
                                     + f" x {nsm} SMs x sm_max_mhz ({pk_kind})",
                      "evaluated_frac": round(dom_eval / (K * J), 4),

@@ -97,3 +97,13 @@ def test_workloads_and_traffic_key(bench):
     assert {"visibility.cu", "formation.cu"} <= set(bench.TRAFFIC_KERNEL_SOURCES)
     a = bench.kernel_sources_sha()
     assert a == bench.kernel_sources_sha() and len(a) == 64
+
+
+def test_traffic_record_of_track_kernels(bench, tmp_path):
+    """Kernels of the track blocks enter the record under the names that the
+    profiler's are turned into."""
+    kern = "void viss::<unnamed>::k_track_adj_nodes<1>(viss::TrackNodeParams)"
+    rows = [(kern, "dram__bytes_read.sum", "Mbyte", "30"), (kern, "dram__bytes_write.sum", "Mbyte", "2")]
+    rec = bench.record_traffic(_csv(tmp_path, rows), "c3_10mhz", "ncu ...")
+    assert rec["bytes_per_launch"]["c3_10mhz"] == {"k_track_adj_nodes<1>": 32_000_000}
+    assert bench.measured_traffic("c3_10mhz", "k_track_adj_nodes<1>")[0] == 32_000_000
