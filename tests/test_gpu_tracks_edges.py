@@ -185,3 +185,78 @@ def test_occulted_calls_take_the_faster_way(cuda_device, nside, n_sat, n_snap, f
     got = plan.forward(sky)
     assert by_blocks(plan) == blocks
     close(got, plan.forward(sky, fp64=True))
+
+
+@pytest.mark.parametrize("nside,n_sat,n_snap,f_hz,moon,earth,channels", [
+    (64, 8, 7777, 2e6, True, True, 1),
+    (101, 7, 4099, 1e6, True, False, 1),
+    (64, 6, 5000, 1e6, False, False, 3),
+    (60, 10, 2300, 4e5, True, True, 3),
+])
+def test_compared_calls_do_go_through_blocks(cuda_device, nside, n_sat, n_snap, f_hz, moon, earth, channels):
+    """The observations that test_gpu_tracks.py compares with FP64, and their
+    satellite vectors."""
+    obs = observation(nside, n_sat, n_snap, f_hz, moon, earth)
+    refs, occ = tables(obs, cuda_device)
+    u = torch.as_tensor(obs.uvw(f_hz), device=cuda_device)
+    plan = api.Plan(api.pix2lmn(nside, "ring", device=cuda_device),
+                    torch.cat([u * (1 + 0.1 * c) for c in range(channels)]), None,
+                    None if refs is None else refs.repeat(channels, 1), occ, channels=channels)
+    sky = torch.ones(channels * plan.J, device=cuda_device)
+    coef = torch.ones(plan.K, dtype=torch.complex64, device=cuda_device)
+    for kw in (dict(), dict(mask=False)):
+        plan.forward(sky, **kw)
+        assert by_blocks(plan)
+        plan.adjoint(coef, **kw)
+        assert by_blocks(plan)
+        plan.forward(sky, all_terms=True, **kw)
+        assert not by_blocks(plan)
+
+
+@pytest.mark.parametrize("bright", [1, 30])
+def test_sky_of_a_few_bright_pixels(cuda_device, bright):
+    """Weights fitted to directions spread over a group hold for single ones."""
+    obs = observation(64, 8, 7777, 1e6, False, False)
+    plan = api.Plan(api.pix2lmn(64, "ring", device=cuda_device), torch.as_tensor(obs.uvw(1e6), device=cuda_device))
+    g = torch.Generator(device=cuda_device).manual_seed(bright)
+    for _ in range(4):
+        sky = torch.zeros(plan.J, device=cuda_device)
+        sky[torch.randint(plan.J, (bright,), generator=g, device=cuda_device)] = 2.0
+        got = plan.forward(sky)
+        assert by_blocks(plan)
+        close(got, plan.forward(sky, fp64=True))
+
+
+def test_values_that_are_not_finite(cuda_device):
+    """An infinite sky value or coefficient reaches what sees it and nothing else,
+    as term by term."""
+    obs = observation(64, 8, 7777, 1e6, True, False)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(api.pix2lmn(64, "ring", device=cuda_device), torch.as_tensor(obs.uvw(1e6), device=cuda_device),
+                    None, refs, occ)
+    for bad in (float("inf"), float("nan")):
+        sky, coef = inputs(plan, cuda_device)
+        sky[31000], coef[4000] = bad, bad
+        V, img = plan.forward(sky), plan.adjoint(coef)
+        assert by_blocks(plan)
+        for got, want in ((V, plan.forward(sky, all_terms=True)), (img, plan.adjoint(coef, all_terms=True))):
+            ok = torch.isfinite(want.abs())
+            assert 0 < int(ok.sum()) < len(ok) and torch.equal(torch.isfinite(got.abs()), ok)
+            close(got[ok], want[ok])
+
+
+def test_pixels_that_are_no_grid(cuda_device):
+    """Directions drawn at random, and the call's pixel groups with them."""
+    g = torch.Generator(device=cuda_device).manual_seed(9)
+    lmn = torch.nn.functional.normalize(torch.randn(50001, 3, generator=g, device=cuda_device, dtype=torch.float64), dim=1)
+    obs = observation(64, 8, 7777, 3e5, True, True)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(lmn, torch.as_tensor(obs.uvw(3e5), device=cuda_device), None, refs, occ)
+    sky, coef = inputs(plan, cuda_device)
+    for kw in (dict(), dict(mask=False)):
+        got = plan.forward(sky, **kw)
+        assert by_blocks(plan)
+        close(got, plan.forward(sky, fp64=True, **kw))
+        got = plan.adjoint(coef, **kw)
+        assert by_blocks(plan)
+        close(got, plan.adjoint(coef, fp64=True, **kw))
