@@ -6,7 +6,7 @@ import torch
 
 from viss_optimize_3d_b200 import _capi, api, synth
 
-from test_gpu_tracks import close, observation, tables
+from test_gpu_tracks import REL, close, observation, tables
 
 pytestmark = pytest.mark.gpu
 
@@ -260,3 +260,20 @@ def test_pixels_that_are_no_grid(cuda_device):
         got = plan.adjoint(coef, **kw)
         assert by_blocks(plan)
         close(got, plan.adjoint(coef, fp64=True, **kw))
+
+
+@pytest.mark.parametrize("size", [1e-40, 1e-37, 1e35])
+def test_sizes_near_the_ends_of_fp32(cuda_device, size):
+    """The smallest and largest skies and coefficients are as accurate as term by
+    term (1e-40 has 17 bits itself: the same inputs on both sides)."""
+    obs = observation(64, 8, 7777, 1e6, True, False)
+    refs, occ = tables(obs, cuda_device)
+    plan = api.Plan(api.pix2lmn(64, "ring", device=cuda_device), torch.as_tensor(obs.uvw(1e6), device=cuda_device),
+                    None, refs, occ)
+    sky, coef = inputs(plan, cuda_device)
+    rel = lambda a, b: float((a.to(torch.complex128) - b.to(torch.complex128)).norm() / b.to(torch.complex128).norm())
+    for call, x in ((plan.forward, sky * size), (plan.adjoint, coef * size)):
+        want = call(x, fp64=True)
+        err = rel(call(x), want)
+        assert by_blocks(plan)
+        assert err <= max(1.1 * rel(call(x, all_terms=True), want), REL)

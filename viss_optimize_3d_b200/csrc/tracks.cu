@@ -77,6 +77,7 @@ struct TrackNodeParams {
   unsigned long long *counter;
   int *err;
   int drop_tile;
+  const unsigned *peak;        // forward
 };
 
 // Node sums are stored per unit: a half tile (2 t + h) in the 64-pixel class, else
@@ -94,6 +95,28 @@ constexpr double kTurn32 = 1572864.0;            // 1.5 * 2^20
 __device__ __forceinline__ float turn_angle32(double t) {
   return static_cast<float>(__double2loint(t)) * 1.46291807926716e-9f;
 }
+
+// The tensor cores take operands below 2^-126 for zero, and the low half of a split
+// value is 2^-12 of it: skies below 1e-36 and coefficients below 1e-35 lost up to all
+// their accuracy.  A call's operands are scaled by the power of two that brings its
+// largest finite value to [1, 2), and the sums back in FP64; both are exact.
+__global__ void k_track_peak(long long n, const double4 *pixsky, const float2 *coef, unsigned *peak) {
+  unsigned top = 0;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const float2 v = pixsky ? make_float2(sky_of(pixsky[i]), 0.f) : coef[i];
+    if (isfinite(v.x)) top = max(top, __float_as_uint(fabsf(v.x)));
+    if (isfinite(v.y)) top = max(top, __float_as_uint(fabsf(v.y)));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top) atomicMax(peak, top);
+}
+__device__ __forceinline__ int peak_exponent(const unsigned *peak) {
+  const unsigned bits = *peak;
+  return bits ? min(max(static_cast<int>(bits >> 23) - 127, -126), 126) : 0;
+}
+__device__ __forceinline__ float scale_of(int e) { return __int_as_float((127 - e) << 23); }
+__device__ __forceinline__ double unscale_of(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
 constexpr int kNodeNT = 256;
 constexpr int kNodeR = 4;
@@ -153,6 +176,7 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
   float g_re[R], g_im[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) g_re[r] = g_im[r] = 0.f;
+  const float scale = scale_of(peak_exponent(p.peak));
   unsigned long long evaluated = 0;
   int next = 0;
   for (int it = 0; it < ntile; ++it) {
@@ -236,14 +260,14 @@ __global__ void __launch_bounds__(kNodeNT, 2) k_track_fwd_nodes(const TrackNodeP
           if (!((word[r] >> (t & 31)) & 1u)) continue;
           const int n = nb + r * NT + tid;
           if (HALF) {
-            p.sums[(2LL * t + h) * p.ld + n] = make_float2(t_re[r], t_im[r]);
+            p.sums[(2LL * t + h) * p.ld + n] = make_float2(scale * t_re[r], scale * t_im[r]);
           } else if (!((merged[r] >> (t & 31)) & 1u)) {
-            p.sums[static_cast<long long>(t) * p.ld + n] = make_float2(t_re[r], t_im[r]);
+            p.sums[static_cast<long long>(t) * p.ld + n] = make_float2(scale * t_re[r], scale * t_im[r]);
           } else {
             g_re[r] += t_re[r];
             g_im[r] += t_im[r];
             if (t % gt == gt - 1 || t == p.ntiles - 1) {   // the chunk holds whole groups
-              p.sums[static_cast<long long>(t / gt * gt) * p.ld + n] = make_float2(g_re[r], g_im[r]);
+              p.sums[static_cast<long long>(t / gt * gt) * p.ld + n] = make_float2(scale * g_re[r], scale * g_im[r]);
               g_re[r] = g_im[r] = 0.f;
             }
           }
@@ -279,6 +303,7 @@ struct TrackInterpParams {
   const float2 *coef;          // adjoint: slots
   int *err;
   bool drop;                   // test hook: block (0, 0) never signals its first product
+  const unsigned *peak;        // forward
 };
 
 // A wait that gave up ends an interpolation block at its next barrier (all threads
@@ -570,7 +595,7 @@ __global__ void __launch_bounds__(kInterpNT, 3) k_track_fwd_interp(const TrackIn
   if (warp == 0) tmem_free(tmem, 128);
   if (half == 0) {
     const double2 o = s_meet[row];
-    const double scale = 1.0 + static_cast<double>(interp_scale(r, false));
+    const double scale = unscale_of(peak_exponent(p.peak)) * (1.0 + static_cast<double>(interp_scale(r, false)));
     p.vacc[blockIdx.y * p.vstride + static_cast<long long>(blockIdx.x) * kTrackT + row] =
         make_double2(scale * (vre + o.x), scale * (vim + o.y));
   }
@@ -835,11 +860,12 @@ __global__ void __launch_bounds__(kRestNT, 6) k_track_adj_rest(const TrackRestPa
 }
 
 // ---------------------------------------------------------------- adjoint
-__global__ void k_track_coef(long long Ks, const int *slot, const float2 *coef, float2 *out) {
+__global__ void k_track_coef(long long Ks, const int *slot, const float2 *coef, const unsigned *peak, float2 *out) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= Ks) return;
   const int k = slot[i];
-  out[i] = k >= 0 ? coef[k] : make_float2(0.f, 0.f);
+  const float scale = scale_of(peak_exponent(peak));
+  out[i] = k >= 0 ? make_float2(scale * coef[k].x, scale * coef[k].y) : make_float2(0.f, 0.f);
 }
 
 constexpr int kAdjUnits = 64;          // units per pass, adjoint: 128 rows of the product (re, then im)
@@ -1192,13 +1218,14 @@ __global__ void __launch_bounds__(kAdjNodeNT, 4) k_track_adj_nodes(const TrackNo
 
 // One channel's image: node chunks + remainder chunks (FP64).
 __global__ void k_track_reduce_adj(long long J, long long Jpad, int nnode, const double *node, int nrest,
-                                   const double *rest, const int *perm, float scale, float *img, int accumulate) {
+                                   const double *rest, const int *perm, const unsigned *peak, float scale, float *img,
+                                   int accumulate) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= J) return;
   double s = 0;
   for (int c = 0; c < nnode; ++c) s += node[static_cast<long long>(c) * Jpad + i];
   for (int c = 0; c < nrest; ++c) s += rest[static_cast<long long>(c) * Jpad + i];
-  s *= static_cast<double>(scale);
+  s *= static_cast<double>(scale) * unscale_of(peak_exponent(peak));
   const long long j = perm[i];
   if (accumulate) s += static_cast<double>(img[j]);
   img[j] = static_cast<float>(s);
@@ -1253,6 +1280,7 @@ TrackInterpParams interp_params(const TrackState &S, const TrackInputs &in, cons
   ip.n0 = sl.n0;
   ip.ld = S.ld_max / (sl.cls == kHalf ? 2 : 1);
   ip.sums = S.sums;
+  ip.peak = S.peak;
   ip.use_off = use_off;
   return ip;
 }
@@ -1274,6 +1302,7 @@ TrackNodeParams node_params(const TrackState &S, const TrackInputs &in, const Tr
   np.nn = sl.n1 - sl.n0;
   np.ld = S.ld_max / (sl.cls == kHalf ? 2 : 1);
   np.sums = S.sums;
+  np.peak = S.peak;
   np.Jpad = in.Jpad;
   np.counter = counter;
   np.err = err;
@@ -1305,6 +1334,13 @@ TrackCut call_sums(TrackState &S, const TrackInputs &in, size_t bytes) {
   return {S.call.reset(bytes) ? S.call.base : nullptr};
 }
 
+int find_peak(const TrackState &S, long long n, const double4 *pixsky, const float2 *coef, int nsm, cudaStream_t st) {
+  TRACK_CUDA(cudaMemsetAsync(S.peak, 0, sizeof(unsigned), st), "peak");
+  k_track_peak<<<std::min<long long>(blks(n, 256), 8LL * nsm), 256, 0, st>>>(n, pixsky, coef, S.peak);
+  TRACK_CUDA(cudaGetLastError(), "peak");
+  return 0;
+}
+
 }  // namespace
 
 int tracks_forward(void *state, const TrackInputs &in, const double4 *pixsky, float2 *V, bool masked,
@@ -1325,6 +1361,7 @@ int tracks_forward(void *state, const TrackInputs &in, const double4 *pixsky, fl
   if (!sums.at) return record_error(-3, "viss_forward: device allocation failed (track block sums)");
   sums.take(vacc_d, vacc);
   sums.take(rest_d, static_cast<size_t>(nrest) * S.Ks);
+  if (int e = find_peak(S, in.channels * in.Jpad, pixsky, nullptr, in.nsm, st)) return e;
   if (nrest) {
     TrackRestParams rp = rest_params(S, in, masked, use_off, counter);
     rp.pix = pixsky;
@@ -1398,7 +1435,8 @@ int tracks_adjoint(void *state, const TrackInputs &in, const float2 *coef, float
   sums.take(coef_d, S.Ks);
   sums.take(node_d, nodes);
   sums.take(rest_d, rests);
-  k_track_coef<<<blks(S.Ks, 256), 256, 0, st>>>(S.Ks, S.slot, coef, coef_d);
+  if (int e = find_peak(S, in.K, nullptr, coef, in.nsm, st)) return e;
+  k_track_coef<<<blks(S.Ks, 256), 256, 0, st>>>(S.Ks, S.slot, coef, S.peak, coef_d);
   TRACK_CUDA(cudaGetLastError(), "coefficients");
   if (nrest) {
     TrackRestParams rp = rest_params(S, in, masked, use_off, counter);
@@ -1444,7 +1482,7 @@ int tracks_adjoint(void *state, const TrackInputs &in, const float2 *coef, float
     }
     k_track_reduce_adj<<<blks(in.J, 256), 256, 0, st>>>(
         in.J, in.Jpad, ny, node_d, nrest, rest_d + static_cast<long long>(ch) * nrest * in.Jpad, in.perm,
-        scale, image + static_cast<long long>(ch) * in.J, accumulate);
+        S.peak, scale, image + static_cast<long long>(ch) * in.J, accumulate);
     TRACK_CUDA(cudaGetLastError(), "reduce");
   }
   return 0;

@@ -814,7 +814,7 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
                     TrackArena::bytes<double4>(S.Ks) + TrackArena::bytes<double4>(nodes) +
                     TrackArena::bytes<int4>(masked ? S.Ks : 0) + TrackArena::bytes<float>(nodes * kTrackT) +
                     4 * TrackArena::bytes<unsigned>(rows) + TrackArena::bytes<int>(rows) +
-                    TrackArena::bytes<float2>(sums) + TrackArena::bytes<unsigned long long>(4)))
+                    TrackArena::bytes<float2>(sums) + TrackArena::bytes<unsigned long long>(4) + TrackArena::bytes<unsigned>(1)))
     return 0;
   S.plan.take(S.mask, room);
   S.plan.take(S.slot, S.Ks);
@@ -829,6 +829,7 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
   S.plan.take(S.sums, sums);
   unsigned long long *counts_d;                    // rest pairs, part pairs, ranks that differ; masks taken
   S.plan.take(counts_d, 4);
+  S.plan.take(S.peak, 1);
   auto up = [&](int *dst, const std::vector<int> &v) {
     return cudaMemcpyAsync(dst, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, st);
   };

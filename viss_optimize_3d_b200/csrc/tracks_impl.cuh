@@ -116,6 +116,7 @@ struct TrackState {
   int *mask_at = nullptr;
   uint4 *mask = nullptr;
   float2 *sums = nullptr;
+  unsigned *peak = nullptr;                // a call's largest finite sky or coefficient, as float bits
   TrackShape shape{};
   int nb = 0, W = 0;
   int gat[kClasses] = {0, 0, 0, 0};        // a class's first centre in gcen
