@@ -36,11 +36,10 @@ int tracks_build(void *state, const TrackInputs &in, cudaStream_t st, bool *usab
 void tracks_free(void *state);
 
 // Modelled time of one call through the blocks, in seconds, from what tracks_try
-// counted in its blocks.  Fitted to 105 observations of 1e10 to 7e11 terms (Nside 48
+// counted in its blocks.  Fitted to 200 observations of 1e10 to 7e11 terms (Nside 48
 // to 512, 500 to 8,640 snapshots, 4 to 10 satellites, 0.3 to 10 MHz), each occulted and
-// not, those near the direct kernels' time weighted most, and checked on 100 others of
-// 1e10 to 4e10: within 24 % (forward) and 24 % below to 58 % above (adjoint), the
-// largest where blocks are several times faster.
+// not: where the blocks take more than .6 of the direct kernels' time, 17 % below to 36 %
+// above what was measured (forward), 17 % below to 28 % above (adjoint).
 double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint);
 // Shares of the (sample, tile) pairs that an occulted call sees, and sees in part.
 void tracks_shares(const void *state, double *seen, double *mixed);

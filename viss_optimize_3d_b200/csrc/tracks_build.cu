@@ -472,23 +472,6 @@ __global__ void k_track_masks(int W, const int *slot, const int4 *refs, const fl
 
 void tracks_free(void *state) { delete static_cast<TrackState *>(state); }
 
-double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint) {
-  const TrackState &S = *static_cast<const TrackState *>(state);
-  const TrackEstimate &e = S.est[masked];
-  if (!adjoint)                                    // few blocks: short slabs, whose last waves are mostly empty
-    return (5.62e-13 * e.nodes + 1.6e-13 * e.units + 9.6e-14 * e.unit_nodes + 9.64e-12 * e.wide_units +
-            1.26e-8 * e.rest_blocks + 1.22e-4 * S.slab_count + 9.2e-5) * (1.0 + 20.0 / S.nb);
-  // unocculted, the few warps of the tiles that are left walk all samples alone
-  return 2.23e-13 * e.nodes + 8.92e-12 * e.units + 5.4e-14 * e.unit_nodes + 1.85e-10 * e.rest_samples +
-         (!masked && S.leaves_tiles ? 2.0e-9 * static_cast<double>(in.K) : 0.0) + 1.5e-4 * S.slab_count + 1.66e-4;
-}
-
-void tracks_shares(const void *state, double *seen, double *mixed) {
-  const TrackState &S = *static_cast<const TrackState *>(state);
-  *seen = S.est[1].seen;
-  *mixed = S.est[1].mixed;
-}
-
 namespace {
 
 // Modelled time of a block's nodes and interpolation per (sample, pixel), in issue
@@ -502,6 +485,25 @@ double block_slots(int c, int r, int len) {
 }
 
 }  // namespace
+
+double tracks_seconds(const void *state, const TrackInputs &in, bool masked, bool adjoint) {
+  const TrackState &S = *static_cast<const TrackState *>(state);
+  const TrackEstimate &e = S.est[masked];
+  if (!adjoint)                                    // few blocks: short slabs, whose last waves are mostly empty
+    return (4.68e-13 * e.nodes + 2.45e-12 * e.units + 1.95e-11 * e.wide_units + 1.12e-8 * e.rest_blocks +
+            1.44e-4 * S.slab_count) * (1.0 + 30.0 / S.nb);
+  if (masked)
+    return 2.23e-13 * e.nodes + 8.92e-12 * e.units + 5.4e-14 * e.unit_nodes + 1.85e-10 * e.rest_samples +
+           1.5e-4 * S.slab_count + 1.66e-4;
+  return 4.99e-13 * e.nodes + 3.95e-12 * e.units + 9.6e-14 * e.unit_nodes + 1.22e-10 * e.rest_samples +
+         (S.leaves_tiles ? 5.8e-9 * static_cast<double>(in.K) : 0.0) + 3.2e-5 * S.slab_count + 1.23e-4;
+}
+
+void tracks_shares(const void *state, double *seen, double *mixed) {
+  const TrackState &S = *static_cast<const TrackState *>(state);
+  *seen = S.est[1].seen;
+  *mixed = S.est[1].mixed;
+}
 
 namespace {
 
@@ -663,6 +665,10 @@ int tracks_try(void **statep, const TrackInputs &in, cudaStream_t st, bool *prom
       for (int q = 0; q < kShares; ++q) {
         double sum = 0;
         for (int i = 0; i < nsamp; ++i) sum += block_cost(c * kShares + q, i);
+        // an unocculted adjoint's few tiles that are left are walked by a few warps alone, about
+        // 1 ms at 360 blocks (7.5 against 6.4 ms at Nside 256 x 45,720 samples, 1 MHz): not for
+        // what the shares of a power-of-two grid differ by; on others they differ severalfold
+        if (within[c * kShares + q] < 1.0) sum *= 1.1;
         if (sum < best_sum) best_sum = sum, pick_q[c] = c * kShares + q;
       }
       for (int i = 0; i < nsamp; ++i) {
