@@ -275,20 +275,28 @@ int auto_adj_shape(const viss_plan *p, bool masked) {
   return adj_load(p, 3) < 0.93 * adj_load(p, 1) ? 3 : 1;
 }
 
-// Bytes of the workspace for any forward or adjoint call on the plan's samples,
-// with the plan's shapes or (-1) any that it may pick, occulted or not: a call must
-// not move the workspace that captured calls hold the address of.
-size_t call_workspace(const viss_plan *p, int fwd_shape, int adj_shape, bool fp64) {
+// Bytes of the workspace for a call in either direction, with the plan's shapes or (-1)
+// any that it may pick, occulted or not.
+size_t fwd_workspace(const viss_plan *p, int shape, bool fp64) {
+  size_t bytes = 0;
+  for (int s = 0; s < viss::kNumFwdShapes; ++s)
+    if (shape == s || (shape < 0 && s != 1 && s != 3))
+      bytes = std::max<size_t>(bytes, sizeof(double2) * static_cast<size_t>(fwd_chunks(p, s, fp64)) * p->K);
+  return bytes;
+}
+size_t adj_workspace(const viss_plan *p, int shape, bool fp64) {
   size_t bytes = 0;
   int spc = 0;
-  for (int s = 0; s < viss::kNumFwdShapes; ++s)
-    if (fwd_shape == s || (fwd_shape < 0 && s != 1 && s != 3))
-      bytes = std::max<size_t>(bytes, sizeof(double2) * static_cast<size_t>(fwd_chunks(p, s, fp64)) * p->K);
   for (int s = 0; s < viss::kNumAdjShapes; ++s)
-    if (adj_shape == s || (adj_shape < 0 && s != 2))
+    if (shape == s || (shape < 0 && s != 2))
       bytes = std::max<size_t>(bytes, sizeof(double) * static_cast<size_t>(adj_chunks(p, s, fp64, &spc)) * p->channels * p->Jpad);
   return bytes;
 }
+
+// What a call makes room for: a call must not move the workspace that captured calls
+// hold the address of, so the other direction's need counts too, unless it is out of
+// proportion (a chunk of very many pixels or samples is 8 or 16 bytes of each).
+size_t call_workspace(size_t own, size_t other) { return other <= (1ull << 28) ? std::max(own, other) : own; }
 
 cudaStream_t as_stream(void *s) { return static_cast<cudaStream_t>(s); }
 
@@ -643,7 +651,7 @@ static int forward_impl(viss_plan *p, const float *sky, float *V, int flags, cud
                         int shape, bool tracks = true, bool first = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
-  if (int s = workspace(p, call_workspace(p, shape, p->adj_shape, fp64))) return s;
+  if (int s = workspace(p, call_workspace(fwd_workspace(p, shape, fp64), adj_workspace(p, p->adj_shape, fp64)))) return s;
   if (shape < 0) shape = auto_fwd_shape(p, masked);
   const int nchunk = fwd_chunks(p, shape, fp64);
   if (int s = ensure(p->pixsky, p->pixsky_cap, sizeof(double4) * p->Jpad * p->channels,
@@ -793,7 +801,7 @@ static int adjoint_impl(viss_plan *p, const float *coef, float *image, float sca
                         bool tracks = true) {
   const bool fp64 = (flags & VISS_FP64) != 0;
   const bool masked = p->has_refs && !(flags & VISS_NO_MASK);
-  if (int s = workspace(p, call_workspace(p, p->fwd_shape, shape, fp64))) return s;
+  if (int s = workspace(p, call_workspace(adj_workspace(p, shape, fp64), fwd_workspace(p, p->fwd_shape, fp64)))) return s;
   if (shape < 0) shape = fcones ? 0 : auto_adj_shape(p, masked);
   int spc = 0;
   const int nchunk = adj_chunks(p, shape, fp64, &spc);
