@@ -277,3 +277,21 @@ def test_sizes_near_the_ends_of_fp32(cuda_device, size):
         err = rel(call(x), want)
         assert by_blocks(plan)
         assert err <= max(1.1 * rel(call(x, all_terms=True), want), REL)
+
+
+@pytest.mark.parametrize("nside,n_snap,f_hz", [
+    (41, 11200, 1e5), (73, 3600, 1e5), (87, 2500, 1e5), (97, 2020, 3e4), (121, 1300, 3e4),
+])
+def test_no_tile_is_left_out_of_uneven_grids(cuda_device, nside, n_snap, f_hz):
+    """Grids whose widest tile, across two base faces, is wider than the widest group
+    of 256 or 1,024 pixels, nothing occulted and every radius taken whole."""
+    obs = observation(nside, 10, n_snap, f_hz, False, False)
+    plan = api.Plan(api.pix2lmn(nside, "ring", device=cuda_device), torch.as_tensor(obs.uvw(f_hz), device=cuda_device))
+    assert plan.K * plan.J >= 1e10
+    sky, coef = inputs(plan, cuda_device)
+    got = plan.forward(sky)
+    assert by_blocks(plan)
+    close(got, plan.forward(sky, fp64=True))
+    got = plan.adjoint(coef)
+    assert by_blocks(plan)
+    close(got, plan.adjoint(coef, fp64=True))
