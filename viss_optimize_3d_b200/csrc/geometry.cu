@@ -60,9 +60,8 @@ __global__ void k_mask_bits(long long K, long long J, const double *lmn, const i
 }
 
 // Locality key of a direction: its base face and the position of its face
-// coordinates at Nside 2^13 (standard ang2pix_nest) along a Hilbert curve (the
-// widely published loop from coordinates to distance, e.g. Wikipedia's "Hilbert
-// curve").  The
+// coordinates at Nside 2^13 (standard ang2pix_nest) along a Hilbert curve (the widely
+// published loop from coordinates to distance, e.g. Wikipedia's "Hilbert curve").  The
 // curve visits the same hierarchy of squares as the NESTED index, so for a
 // HEALPix grid of a power-of-two Nside every aligned run of 4^k records is the
 // NESTED pixel of that size; but it never jumps, so runs that are not aligned
